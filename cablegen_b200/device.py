@@ -102,8 +102,8 @@ def expand_spawns(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
 
 def sort(x: torch.Tensor) -> Tuple[torch.Tensor, int]:
     """Ascending unsigned sort; returns (sorted tensor, digit passes)."""
-    _sync()
     keys = x.clone()
+    _sync()  # the copy runs on torch's stream: it must be complete before the engine sorts it
     tmp = empty(x.numel())
     in_tmp, passes = C.c_int(), C.c_int()
     check(lib().cgb_sort(_ptr(keys), _ptr(tmp), x.numel(), C.byref(in_tmp), C.byref(passes)))

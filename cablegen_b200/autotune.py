@@ -2,12 +2,12 @@
 
 The knobs (cgb_set_option):
 
-* ``sort_variant``  -- the digit pass of the radix sort: 0 ranks a 4096-key tile with warp
-  match, 1 with eight ballots per digit (keys re-read from L2 for the local scatter), 2 keeps
-  persistent CTAs that bulk-copy the next tile into shared memory while ranking the current one,
-  3 is the ballot pass specialised for byte digits (full tiles without bounds tests, digits read
-  from the one 32-bit word that holds them), 4 the same with 8192-key tiles of 512 threads (the
-  tile-size knob), 5 is 4 ranking each key with one warp match in place of eight ballots;
+* ``sort_variant``  -- 4 sorts by sampled buckets; the others are digit passes of a radix sort:
+  0 ranks a 4096-key tile with warp match, 1 with eight ballots per digit (keys re-read from L2
+  for the local scatter), 2 keeps persistent CTAs that bulk-copy the next tile into shared memory
+  while ranking the current one, 3 is the ballot pass specialised for byte digits (full tiles
+  without bounds tests, digits read from the one 32-bit word that holds them), 5 is 3 over
+  8192-key tiles, ranking each key with one warp match in place of eight ballots;
 * ``solve_variant`` -- 0 one thread per board, 1 the (board, empty cell) pairs of 32 boards
   spread over a warp;
 * ``hash_load_pct`` -- load factor of the open-addressing index of solved layers (0 picks it by

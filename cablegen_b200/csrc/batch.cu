@@ -102,9 +102,8 @@ struct BatchSink : LayerSink {
         return !changed || CGB_CUDA(cudaMemcpyAsync(d_active, active.data(), 256, cudaMemcpyHostToDevice, s));
     }
 
-    bool layer(int, u64 *d, u64 n, cudaStream_t s, bool *kept) override
+    bool layer(int, u64 *d, u64 n, cudaStream_t s) override
     {
-        *kept = false;
         Block b;
         if (!store.push(n, s, &b.h)) return false;
         u64 *dst = store.ptr(b.h, s);

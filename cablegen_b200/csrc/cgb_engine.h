@@ -42,9 +42,10 @@ struct GenTimes {
 // receives each generated layer (device pointer, valid on stream s)
 struct LayerSink {
     virtual ~LayerSink() {}
-    // set *kept = true to take ownership of the device buffer (freed later by
-    // the sink with dev_free on the engine stream)
-    virtual bool layer(int sum, u64 *d_boards, u64 n, cudaStream_t s, bool *kept) = 0;
+    // the buffer is reused by the layer after next
+    virtual bool layer(int sum, u64 *d_boards, u64 n, cudaStream_t s) = 0;
+    // whether gen.u4 shall hold the layer's 4-spawns (sorted, unique) at the call
+    virtual bool wants_carry() const { return false; }
 };
 
 // pinned staging for device -> host copies of layers and tables
@@ -111,15 +112,16 @@ struct HostArena {
 // working buffers of the generation sweep, kept between layers and calls
 struct GenBuffers {
     DevBuf<u64> a, b;          // raw move output and its sort scratch
-    DevBuf<u64> c[3];          // raw spawn streams and their sort scratch
+    DevBuf<u64> c[2];          // raw spawns and their sort scratch
     DevBuf<u64> S;             // boards of the next layer to move
-    DevBuf<u64> u2, u4, u4_next;
-    DevBuf<u64> moved;         // the current layer
+    DevBuf<u64> u4;            // 4-spawns still to join an input set: a resumed sweep's, a checkpoint's
+    DevBuf<u64> u2;            // 2-spawns (the cl seam)
+    DevBuf<u64> moved, prev;   // the current layer and the one before it
     DevBuf<u64> t;             // merge scratch of sliced layer steps
-    // empty cells over the moved layer (the size of its spawn streams), counted by
-    // the move step's unique pass; unknown after a sliced move step
-    u64 moved_empties = 0;
-    bool moved_empties_known = false;
+    // empty cells over a layer (the size of its spawn streams), counted by the
+    // move step's unique pass; unknown after a sliced move step
+    static constexpr u64 UNKNOWN = ~0ull;
+    u64 moved_empties = UNKNOWN, prev_empties = 0;
 };
 
 struct Engine {
@@ -130,9 +132,8 @@ struct Engine {
     SortWorkspace ws;
     Counters ctr;
     // pinned words the spawn expansion's count and error word are copied into
-    // without a wait, and the event after that copy (checked at a later wait)
+    // without a wait (checked after the sort that follows)
     u64 *h_spawn_check = nullptr;
-    cudaEvent_t spawn_check_ev = nullptr;
     cgb_rules rules{};
     int index_kind = INDEX_HASH;  // lookup structure of solved layers
     int bucket_bits = 22;         // INDEX_BUCKET: bucket count = 2^bits
@@ -154,11 +155,12 @@ struct Engine {
     HostArena host_layers;      // host copies of a sweep's layers (layers and tables both wanted)
     u64 host_layers_cap = 64ull << 30;  // bytes; beyond it tables carry their own key copy
     bool move_layer(const u64 *d_in, u64 n, GenTimes *tm);
-    bool spawn_layer(GenTimes *tm, bool unique_streams = false);
-    bool sort_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, DevBuf<u64> **out, GenTimes *tm);
+    bool spawn_streams(GenTimes *tm);   // g.u2, g.u4: the sorted unique 2- and 4-spawns of g.moved
+    bool spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm);
+    bool next_inputs(GenTimes *tm);     // g.S from the spawns of g.moved and g.prev
     bool sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
                           u64 *empties = nullptr);
-    bool merge_into(DevBuf<u64> &acc, const u64 *run, u64 n);
+    bool join(DevBuf<u64> &acc, DevBuf<u64> &run, u64 n);
     // layers start..end from the input set of layer `start`; h_carry = the
     // 4-spawns of layer start-2 still to merge into layer start+2's input
     // (empty for a fresh sweep, the checkpointed set when resuming)

@@ -2,15 +2,14 @@
 //
 // Generation (src/generate.c:409-615) keeps the rolling sets on the device:
 //   S_s    boards of tile sum s still to move (the reference's n)
-//   U4     sorted unique 4-spawns of the previous layer (the reference's n4,
-//          carried to become part of n2)
+//   L_s-2  the layer before (its 4-spawns are the reference's n4)
 // and per layer runs
-//   moved = unique(sort(expand_moves(S_s)))           -> the layer s.boards
-//   U2    = sort(spawn2(moved))                        (repeats kept)
-//   U4'   = sort(spawn4(moved))                        (repeats kept)
-//   S_s+2 = merge_unique(U2, U4)                       (src/generate.c:530-544)
-// (the merge drops repeats inside its runs as well as across them; the unique
-// pass of the move step also counts the spawns the next step will make)
+//   L_s   = unique(sort(expand_moves(S_s)))            -> the layer s.boards
+//   S_s+2 = unique(sort(spawn2(L_s) ++ spawn4(L_s-2))) (src/generate.c:530-544)
+// The reference sorts the two spawn streams apart, carries one of them to the
+// next layer and merges; the set is the same, and one sort of both streams
+// takes the place of two sorts and a merge.  The unique pass of the move step
+// also counts the spawns the next steps will make.
 // Layers go to a LayerSink: it keeps them in HBM (the resident gen+solve
 // run) or copies them out (files through the C API).
 //
@@ -322,7 +321,6 @@ bool Engine::init(int dev)
         h_spawn_check = (u64 *)h;
         h_spawn_check[0] = h_spawn_check[1] = 0;
     }
-    if (!spawn_check_ev && !CGB_CUDA(cudaEventCreateWithFlags(&spawn_check_ev, cudaEventDisableTiming))) return false;
     if (!ctr.d) {
         void *p;
         if (!CGB_CUDA(cudaMalloc(&p, 64 * sizeof(u64)))) return false;
@@ -366,43 +364,32 @@ bool Engine::sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, De
                               u64 *empties)
 {
     cudaStream_t s = stream;
-    u64 *sorted = x.p;
+    u64 *u = x.p;
     SortStats st;
-    if (!sort_keys(x.p, y.p, n, &sorted, ws, s, &st)) return false;
+    if (!sort_unique_keys(x.p, y.p, n, &u, nu, ws, s, &st, empties)) return false;
     if (tm) {
         tm->sorted_keys += n;
         tm->sort_passes += (u64)st.passes * n;
     }
-    DevBuf<u64> &full = (sorted == x.p) ? x : y;
-    DevBuf<u64> &dst = (sorted == x.p) ? y : x;
-    if (!unique_keys(full.p, n, dst.p, nu, ws, s, empties)) return false;
-    *out = &dst;
+    *out = (u == x.p) ? &x : &y;
     return true;
 }
 
-// sort of n raw keys in x (y = scratch), repeats kept: the merge that takes the
-// result drops them; returns the buffer holding the sorted keys
-bool Engine::sort_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, DevBuf<u64> **out, GenTimes *tm)
-{
-    u64 *sorted = x.p;
-    SortStats st;
-    if (!sort_keys(x.p, y.p, n, &sorted, ws, stream, &st)) return false;
-    if (tm) {
-        tm->sorted_keys += n;
-        tm->sort_passes += (u64)st.passes * n;
-    }
-    *out = (sorted == x.p) ? &x : &y;
-    return true;
-}
-
-// acc = acc u run (both sorted), through the scratch buffer t
-bool Engine::merge_into(DevBuf<u64> &acc, const u64 *run, u64 n)
+// acc = acc u run (both sorted and unique), through the scratch buffer t; the
+// first run just changes places with acc
+bool Engine::join(DevBuf<u64> &acc, DevBuf<u64> &run, u64 n)
 {
     cudaStream_t s = stream;
     GenBuffers &g = gen;
+    if (acc.n == 0) {
+        std::swap(acc, run);
+        acc.n = n;
+        return true;
+    }
+    if (n == 0) return true;
     if (!reserve(g.t, acc.n + n, s)) return false;
     u64 nm = 0;
-    if (!merge_unique(acc.p, acc.n, run, n, g.t.p, &nm, ws, s)) return false;
+    if (!merge_unique(acc.p, acc.n, run.p, n, g.t.p, &nm, ws, s)) return false;
     std::swap(acc, g.t);
     acc.n = nm;
     return true;
@@ -417,11 +404,11 @@ bool Engine::move_layer(const u64 *d_in, u64 n, GenTimes *tm)
     const u64 slice = std::max<u64>(1, max_sort_keys / 4);
     const bool chunked = n > slice;
     const u64 m0 = chunked ? slice : n;
-    if (!reserve(g.a, 4 * m0, s) || !reserve(g.b, 4 * m0, s)) return false;
     if (chunked) g.moved.n = 0;
-    g.moved_empties_known = false;
+    g.moved_empties = GenBuffers::UNKNOWN;
     for (u64 off = 0; off < n || (n == 0 && off == 0); off += m0) {
         const u64 m = std::min(m0, n - off);
+        if (!reserve(g.a, 4 * m0, s) || !reserve(g.b, 4 * m0, s)) return false;
         u64 nr = 0;
         if (!expand_moves(d_in + off, m, g.a.p, 4 * m, &nr, rt, prune_params(), ctr, s, filter, plan)) return false;
         u64 nu = 0, empties = 0;
@@ -431,91 +418,95 @@ bool Engine::move_layer(const u64 *d_in, u64 n, GenTimes *tm)
             std::swap(*u, g.moved);   // the layer; the old layer buffer becomes scratch
             g.moved.n = nu;
             g.moved_empties = empties;
-            g.moved_empties_known = true;
             return true;
         }
-        if (!merge_into(g.moved, u->p, nu)) return false;
+        if (!join(g.moved, *u, nu)) return false;
         if (tm) tm->chunks++;
     }
     return true;
 }
 
-// U2 / U4: sorted canonical 2-spawns and 4-spawns of the moved layer (unique
-// when unique_streams; else repeats stay for the next merge to drop);
-// U2 lands in g.u2, U4 in g.u4_next.  Spawn streams longer than max_sort_keys
-// are produced slice by slice and merged.
-bool Engine::spawn_layer(GenTimes *tm, bool unique_streams)
+// acc = acc u the spawns of src, in slices of at most max_sort_keys spawns
+bool Engine::spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm)
 {
     cudaStream_t s = stream;
     GenBuffers &g = gen;
-    const u64 *d_moved = g.moved.p;
-    const u64 n = g.moved.n;
-    // the spawn total: counted by the move step's unique pass, else by a kernel
-    u64 total = 0;
-    if (g.moved_empties_known) total = g.moved_empties;
-    else if (!count_spawns(d_moved, n, &total, ctr, s)) return false;
-    g.moved_empties_known = false;  // it belongs to this layer only
+    const u64 total = src.total;
     const bool chunked = total > max_sort_keys;
     const u64 cap = chunked ? max_sort_keys : total;
-    for (auto &x : g.c)
-        if (!reserve(x, cap, s)) return false;
-    if (chunked) g.u2.n = g.u4_next.n = 0;
     // first guess of a slice that fits; halved while its count does not
-    u64 step = chunked ? std::max<u64>(1, (u64)((double)n * 0.9 * (double)max_sort_keys / (double)total)) : n;
-    for (u64 off = 0; off < n || (n == 0 && off == 0);) {
-        u64 m = std::min(step, n - off);
-        u64 t = total;
+    const u64 step =
+        chunked ? std::max<u64>(1, (u64)((double)src.n * 0.9 * (double)max_sort_keys / (double)total)) : src.n;
+    for (u64 off = 0; off < src.n;) {
+        SpawnSource part = src;
+        part.boards = src.boards + off;
+        part.n = std::min(step, src.n - off);
         if (chunked) {
             for (;;) {
-                if (!count_spawns(d_moved + off, m, &t, ctr, s)) return false;
-                if (t <= max_sort_keys || m == 1) break;
-                m = (m + 1) / 2;
+                if (!count_spawns(part.boards, part.n, &part.total, ctr, s)) return false;
+                if (part.total <= max_sort_keys || part.n == 1) break;
+                part.n = (part.n + 1) / 2;
             }
-            if (t > max_sort_keys) {
-                set_error("spawn_layer: one board spawns more keys than max_sort_keys");
+            if (part.total > max_sort_keys) {
+                set_error("spawn_into: one board spawns more keys than max_sort_keys");
                 return false;
             }
         }
-        u64 ns = 0;
-        // one slice: the streams hold exactly t keys each; the kernel's count and
-        // error word are checked after the first sort below has waited on the
-        // stream anyway.  Slices keep the synchronous check.
-        const bool deferred = !chunked;
-        if (deferred) {
-            if (!expand_spawns_deferred(d_moved + off, m, g.c[0].p, g.c[1].p, t, ctr, s, plan, h_spawn_check,
-                                        spawn_check_ev))
-                return false;
-            ns = t;
-        } else if (!expand_spawns(d_moved + off, m, g.c[0].p, g.c[1].p, t, &ns, ctr, s, plan)) {
-            return false;
-        }
-        // the 2-spawns sort c[0] with c[2] as scratch; the 4-spawns then sort
-        // c[1] with the buffer the first sort left free.  Without unique_streams
-        // the sorted streams keep their repeats: every later merge drops them
-        DevBuf<u64> *u2 = nullptr, *u4 = nullptr;
-        u64 n2 = ns, n4 = ns;
-        if (unique_streams) {
-            if (!sort_unique_step(g.c[0], g.c[2], ns, &n2, &u2, tm)) return false;
-        } else if (!sort_step(g.c[0], g.c[2], ns, &u2, tm)) {
-            return false;
-        }
-        if (deferred && !check_spawns_deferred(h_spawn_check, spawn_check_ev, t)) return false;
-        DevBuf<u64> &spare = (u2 == &g.c[0]) ? g.c[2] : g.c[0];
-        if (unique_streams) {
-            if (!sort_unique_step(g.c[1], spare, ns, &n4, &u4, tm)) return false;
-        } else if (!sort_step(g.c[1], spare, ns, &u4, tm)) {
-            return false;
-        }
-        if (!chunked) {
-            std::swap(g.u2, *u2);
-            g.u2.n = n2;
-            std::swap(g.u4_next, *u4);
-            g.u4_next.n = n4;
-            return true;
-        }
-        if (!merge_into(g.u2, u2->p, n2) || !merge_into(g.u4_next, u4->p, n4)) return false;
-        if (tm) tm->chunks++;
-        off += m;
+        for (auto &x : g.c)
+            if (!reserve(x, cap, s)) return false;
+        if (!expand_next(part, SpawnSource{}, g.c[0].p, ctr, s, plan, h_spawn_check)) return false;
+        u64 nu = 0;
+        DevBuf<u64> *u = nullptr;
+        if (!sort_unique_step(g.c[0], g.c[1], part.total, &nu, &u, tm)) return false;
+        if (!check_spawns(h_spawn_check, part.total)) return false;
+        if (!join(acc, *u, nu)) return false;
+        if (chunked && tm) tm->chunks++;
+        off += part.n;
+    }
+    return true;
+}
+
+// the sorted unique 2- and 4-spawns of the moved layer (the cl seam's streams)
+bool Engine::spawn_streams(GenTimes *tm)
+{
+    GenBuffers &g = gen;
+    u64 total = g.moved_empties;
+    if (total == GenBuffers::UNKNOWN && !count_spawns(g.moved.p, g.moved.n, &total, ctr, stream)) return false;
+    g.moved_empties = GenBuffers::UNKNOWN;  // it belongs to this layer only
+    g.u2.n = g.u4.n = 0;
+    if (!reserve(g.u2, 1, stream) || !reserve(g.u4, 1, stream)) return false;
+    return spawn_into(SpawnSource{g.moved.p, g.moved.n, 1, total}, g.u2, tm) &&
+           spawn_into(SpawnSource{g.moved.p, g.moved.n, 2, total}, g.u4, tm);
+}
+
+// S = the 2-spawns of the moved layer and the 4-spawns of the one before it
+// (and a resumed sweep's carried 4-spawns): one sort of both streams, or, where
+// they are too long for one, their slices sorted apart and merged
+bool Engine::next_inputs(GenTimes *tm)
+{
+    cudaStream_t s = stream;
+    GenBuffers &g = gen;
+    if (g.moved_empties == GenBuffers::UNKNOWN && !count_spawns(g.moved.p, g.moved.n, &g.moved_empties, ctr, s))
+        return false;
+    const SpawnSource two{g.moved.p, g.moved.n, 1, g.moved_empties}, four{g.prev.p, g.prev.n, 2, g.prev_empties};
+    const u64 total = two.total + four.total;
+    g.S.n = 0;
+    if (total <= std::min(max_sort_keys, BUCKET_SORT_KEYS)) {
+        for (auto &x : g.c)
+            if (!reserve(x, total, s)) return false;
+        if (!expand_next(two, four, g.c[0].p, ctr, s, plan, h_spawn_check)) return false;
+        u64 nu = 0;
+        DevBuf<u64> *u = nullptr;
+        if (!sort_unique_step(g.c[0], g.c[1], total, &nu, &u, tm)) return false;
+        if (total && !check_spawns(h_spawn_check, total)) return false;
+        std::swap(g.S, *u);
+        g.S.n = nu;
+    } else if (!spawn_into(two, g.S, tm) || !spawn_into(four, g.S, tm)) {
+        return false;
+    }
+    if (g.u4.n) {  // carried in from a checkpoint
+        if (!join(g.S, g.u4, g.u4.n)) return false;
+        g.u4.n = 0;
     }
     return true;
 }
@@ -530,32 +521,22 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
     if (n_carry && !CGB_CUDA(cudaMemcpyAsync(g.u4.p, h_carry, n_carry * 8, cudaMemcpyHostToDevice, s))) return false;
     g.S.n = n_init;
     g.u4.n = n_carry;
+    g.prev.n = g.prev_empties = 0;
     // canonical layer boards share the 0xf mask of the canonical first board (fixed
     // formation cells); the kernels check every board against it
     plan = (n_init && !filter.fid) ? make_canon_plan(canonical(h_initial[0]), rules.free_formation != 0) : CanonPlan{};
     bool ok = true;
     for (int layer = start; layer <= end && ok; layer += 2) {
-        ok = move_layer(g.S.p, g.S.n, tm);
+        ok = move_layer(g.S.p, g.S.n, tm) && next_inputs(tm);
         if (!ok) break;
-        ok = spawn_layer(tm);
-        if (!ok) break;
-        // S_{s+2} = U2 u U4(previous layer)
-        if (!reserve(g.S, g.u2.n + g.u4.n, s)) {
-            ok = false;
-            break;
-        }
-        u64 nm = 0;
-        ok = merge_unique(g.u2.p, g.u2.n, g.u4.p, g.u4.n, g.S.p, &nm, ws, s);
-        if (!ok) break;
-        g.S.n = nm;
-        std::swap(g.u4, g.u4_next);
         if (tm) tm->boards += g.moved.n;
-        bool kept = false;
-        ok = sink.layer(layer, g.moved.p, g.moved.n, s, &kept);
-        if (kept) {
-            g.moved.p = nullptr;
-            g.moved.cap = g.moved.n = 0;
-        }
+        const bool carry = sink.wants_carry();
+        if (carry)
+            ok = reserve(g.u4, 1, s) && spawn_into(SpawnSource{g.moved.p, g.moved.n, 2, g.moved_empties}, g.u4, tm);
+        ok = ok && sink.layer(layer, g.moved.p, g.moved.n, s);
+        g.u4.n = 0;  // the next input set takes the 4-spawns from the layer itself
+        std::swap(g.moved, g.prev);
+        g.prev_empties = g.moved_empties;
     }
     if (ok) ok = sync();
     return ok;
@@ -564,8 +545,9 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
 void Engine::release_buffers()
 {
     GenBuffers &g = gen;
-    for (DevBuf<u64> *b : {&g.a, &g.b, &g.c[0], &g.c[1], &g.c[2], &g.S, &g.u2, &g.u4, &g.u4_next, &g.moved, &g.t})
+    for (DevBuf<u64> *b : {&g.a, &g.b, &g.c[0], &g.c[1], &g.S, &g.u2, &g.u4, &g.moved, &g.prev, &g.t})
         drop(*b, stream);
+    ws.buckets.release(stream);
 }
 
 }  // namespace cgb

@@ -10,6 +10,52 @@
 
 namespace cgb {
 
+// ---- device memory --------------------------------------------------------
+template <typename T>
+struct DevBuf {
+    T *p = nullptr;
+    u64 n = 0;     // elements in use
+    u64 cap = 0;   // elements allocated
+};
+
+bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
+void dev_free(void *p, cudaStream_t s);
+template <typename T>
+bool grow(DevBuf<T> &b, u64 n, cudaStream_t s)
+{
+    if (b.cap >= n && b.p) return true;
+    if (b.p) dev_free(b.p, s);
+    b.p = nullptr;
+    b.cap = 0;
+    u64 want = n < 64 ? 64 : n;
+    if (!dev_alloc((void **)&b.p, want * sizeof(T), s)) return false;
+    b.cap = want;
+    return true;
+}
+template <typename T>
+void drop(DevBuf<T> &b, cudaStream_t s)
+{
+    if (b.p) dev_free(b.p, s);
+    b.p = nullptr;
+    b.n = b.cap = 0;
+}
+
+// ---- bucket sort (bucketsort.cu) ------------------------------------------
+constexpr u64 BUCKET_SORT_KEYS = 160ull << 20;  // the most keys one call takes (512 x 512 buckets hold them)
+struct BucketWorkspace {
+    DevBuf<u32> ctl;           // control words, bucket counts, look-back words, boundaries
+    DevBuf<u64> coarse, fine;  // the buckets
+    u32 *host = nullptr;       // pinned copy of the first control words
+    void release(cudaStream_t s);
+};
+// out[0, *n_out) = keys[0, n) ascending, without repeats when `unique`; out must
+// not alias keys, which are only read.  empties (optional): the empty cells over
+// the keys kept.  *done = false (and nothing written) where the sort by buckets
+// does not apply: too many keys, no memory for the buckets, or keys that repeat
+// too often.
+bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 *empties, int *passes,
+                 BucketWorkspace &w, cudaStream_t s, bool *done);
+
 // ---- sort / unique / merge (sort.cu) ------------------------------------
 struct SortWorkspace {
     static constexpr int SMALL_WORDS = 8192;
@@ -17,6 +63,7 @@ struct SortWorkspace {
     u32 *lookback = nullptr;    // decoupled look-back state
     u64 lookback_bytes = 0;
     bool err_dirty = false;     // a sort left its errors in the word for unique to report
+    BucketWorkspace buckets;
     bool reserve(u64 words, cudaStream_t s);
     void release(cudaStream_t s);
 };
@@ -32,6 +79,10 @@ bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cuda
                SortStats *stats = nullptr);
 // reports device errors a sort left behind (when no unique_keys follows)
 bool sort_check(SortWorkspace &ws, cudaStream_t s);
+// sort_keys then unique_keys, in one pass over the buckets where they apply:
+// *out points at keys or tmp
+bool sort_unique_keys(u64 *keys, u64 *tmp, u64 n, u64 **out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
+                      SortStats *stats = nullptr, u64 *empties = nullptr);
 // out must not alias in
 // empties (optional): the number of empty cells over the kept keys
 bool unique_keys(const u64 *in, u64 n, u64 *out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
@@ -66,11 +117,19 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
                   const CanonPlan &plan = CanonPlan{});
 // number of empty cells over all boards (exact size of the spawn streams)
 bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s);
-// expand_spawns with cap = the exact spawn total and no wait: its count and error
-// word land in h_check (pinned, 2 words) behind `done`, for check_spawns_deferred
-bool expand_spawns_deferred(const u64 *in, u64 n, u64 *out2, u64 *out4, u64 cap, Counters &c, cudaStream_t s,
-                            const CanonPlan &plan, u64 *h_check, cudaEvent_t done);
-bool check_spawns_deferred(const u64 *h_check, cudaEvent_t done, u64 expect);
+// one spawn stream: every empty cell of a set of boards filled with `value`
+struct SpawnSource {
+    const u64 *boards = nullptr;
+    u64 n = 0;
+    u32 value = 1;  // 1: a 2 tile, 2: a 4 tile
+    u64 total = 0;  // empty cells over the boards
+};
+// the canonical spawns of both sources, a.total + b.total of them, in one array
+// and without a wait: the kernel's count and error word land in h_check (pinned,
+// 2 words), for check_spawns once the stream has been waited for
+bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters &c, cudaStream_t s,
+                 const CanonPlan &plan, u64 *h_check);
+bool check_spawns(const u64 *h_check, u64 expect);
 // canonical 2-spawn and 4-spawn of every empty cell of every board
 bool expand_spawns(const u64 *in, u64 n, u64 *out2, u64 *out4, u64 cap, u64 *n_out, Counters &c,
                    cudaStream_t s, const CanonPlan &plan = CanonPlan{});
@@ -142,36 +201,7 @@ bool solve_layer_f32(const u64 *keys, u64 n, float *out, const LayerIndex &t2, c
                      const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
                      const CanonPlan &plan = CanonPlan{});
 
-// ---- device memory --------------------------------------------------------
-template <typename T>
-struct DevBuf {
-    T *p = nullptr;
-    u64 n = 0;     // elements in use
-    u64 cap = 0;   // elements allocated
-};
-
-bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
-void dev_free(void *p, cudaStream_t s);
-template <typename T>
-bool grow(DevBuf<T> &b, u64 n, cudaStream_t s)
-{
-    if (b.cap >= n && b.p) return true;
-    if (b.p) dev_free(b.p, s);
-    b.p = nullptr;
-    b.cap = 0;
-    u64 want = n < 64 ? 64 : n;
-    if (!dev_alloc((void **)&b.p, want * sizeof(T), s)) return false;
-    b.cap = want;
-    return true;
-}
-template <typename T>
-void drop(DevBuf<T> &b, cudaStream_t s)
-{
-    if (b.p) dev_free(b.p, s);
-    b.p = nullptr;
-    b.n = b.cap = 0;
-}
-
+// ---- resident layers ------------------------------------------------------
 // Resident layers of a sweep.  Layers are appended during generation and
 // released top-down during the solve (last in, first out), so they are packed
 // into a few large chunks instead of one allocation per layer; nothing is

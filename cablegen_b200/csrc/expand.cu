@@ -285,6 +285,58 @@ __global__ void __launch_bounds__(256) expand_spawns_kernel(const u64 *__restric
     }
 }
 
+// One spawn value per source, both sources into one array.  A board's canonical
+// spawn is the maximum over its images with the one nibble added (the images
+// the plan names where the warp's boards have its mask).
+template <bool PLANNED>
+__device__ __forceinline__ u64 spawn_one(const u64 im[8], int cell, u64 value, u32 cand)
+{
+    u64 m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (PLANNED && !((cand >> k) & 1u)) continue;
+        m = umax64(m, im[k] | (value << (60 - 4 * image_cell(k, cell))));
+    }
+    return m;
+}
+
+__global__ void __launch_bounds__(256) expand_next_kernel(SpawnSource a, SpawnSource b, u64 *__restrict__ out, u64 cap,
+                                                          u64 *out_count, u32 *err, CanonPlan plan)
+{
+    __shared__ u32 scan_scratch[33];
+    __shared__ u64 base_sh;
+    // whole blocks of 256 boards of a, then of b
+    const u64 blocks_a = (a.n + 255) / 256, blocks = blocks_a + (b.n + 255) / 256;
+    for (u64 block = blockIdx.x; block < blocks; block += gridDim.x) {
+        const bool first = block < blocks_a;
+        const u64 idx = (first ? block : block - blocks_a) * 256 + threadIdx.x;
+        const u64 n = first ? a.n : b.n, value = first ? a.value : b.value;
+        const u64 board = idx < n ? (first ? a.boards : b.boards)[idx] : ~0ull;
+        u64 e = empty_mask(board);
+        const bool planned = __all_sync(0xffffffffu, idx >= n || fixed_pattern(board) == plan.mask);
+        const u32 cnt = popc64(e);
+        u32 total;
+        const u32 excl = block_exclusive_scan<u32>(cnt, scan_scratch, &total);
+        if (threadIdx.x == 0)
+            base_sh = total ? (u64)atomicAdd((unsigned long long *)out_count, (unsigned long long)total) : 0;
+        __syncthreads();
+        u64 pos = base_sh + excl;
+        if (pos + cnt > cap) {
+            if (cnt) atomicOr(err, ERR_CAPACITY);
+            continue;
+        }
+        u64 im[8];
+        images(board, im);
+        while (e) {
+            const int bit = 63 - __clzll(e);
+            e &= ~(1ull << bit);
+            const int cell = (60 - bit) >> 2;
+            out[pos++] = planned ? spawn_one<true>(im, cell, value, plan.cand(0))
+                                 : spawn_one<false>(im, cell, value, 0xFFu);
+        }
+    }
+}
+
 static int sm_count()
 {
     static int sms = 0;
@@ -396,39 +448,36 @@ bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s)
     return true;
 }
 
-// expand_spawns without the wait: the count and the error word are copied into
-// h_check (pinned, two words) behind the kernel and `done` is recorded after the
-// copy; check_spawns_deferred reads them once the caller has waited anyway
-bool expand_spawns_deferred(const u64 *in, u64 n, u64 *out2, u64 *out4, u64 cap, Counters &c, cudaStream_t s,
-                            const CanonPlan &plan, u64 *h_check, cudaEvent_t done)
+bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters &c, cudaStream_t s,
+                 const CanonPlan &plan, u64 *h_check)
 {
-    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
-    if (n) {
-        const int grid = (int)std::min<u64>((n + 255) / 256, (u64)sm_count() * 8);
+    // the count and, 32 words on, the error word
+    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s)) || !CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s)))
+        return false;
+    const u64 blocks = (a.n + 255) / 256 + (b.n + 255) / 256, cap = a.total + b.total;
+    if (blocks) {
+        const int grid = (int)std::min<u64>(blocks, (u64)sm_count() * 8);
         kclock().begin(s, &kstats().spawn_ms);
-        expand_spawns_kernel<<<grid, 256, 0, s>>>(in, n, out2, out4, cap, c.d, c.err, plan);
+        expand_next_kernel<<<grid, 256, 0, s>>>(a, b, out, cap, c.d, c.err, plan);
         kclock().end(s);
         if (!CGB_CUDA(cudaGetLastError())) return false;
     }
     if (!CGB_CUDA(cudaMemcpyAsync(h_check, c.d, sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaMemcpyAsync(h_check + 1, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaEventRecord(done, s)))
+        !CGB_CUDA(cudaMemcpyAsync(h_check + 1, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s)))
         return false;
-    kstats().spawn_bytes += 8 * n + 16 * cap;
+    kstats().spawn_bytes += 8 * (a.n + b.n) + 8 * cap;
     return true;
 }
 
-bool check_spawns_deferred(const u64 *h_check, cudaEvent_t done, u64 expect)
+bool check_spawns(const u64 *h_check, u64 expect)
 {
-    if (!CGB_CUDA(cudaEventSynchronize(done))) return false;
     const u32 e = (u32)h_check[1];
     if (e) {
-        set_error(std::string("expand_spawns: device error ") + err_string(e));
+        set_error(std::string("expand_next: device error ") + err_string(e));
         return false;
     }
     if (h_check[0] != expect) {
-        set_error("expand_spawns: " + std::to_string(h_check[0]) + " spawns written, " + std::to_string(expect) +
+        set_error("expand_next: " + std::to_string(h_check[0]) + " spawns written, " + std::to_string(expect) +
                   " expected");
         return false;
     }

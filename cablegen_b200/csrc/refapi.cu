@@ -483,10 +483,10 @@ struct FileSink : cgb::LayerSink {
     const char *fmt = nullptr;
     FileWriter *writer = nullptr;
     bool checkpoint = false;
+    bool wants_carry() const override { return checkpoint; }
     std::string last_checkpoint;  // written by the writer thread, removed when superseded
-    bool layer(int sum, u64 *d, u64 n, cudaStream_t s, bool *kept) override
+    bool layer(int sum, u64 *d, u64 n, cudaStream_t s) override
     {
-        *kept = false;
         cgb::Engine &e = cgb::Engine::get();
         void *h = nullptr;
         const int slot = writer->take(n * 8, &h);

@@ -4,12 +4,16 @@
 // (src/array.c:246-291, inc/external/fluxsort.h:112-120): layers must come out
 // ascending and duplicate-free, bit-for-bit.
 //
+// * the sort by sampled buckets of bucketsort.cu is the default; the passes
+//   here take what it does not: inputs beyond its size, keys that repeat so
+//   often that a bucket overflows, no memory for the buckets, and the other
+//   values of the "sort_variant" option.
 // * LSD radix sort with 8-bit digits in the single-pass "onesweep" form
 //   (Adinets & Merrill 2022): one histogram pass for all eight digits, then
-//   one pass per non-constant digit that ranks a 4096-key tile in shared
-//   memory and finds its global bin offsets by a decoupled look-back.  Digits
-//   on which every key agrees (the 0xff prefix that canonical formation
-//   boards share) are skipped.
+//   one pass per non-constant digit that ranks a tile in shared memory and
+//   finds its global bin offsets by a decoupled look-back.  Digits on which
+//   every key agrees (the 0xff prefix that canonical formation boards share)
+//   are skipped.
 // * unique: adjacent-difference flags, ballot/popc compaction, decoupled
 //   look-back for the tile prefix.
 // * merge_unique: merge-path partition of two sorted runs, per-thread
@@ -20,6 +24,7 @@
 // sets ERR_LOOKBACK_TIMEOUT in the error word and finishes without waiting.
 #include "common.cuh"
 #include "engine.h"
+#include "lookback.cuh"
 #include <cstring>
 
 namespace cgb {
@@ -86,64 +91,6 @@ __device__ __forceinline__ u32 lookback_sum(const u32 *words, u64 stride, int j,
     }
     return excl;
 }
-
-__device__ __forceinline__ u64 ld_relaxed64(const u64 *p)
-{
-    u64 v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed64(u64 *p, u64 v)
-{
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// Warp-wide form of the walk back over one count per tile, called by all 32
-// lanes of one warp: lane i reads the word of tile j - i, so one round trip
-// covers 32 predecessors.  The words from tile j down to the nearest inclusive
-// prefix (or down to the first one not yet published, which is polled again)
-// are summed with a warp reduction.  Every lane returns the same prefix.
-template <typename W>
-__device__ __forceinline__ W warp_lookback_sum(const W *words, int j, u32 *err)
-{
-    constexpr W PRE = (W)2 << (8 * sizeof(W) - 2);
-    constexpr W MASK = ((W)1 << (8 * sizeof(W) - 2)) - 1;
-    const int lane = threadIdx.x & 31;
-    W excl = 0;
-    u32 spins = 0;
-    const u32 limit = g_spin_limit;
-    while (j >= 0) {
-        const int k = j - lane;
-        W v;
-        if (k >= 0) {
-            if constexpr (sizeof(W) == 8) v = ld_relaxed64((const u64 *)words + k);
-            else v = ld_relaxed((const u32 *)words + k);
-        } else {
-            v = PRE;  // before tile 0: an empty inclusive prefix ends the walk
-        }
-        const W flag = v & ~MASK;
-        const u32 pre = __ballot_sync(0xffffffffu, flag == PRE);
-        const u32 unready = __ballot_sync(0xffffffffu, flag == 0);
-        // lanes that count: up to the nearest inclusive prefix, and short of
-        // the first word not yet published
-        const u32 upto = pre ? ((pre & (0u - pre)) << 1) - 1 : 0xffffffffu;
-        const u32 stop = unready & upto;
-        const u32 take = stop ? (stop & (0u - stop)) - 1 : upto;
-        W c = ((take >> lane) & 1) ? (v & MASK) : (W)0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        excl += c;
-        if (!stop && pre) break;
-        j -= __popc(take);
-        // a round trip to L2 per poll is the wait; the poll count bounds it
-        if (stop && ++spins > limit) {
-            if (lane == 0) atomicOr(err, ERR_LOOKBACK_TIMEOUT);
-            break;
-        }
-    }
-    return excl;
-}
-
 
 // ---------------------------------------------------------------------------
 // histogram of all eight byte digits in one pass
@@ -712,8 +659,9 @@ static int pipe_grid(int device)
 }
 
 // 0: match ranking, 1: ballot ranking, 2: pipelined persistent, 3: byte-digit ballot
-// (4096-key tiles), 4: byte-digit ballot with 8192-key tiles (the default: measured
-// 9 % faster than 3 on the LL sweep), 5: 4 with match ranking
+// (4096-key tiles), 4 (the default): the sort by buckets, and byte-digit ballot with
+// 8192-key tiles (measured 9 % faster than 3 on the LL sweep) for what it does not
+// take, 5: byte-digit with 8192-key tiles and match ranking
 int g_sort_variant = 4;
 
 // the 8192-key byte pass needs more than the default 48 KiB of shared memory
@@ -761,13 +709,6 @@ struct UniqueSmem {
     u32 tile;
 };
 
-// empty cells (0 nibbles) of a board
-__device__ __forceinline__ u32 zero_nibbles(u64 k)
-{
-    const u64 x = k | (k >> 1) | (k >> 2) | (k >> 3);
-    return (u32)__popcll(~x & 0x1111111111111111ull);
-}
-
 template <bool FULL>
 __device__ __forceinline__ void unique_tile(const u64 *__restrict__ in, u32 n, u64 *__restrict__ out, u32 *lookback,
                                             u32 tile, u32 *out_count, u32 *err, UniqueSmem &S,
@@ -812,7 +753,7 @@ __device__ __forceinline__ void unique_tile(const u64 *__restrict__ in, u32 n, u
             if (lane == 0) st_relaxed(lookback, LB_PRE | tile_total);
         } else {
             if (lane == 0) st_relaxed(lookback + tile, LB_AGG | tile_total);
-            prefix = warp_lookback_sum<u32>(lookback, (int)tile - 1, err);
+            prefix = warp_lookback_sum<u32>(lookback, (int)tile - 1, err, g_spin_limit);
             if (lane == 0) st_relaxed(lookback + tile, LB_PRE | (prefix + tile_total));
         }
         if (lane < UNQ_THREADS / 32) S.warp_base[lane] = prefix + incl - c;
@@ -1014,7 +955,7 @@ __global__ void __launch_bounds__(MRG_THREADS) merge_unique_kernel(const u64 *__
             if (lane == 0) st_relaxed64(lookback, LB64_PRE | tile_total);
         } else {
             if (lane == 0) st_relaxed64(lookback + tile, LB64_AGG | tile_total);
-            prefix = warp_lookback_sum<u64>(lookback, (int)tile - 1, err);
+            prefix = warp_lookback_sum<u64>(lookback, (int)tile - 1, err, g_spin_limit);
             if (lane == 0) st_relaxed64(lookback + tile, LB64_PRE | (prefix + tile_total));
         }
         if (lane < MRG_THREADS / 32) warp_sh[lane] = wi - c;
@@ -1069,6 +1010,7 @@ void SortWorkspace::release(cudaStream_t s)
     lookback = nullptr;
     small = nullptr;
     lookback_bytes = 0;
+    buckets.release(s);
 }
 
 // small words: [0,2048) histograms, [2048,2064) tile counters, 2064 err, 2065 count,
@@ -1109,11 +1051,57 @@ int sort_plan(const u32 *hist_host, u64 n, int *digits)
     return np;
 }
 
+static bool digit_sort(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s,
+                       SortStats *stats);
+
 bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s, SortStats *stats)
 {
     *sorted = keys;
     if (stats) *stats = SortStats{};
     if (n <= 1) return true;
+    if (g_sort_variant == 4) {
+        bool done = false;
+        int passes = 0;
+        u64 m = 0;
+        if (!bucket_sort(keys, n, tmp, false, &m, nullptr, &passes, ws.buckets, s, &done)) return false;
+        if (done) {
+            *sorted = tmp;
+            if (stats) {
+                stats->passes = passes;
+                stats->n = n;
+            }
+            return true;
+        }
+    }
+    return digit_sort(keys, tmp, n, sorted, ws, s, stats);
+}
+
+bool sort_unique_keys(u64 *keys, u64 *tmp, u64 n, u64 **out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
+                      SortStats *stats, u64 *empties)
+{
+    if (stats) *stats = SortStats{};
+    if (g_sort_variant == 4 && !ws.err_dirty) {
+        bool done = false;
+        int passes = 0;
+        if (!bucket_sort(keys, n, tmp, true, n_out, empties, &passes, ws.buckets, s, &done)) return false;
+        if (done) {
+            *out = tmp;
+            if (stats) {
+                stats->passes = passes;
+                stats->n = n;
+            }
+            return true;
+        }
+    }
+    u64 *sorted = keys;
+    if (n > 1 && !digit_sort(keys, tmp, n, &sorted, ws, s, stats)) return false;
+    *out = sorted == keys ? tmp : keys;
+    return unique_keys(sorted, n, *out, n_out, ws, s, empties);
+}
+
+static bool digit_sort(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s, SortStats *stats)
+{
+    *sorted = keys;
     if (n > (u64)LB_MASK) {
         set_error("sort_keys: more than 2^30 keys in one call");
         return false;

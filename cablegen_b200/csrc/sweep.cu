@@ -81,11 +81,10 @@ struct StoreSink : LayerSink {
         }
         return true;
     }
-    bool layer(int sum, u64 *d, u64 n, cudaStream_t s, bool *kept) override
+    bool layer(int sum, u64 *d, u64 n, cudaStream_t s) override
     {
         // the engine's layer buffer is reused by the next layer step: keep an
         // exact-size copy in the store (8 B/board)
-        *kept = false;
         Layer L{sum, {}, true};
         if (!store.push(n, s, &L.h)) return false;
         u64 *keys = store.ptr(L.h, s);

@@ -403,9 +403,8 @@ struct CopyOutSink : LayerSink {
     HostStage stage;
     u64 d2h = 0;
     bool failed = false;
-    bool layer(int sum, u64 *d, u64 n, cudaStream_t s, bool *kept) override
+    bool layer(int sum, u64 *d, u64 n, cudaStream_t s) override
     {
-        *kept = false;
         if (!fn) return true;
         if (!stage.reserve(n * 8 + 8)) return false;
         if (n && !CGB_CUDA(cudaMemcpyAsync(stage.p, d, n * 8, cudaMemcpyDeviceToHost, s))) return false;

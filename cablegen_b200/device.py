@@ -101,7 +101,7 @@ def expand_spawns(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
 
 
 def sort(x: torch.Tensor) -> Tuple[torch.Tensor, int]:
-    """Ascending unsigned sort; returns (sorted tensor, digit passes)."""
+    """Ascending unsigned sort; returns (sorted tensor, passes over the keys)."""
     keys = x.clone()
     _sync()  # the copy runs on torch's stream: it must be complete before the engine sorts it
     tmp = empty(x.numel())

@@ -41,7 +41,8 @@ int cgb_set_rules(const cgb_rules *rules);
  * kind 1), "solve_variant" (0 one thread per board, 1 warp-compacted),
  * "sort_variant" (0 match ranking, 1 ballot ranking, 2 persistent CTAs with
  * bulk-copy prefetch of the next tile, 3 byte-digit passes over 4096-key tiles,
- * 4 byte-digit passes over 8192-key tiles, the default, 5 as 4 with one match
+ * 4, the default: sort by sampled buckets, with byte-digit passes over 8192-key
+ * tiles for inputs that it does not take, 5 those passes with one match
  * instruction per key in place of eight ballots), "spill_reserve_mb"
  * (free device memory kept before resident layers spill to host memory),
  * "max_sort_keys" (larger layer steps are cut into chunks and merged),
@@ -76,9 +77,10 @@ int cgb_count_spawns(const uint64_t *d_in, uint64_t n, uint64_t *total);
 /* Canonical 2- and 4-spawns of every empty cell (src/generate.c:177-199). */
 int cgb_expand_spawns(const uint64_t *d_in, uint64_t n, uint64_t *d_out2, uint64_t *d_out4, uint64_t cap,
                       uint64_t *n_out);
-/* Ascending LSD radix sort of d_keys[0,n) with scratch d_tmp[0,n) (replaces
+/* Ascending sort of d_keys[0,n) with scratch d_tmp[0,n) (replaces
  * qs_sort_h/fluxsort_uint64, src/array.c:289-291).  *result_in_tmp tells which
- * buffer holds the result; *passes = digit passes executed. */
+ * buffer holds the result; *passes = passes over the keys (digit passes, or the
+ * steps of the sort by buckets). */
 int cgb_sort(uint64_t *d_keys, uint64_t *d_tmp, uint64_t n, int *result_in_tmp, int *passes);
 /* Drop repeats of a sorted array into d_out (must not alias d_in). */
 int cgb_unique(const uint64_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *n_out);

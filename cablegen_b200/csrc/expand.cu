@@ -134,10 +134,10 @@ __device__ __forceinline__ bool set_insert(unsigned long long *set, u64 key)
     return true;
 }
 
-// the four moves of b, pruned, canonicalised (over the plan's images when
-// PLANNED, chosen once per warp so that the choice is a uniform branch) and
-// checked against the CTA's set; returns the mask of results to write
-template <bool PLANNED>
+// the four moves of b, pruned, canonicalised (by the plan's form, or its list of
+// images; FORM -1: over all eight) and checked against the CTA's set; returns
+// the mask of results to write
+template <int FORM>
 __device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const PruneParams &pp, const PruneTable &pt,
                                            const CanonPlan &plan, unsigned long long *set, u64 r[4], u32 *raw)
 {
@@ -151,7 +151,7 @@ __device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const Prune
     for (int k = 0; k < 4; k++) {
         u64 m;
         if (move_left(t, v[k], &m) == 2 && !(pp.enabled && popc64(empty_mask(m)) != empties && prune_by_table(m, pt))) {
-            r[k] = PLANNED ? canon_cand(m, plan.cand(k)) : canonical(m);
+            r[k] = canon_planned<FORM>(m, plan, k);
             (*raw)++;
             if (set_insert(set, r[k])) mask |= 1u << k;
         }
@@ -159,6 +159,7 @@ __device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const Prune
     return mask;
 }
 
+template <int FORM>
 __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 *__restrict__ in, u64 n,
                                                                       u64 *__restrict__ out, u64 cap,
                                                                       u64 *out_count, const unsigned short *g_move,
@@ -197,8 +198,8 @@ __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 
             // boards of a formation that has reached its last layer stop here
             const bool live = !ff.fid || __ldg(ff.active + __ldg(ff.fid + fixed_pattern(b)));
             if (live && !(pp.enabled && prune_by_table(b, *pt))) {
-                if (planned) mask = board_moves<true>(t, b, pp, *pt, plan, set, r, &raw);
-                else mask = board_moves<false>(t, b, pp, *pt, plan, set, r, &raw);
+                if (planned) mask = board_moves<FORM>(t, b, pp, *pt, plan, set, r, &raw);
+                else mask = board_moves<-1>(t, b, pp, *pt, plan, set, r, &raw);
             }
         }
         const u32 cnt = __popc(mask);
@@ -285,21 +286,19 @@ __global__ void __launch_bounds__(256) expand_spawns_kernel(const u64 *__restric
     }
 }
 
-// One spawn value per source, both sources into one array.  A board's canonical
-// spawn is the maximum over its images with the one nibble added (the images
-// the plan names where the warp's boards have its mask).
-template <bool PLANNED>
-__device__ __forceinline__ u64 spawn_one(const u64 im[8], int cell, u64 value, u32 cand)
+// One spawn value per source, both sources into one array.  A spawn keeps the
+// board's 0xf cells, so its canonical form follows view 0 of the plan where the
+// warp's boards have the plan's mask; without a plan it is the maximum over the
+// board's eight images with the one nibble added.
+__device__ __forceinline__ u64 spawn_any(const u64 im[8], int cell, u64 value)
 {
     u64 m = 0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        if (PLANNED && !((cand >> k) & 1u)) continue;
-        m = umax64(m, im[k] | (value << (60 - 4 * image_cell(k, cell))));
-    }
+    for (int k = 0; k < 8; k++) m = umax64(m, im[k] | (value << (60 - 4 * image_cell(k, cell))));
     return m;
 }
 
+template <int FORM>
 __global__ void __launch_bounds__(256) expand_next_kernel(SpawnSource a, SpawnSource b, u64 *__restrict__ out, u64 cap,
                                                           u64 *out_count, u32 *err, CanonPlan plan)
 {
@@ -325,14 +324,20 @@ __global__ void __launch_bounds__(256) expand_next_kernel(SpawnSource a, SpawnSo
             if (cnt) atomicOr(err, ERR_CAPACITY);
             continue;
         }
+        if (planned) {
+            while (e) {
+                const int bit = 63 - __clzll(e);  // nibble's low bit
+                e &= ~(1ull << bit);
+                out[pos++] = canon_planned<FORM>(board | (value << bit), plan, 0);
+            }
+            continue;
+        }
         u64 im[8];
         images(board, im);
         while (e) {
             const int bit = 63 - __clzll(e);
             e &= ~(1ull << bit);
-            const int cell = (60 - bit) >> 2;
-            out[pos++] = planned ? spawn_one<true>(im, cell, value, plan.cand(0))
-                                 : spawn_one<false>(im, cell, value, 0xFFu);
+            out[pos++] = spawn_any(im, (60 - bit) >> 2, value);
         }
     }
 }
@@ -392,8 +397,11 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
     if (n == 0) return true;
     static bool attr = false;
     if (!attr) {
-        if (!CGB_CUDA(cudaFuncSetAttribute(expand_moves_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           EXP_SMEM)))
+        const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if (!CGB_CUDA(cudaFuncSetAttribute(expand_moves_kernel<CANON_LIST>, smem, EXP_SMEM)) ||
+            !CGB_CUDA(cudaFuncSetAttribute(expand_moves_kernel<CANON_ONE>, smem, EXP_SMEM)) ||
+            !CGB_CUDA(cudaFuncSetAttribute(expand_moves_kernel<CANON_DIAGONAL>, smem, EXP_SMEM)) ||
+            !CGB_CUDA(cudaFuncSetAttribute(expand_moves_kernel<CANON_MIRROR>, smem, EXP_SMEM)))
             return false;
         attr = true;
     }
@@ -419,8 +427,12 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
     const u64 chunks = (n + (u64)window * EXP_THREADS - 1) / ((u64)window * EXP_THREADS);
     const int grid = (int)std::min<u64>(chunks, sms);
     kclock().begin(s, &kstats().expand_ms);
-    expand_moves_kernel<<<grid, EXP_THREADS, EXP_SMEM, s>>>(in, n, out, cap, c.d, t.move, p, d_prune, c.err, ff,
-                                                            plan, c.d + 5, window);
+    const auto kernel = plan.form == CANON_ONE        ? expand_moves_kernel<CANON_ONE>
+                        : plan.form == CANON_DIAGONAL ? expand_moves_kernel<CANON_DIAGONAL>
+                        : plan.form == CANON_MIRROR   ? expand_moves_kernel<CANON_MIRROR>
+                                                      : expand_moves_kernel<CANON_LIST>;
+    kernel<<<grid, EXP_THREADS, EXP_SMEM, s>>>(in, n, out, cap, c.d, t.move, p, d_prune, c.err, ff, plan, c.d + 5,
+                                               window);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
     u64 raw = 0;
@@ -458,7 +470,11 @@ bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters 
     if (blocks) {
         const int grid = (int)std::min<u64>(blocks, (u64)sm_count() * 8);
         kclock().begin(s, &kstats().spawn_ms);
-        expand_next_kernel<<<grid, 256, 0, s>>>(a, b, out, cap, c.d, c.err, plan);
+        const auto kernel = plan.form == CANON_ONE        ? expand_next_kernel<CANON_ONE>
+                            : plan.form == CANON_DIAGONAL ? expand_next_kernel<CANON_DIAGONAL>
+                            : plan.form == CANON_MIRROR   ? expand_next_kernel<CANON_MIRROR>
+                                                          : expand_next_kernel<CANON_LIST>;
+        kernel<<<grid, 256, 0, s>>>(a, b, out, cap, c.d, c.err, plan);
         kclock().end(s);
         if (!CGB_CUDA(cudaGetLastError())) return false;
     }

@@ -49,6 +49,11 @@ __host__ __device__ __forceinline__ uint64_t home_slot(uint64_t key, uint64_t ca
     return mulhi64(hash64(key), cap);
 }
 
+// A key's chain starts at the even slot at or below its home: the 32-byte sector
+// that a lookup's first load brings in then holds the second slot of the chain
+// too, so the one lane in eight that needs it finds it in L1.
+__host__ __device__ __forceinline__ uint64_t home_pair(uint64_t key, uint64_t cap) { return home_slot(key, cap) & ~1ull; }
+
 // slots for n keys at a load factor of at most pct percent, a multiple of 64
 __host__ __device__ __forceinline__ uint64_t hash_capacity_for(uint64_t n, uint64_t pct)
 {

@@ -127,7 +127,7 @@ __device__ __forceinline__ V table_value(const DevTable<V> &t, u64 key)
     }
     if (t.kind == INDEX_HASH) {
         if (t.cap == 0) return V(0);
-        const u64 s = home_slot(key, t.cap);
+        const u64 s = home_pair(key, t.cap);
         const ulonglong2 e = __ldg(t.slots + s);
         if (e.x == key) return from_bits<V>(e.y);
         if (e.x == 0) return V(0);
@@ -231,7 +231,7 @@ __device__ __forceinline__ void probe4(const DevTable<V> &t, const u64 *key, u32
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const bool on = (legal >> j) & 1 && t.cap;
-            s[j] = on ? home_slot(key[j], t.cap) : 0;
+            s[j] = on ? home_pair(key[j], t.cap) : 0;
             e[j] = on ? __ldg(t.slots + s[j]) : make_ulonglong2(0, 0);
         }
 #pragma unroll
@@ -291,7 +291,7 @@ __device__ __forceinline__ V probe1(const DevTable<V> &t, u64 key, bool legal)
     }
     if (t.kind == INDEX_HASH) {
         if (t.cap == 0) return V(0);
-        const u64 s = home_slot(key, t.cap);
+        const u64 s = home_pair(key, t.cap);
         const ulonglong2 e = __ldg(t.slots + s);
         if (e.x == key) return from_bits<V>(e.y);
         if (e.x == 0) return V(0);
@@ -300,11 +300,12 @@ __device__ __forceinline__ V probe1(const DevTable<V> &t, u64 key, bool legal)
     return sorted_lookup(t, key);
 }
 
-// cell_bests with the four views in a loop that is not unrolled: one view's
-// two successors per iteration (two loads in flight per lane, hidden by the
-// other warps), a quarter of the code.  The unrolled body of all eight
-// successors is large enough that warps wait on instruction fetch.
-template <bool PLANNED, typename V>
+// cell_bests with the four views in a loop that is not unrolled: one view's two
+// successors per iteration, a quarter of the code (the unrolled body of all
+// eight successors is large enough that warps wait on instruction fetch).  Both
+// successors' first slots are loaded before either is looked at: 1.06 -> 0.96 ms
+// for 5M LL boards, the kernel being bound by the latency of these loads.
+template <int FORM, typename V>
 __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int cell, const CanonPlan &plan,
                                                   const DevTable<V> &t2, const DevTable<V> &t4, V &best2, V &best4,
                                                   u32 &probes)
@@ -313,6 +314,8 @@ __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int
     const int r0 = cell >> 2, q0 = cell & 3;
     best2 = V(0);
     best4 = V(0);
+    const bool wide = t2.kind == INDEX_HASH && t4.kind == INDEX_HASH && !t2.ch.on && !t4.ch.on;
+    const bool compact = sizeof(V) == 4 && t2.kind == INDEX_HASH && t4.kind == INDEX_HASH && t2.ch.on && t4.ch.on;
 #pragma unroll 1
     for (int k = 0; k < 4; k++) {
         // view k: id, H, T, H.T; the cell of the spawn in it
@@ -324,11 +327,40 @@ __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int
         u64 m2, m4;
         const bool ok2 = move_left(rt, y | (1ull << sh), &m2) == 2;
         const bool ok4 = move_left(rt, y | (2ull << sh), &m4) == 2;
-        const u64 c2 = PLANNED ? canon_cand(m2, plan.cand(k)) : canonical(m2);
-        const u64 c4 = PLANNED ? canon_cand(m4, plan.cand(k)) : canonical(m4);
+        const u64 c2 = canon_planned<FORM>(m2, plan, k);
+        const u64 c4 = canon_planned<FORM>(m4, plan, k);
         probes += (u32)ok2 + (u32)ok4;
-        best2 = vmax(best2, probe1(t2, c2, ok2));
-        best4 = vmax(best4, probe1(t4, c4, ok4));
+        V v2 = V(0), v4 = V(0);
+        if (wide) {
+            const u64 s2 = home_pair(c2, t2.cap), s4 = home_pair(c4, t4.cap);
+            ulonglong2 e2 = make_ulonglong2(0, 0), e4 = e2;
+            if (ok2) e2 = __ldg(t2.slots + s2);
+            if (ok4) e4 = __ldg(t4.slots + s4);
+            v2 = from_bits<V>(e2.y);
+            v4 = from_bits<V>(e4.y);
+            // an empty slot (and a move that was not looked up) holds key 0 and value 0
+            if (e2.x != c2) v2 = e2.x == 0 ? V(0) : hash_probe_rest<V>(t2.slots, t2.cap, c2, s2);
+            if (e4.x != c4) v4 = e4.x == 0 ? V(0) : hash_probe_rest<V>(t4.slots, t4.cap, c4, s4);
+        } else if (compact) {
+            u32 g2, g4;
+            const u64 s2 = compact_home(t2.ch, c2, &g2), s4 = compact_home(t4.ch, c4, &g4);
+            u64 e2 = 0, e4 = 0;
+            if (ok2 && (c2 & t2.ch.cmask) == t2.ch.cval) e2 = __ldg((const u64 *)t2.slots + s2);
+            if (ok4 && (c4 & t4.ch.cmask) == t4.ch.cval) e4 = __ldg((const u64 *)t4.slots + s4);
+            v2 = from_bits<V>(e2 >> 32);
+            v4 = from_bits<V>(e4 >> 32);
+            if ((u32)e2 != g2)
+                v2 = (u32)e2 == 0u ? V(0)
+                                   : compact_probe_rest<V>((const u64 *)t2.slots, t2.cap, t2.ch.dbits, s2, g2);
+            if ((u32)e4 != g4)
+                v4 = (u32)e4 == 0u ? V(0)
+                                   : compact_probe_rest<V>((const u64 *)t4.slots, t4.cap, t4.ch.dbits, s4, g4);
+        } else {
+            v2 = probe1(t2, c2, ok2);
+            v4 = probe1(t4, c4, ok4);
+        }
+        best2 = vmax(best2, v2);
+        best4 = vmax(best4, v4);
     }
 }
 
@@ -386,7 +418,7 @@ constexpr int ITEM_MAX = 32 * 16;  // pairs of 32 boards at most
 template <typename V>
 constexpr int item_smem() { return TABLE_BYTES_S + ITEM_WARPS * (ITEM_MAX * 2 + 2 * 32 * (int)sizeof(V)); }
 
-template <typename V>
+template <typename V, int FORM>
 __global__ void __launch_bounds__(ITEM_THREADS, 1)
     solve_items_kernel(const u64 *__restrict__ keys, u64 n, V *__restrict__ out, DevTable<V> t2, DevTable<V> t4,
                        SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan)
@@ -427,8 +459,8 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
             const u64 ob = __shfl_sync(0xffffffffu, b, owner);
             V best2 = 0, best4 = 0;
             if (has) {
-                if (planned) cell_bests_rolled<true>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
-                else cell_bests_rolled<false>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
+                if (planned) cell_bests_rolled<FORM>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
+                else cell_bests_rolled<-1>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
             }
             best_sh[lane] = best2;
             best_sh[32 + lane] = best4;
@@ -464,7 +496,7 @@ __global__ void hash_build_kernel(const u64 *__restrict__ keys, const V *__restr
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
         const u64 key = keys[i];
-        u64 s = home_slot(key, cap);
+        u64 s = home_pair(key, cap);
         bool placed = false;
         for (u64 p = 0; p < cap; p++) {
             const u64 prev = atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)key);
@@ -554,7 +586,7 @@ __global__ void __launch_bounds__(256) region_scatter_kernel(const u64 *__restri
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            r[u] = (u32)(home_slot(key[u], cap) / BUILD_REGION);
+            r[u] = (u32)(home_pair(key[u], cap) / BUILD_REGION);
             p[u] = i0 + u * stride < n ? atomicAdd(cursor + r[u], 1u) : 0u;
         }
 #pragma unroll
@@ -588,7 +620,7 @@ __global__ void __launch_bounds__(512) region_build_kernel(const ulonglong2 *__r
         for (u32 j = threadIdx.x; j < cnt; j += blockDim.x) {
             const ulonglong2 e = bucket[j];
             bool placed = false;
-            for (u32 sl = (u32)(home_slot(e.x, cap) - base); sl < len; sl++) {
+            for (u32 sl = (u32)(home_pair(e.x, cap) - base); sl < len; sl++) {
                 if (atomicCAS((unsigned long long *)&tab[sl].x, 0ull, (unsigned long long)e.x) == 0ull) {
                     tab[sl].y = e.y;
                     placed = true;
@@ -613,7 +645,7 @@ __global__ void overflow_insert_kernel(const ulonglong2 *__restrict__ over, u32 
 {
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const ulonglong2 e = over[i];
-        u64 s = home_slot(e.x, cap);
+        u64 s = home_pair(e.x, cap);
         bool placed = false;
         for (u64 p = 0; p < cap; p++) {
             if (atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)e.x) == 0ull) {
@@ -844,14 +876,24 @@ static DevTable<V> dev_table(const LayerIndex &ix)
 
 int g_solve_variant = 1;  // 0: direct (one thread per board), 1: (board, cell) pairs per warp
 
+template <typename V, int FORM>
+static bool items_attr_one()
+{
+    return CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<V, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         item_smem<V>()));
+}
+template <typename V>
+static bool items_attr()
+{
+    return items_attr_one<V, CANON_LIST>() && items_attr_one<V, CANON_ONE>() && items_attr_one<V, CANON_DIAGONAL>() &&
+           items_attr_one<V, CANON_MIRROR>();
+}
+
 static bool solve_attrs()
 {
     static bool attr = false;
     if (!attr) {
-        if (!CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<double>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, item_smem<double>())) ||
-            !CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<float>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, item_smem<float>())) ||
+        if (!items_attr<double>() || !items_attr<float>() ||
             !CGB_CUDA(cudaFuncSetAttribute(solve_direct_kernel<double>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, TABLE_BYTES_S)) ||
             !CGB_CUDA(cudaFuncSetAttribute(solve_direct_kernel<float>,
@@ -868,12 +910,17 @@ static void enqueue_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, 
                           const SolveRules &r, const DeviceRowTable &rt, u64 *probes, cudaStream_t s,
                           const CanonPlan &plan)
 {
-    if (g_solve_variant == 1)
-        solve_items_kernel<V><<<grid_for(n, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
+    if (g_solve_variant == 1) {
+        const auto kernel = plan.form == CANON_ONE        ? solve_items_kernel<V, CANON_ONE>
+                            : plan.form == CANON_DIAGONAL ? solve_items_kernel<V, CANON_DIAGONAL>
+                            : plan.form == CANON_MIRROR   ? solve_items_kernel<V, CANON_MIRROR>
+                                                          : solve_items_kernel<V, CANON_LIST>;
+        kernel<<<grid_for(n, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
             keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan);
-    else
+    } else {
         solve_direct_kernel<V><<<grid_for(n, DIRECT_THREADS, 1), DIRECT_THREADS, TABLE_BYTES_S, s>>>(
             keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan);
+    }
 }
 
 template <class V>

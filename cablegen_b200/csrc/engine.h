@@ -192,6 +192,8 @@ bool build_index(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int buc
 // layer, widened to double; 0.0 for a board not in it
 bool lookup_batch(const LayerIndex &ix, int vbytes, const u64 *boards, u64 m, bool canon, double *out,
                   cudaStream_t s);
+// the same by search in the sorted layer: ix needs keys, vals and n only
+bool lookup_sorted(const LayerIndex &ix, int vbytes, const u64 *boards, u64 m, bool canon, double *out, cudaStream_t s);
 
 // plan: images that can be canonical for the layer's 0xf mask (CanonPlan{}: all eight)
 bool solve_layer_f64(const u64 *keys, u64 n, double *out, const LayerIndex &t2, const LayerIndex &t4,

@@ -1008,6 +1008,8 @@ bool solve_layer_f32(const u64 *keys, u64 n, float *out, const LayerIndex &t2, c
 }
 
 // ---- batch lookup (lookup(), src/solve.c:108-164, for many boards) --------
+constexpr u64 LOOKUP_FEW = 4096;  // boards up to which a warp takes each: every warp is resident at once
+
 template <typename V>
 __global__ void __launch_bounds__(256) lookup_batch_kernel(DevTable<V> t, const u64 *__restrict__ boards, u64 m,
                                                            int canon, double *__restrict__ out)
@@ -1016,6 +1018,82 @@ __global__ void __launch_bounds__(256) lookup_batch_kernel(DevTable<V> t, const 
         const u64 b = boards[i];
         out[i] = (double)table_value(t, canon ? canonical(b) : b);
     }
+}
+
+// The same lookups by search in the sorted layer, without an index.
+//
+// A few boards: a warp per board, 31 keys probed at once, so that a layer of a
+// million keys takes four dependent loads instead of twenty.
+template <typename V>
+__global__ void __launch_bounds__(256) lookup_few_kernel(const u64 *__restrict__ keys, const V *__restrict__ vals, u64 n,
+                                                         const u64 *__restrict__ boards, u64 m, int canon,
+                                                         double *__restrict__ out)
+{
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64)gridDim.x * (256 / 32);
+    for (u64 i = ((u64)blockIdx.x * 256 + threadIdx.x) >> 5; i < m; i += warps) {
+        const u64 b = boards[i], key = canon ? canonical(b) : b;
+        u64 lo = 0, len = n;
+        while (len > 32) {
+            // 32 stretches; the last keys of the first 31 decide
+            const u64 step = (len + 31) / 32, at = (lane + 1) * step - 1;
+            const bool below = lane < 31 && at < len && __ldg(keys + lo + at) < key;
+            const u64 skip = __popc(__ballot_sync(0xffffffffu, below)) * step;
+            lo += skip;
+            len = min(step, len - skip);
+        }
+        const u32 hit = __ballot_sync(0xffffffffu, lane < len && __ldg(keys + lo + lane) == key);
+        if (lane == 0) out[i] = hit ? (double)__ldg(vals + lo + __ffs(hit) - 1) : 0.0;
+    }
+}
+
+// Many boards: a thread per board; the first ten halvings run over 1024 evenly
+// spaced keys in shared memory.
+constexpr u32 LOOKUP_TOP = 1024;
+template <typename V>
+__global__ void __launch_bounds__(256) lookup_search_kernel(const u64 *__restrict__ keys, const V *__restrict__ vals,
+                                                            u64 n, const u64 *__restrict__ boards, u64 m, int canon,
+                                                            double *__restrict__ out)
+{
+    __shared__ u64 top[LOOKUP_TOP];
+    const u64 step = (n + LOOKUP_TOP - 1) / LOOKUP_TOP;  // top[j] = the first key of stretch j
+    for (u32 j = threadIdx.x; j < LOOKUP_TOP; j += 256) top[j] = j * step < n ? __ldg(keys + j * step) : ~0ull;
+    __syncthreads();
+    const u32 stretches = (u32)((n + step - 1) / step);
+    for (u64 i = (u64)blockIdx.x * 256 + threadIdx.x; i < m; i += (u64)gridDim.x * 256) {
+        const u64 b = boards[i], key = canon ? canonical(b) : b;
+        u32 j = 0;
+#pragma unroll
+        for (u32 w = LOOKUP_TOP / 2; w; w >>= 1)
+            if (j + w < stretches && top[j + w] <= key) j += w;
+        u64 lo = j * step, len = min(step, n - lo);
+        while (len > 1) {
+            const u64 half = len >> 1;
+            lo = __ldg(keys + lo + half) <= key ? lo + half : lo;
+            len -= half;
+        }
+        out[i] = __ldg(keys + lo) == key ? (double)__ldg(vals + lo) : 0.0;
+    }
+}
+
+template <typename V>
+static void launch_search(const LayerIndex &ix, const u64 *boards, u64 m, bool canon, double *out, cudaStream_t s)
+{
+    const V *vals = (const V *)ix.vals;
+    if (m <= LOOKUP_FEW)
+        lookup_few_kernel<V><<<grid_for(m * 32, 256, 8), 256, 0, s>>>(ix.keys, vals, ix.n, boards, m, canon ? 1 : 0, out);
+    else
+        lookup_search_kernel<V><<<grid_for(m, 256, 8), 256, 0, s>>>(ix.keys, vals, ix.n, boards, m, canon ? 1 : 0, out);
+}
+
+bool lookup_sorted(const LayerIndex &ix, int vbytes, const u64 *boards, u64 m, bool canon, double *out, cudaStream_t s)
+{
+    if (m == 0) return true;
+    if (ix.n == 0) return CGB_CUDA(cudaMemsetAsync(out, 0, m * sizeof(double), s));
+    if (vbytes == 4) launch_search<float>(ix, boards, m, canon, out, s);
+    else launch_search<double>(ix, boards, m, canon, out, s);
+    kstats().launches++;
+    return CGB_CUDA(cudaGetLastError());
 }
 
 bool lookup_batch(const LayerIndex &ix, int vbytes, const u64 *boards, u64 m, bool canon, double *out,

@@ -119,8 +119,9 @@ int cgb_solve_layer(const uint64_t *d_keys, uint64_t n, void *d_out, int precisi
 
 /* ---- lookup of many boards (lookup(), src/solve.c:108-164) ---------------
  * (d_keys, d_vals, n): one solved layer on the device, keys sorted; d_vals
- * double (precision 64) or float (32).  The layer gets the index the solve
- * builds (option "index"), then every board of d_boards[m] is looked up --
+ * double (precision 64) or float (32).  Every board of d_boards[m] is looked
+ * up -- through the index the solve builds (option "index"), or by a search of
+ * the sorted layer where m boards do not pay for a hash index of n keys --
  * canonicalised first when canonicalize, as lookup() does -- and its value
  * written to d_out[m] as a double (0.0 for a board not in the layer).  For
  * consumers that look up many positions at once; lookup() itself stays the

@@ -53,9 +53,18 @@ constexpr int BUCKET_THREADS = 256;
 constexpr u64 KEY_MAX = ~0ull;
 constexpr u32 BK_OVERFLOW = 1u << 16;   // a bucket ran full (beside the ERR_* bits)
 
-// control words of one sort (u32 indexes)
-constexpr u32 C_TICKET = 0, C_FLAGS = 1, C_BUCKETS = 2, C_COUNT = 4, C_EMPTIES = 6, C_COARSE = 16,
-              C_BASE = C_COARSE + BK_COARSE, C_NUM = C_BASE + BK_COARSE, C_FINE = C_NUM + BK_COARSE;
+// control words of one sort (u32 indexes): its head, and its arrays, which start
+// with the counts of the coarse buckets
+constexpr u32 H_TICKET = 0, H_FLAGS = 1, H_BUCKETS = 2, H_COUNT = BUCKET_COUNT_AT, H_EMPTIES = 6;
+constexpr u32 A_COARSE = 0, A_BASE = A_COARSE + BK_COARSE, A_NUM = A_BASE + BK_COARSE, A_FINE = A_NUM + BK_COARSE;
+
+// The number of keys of a call: known on the host, or counted by a kernel before
+// it (at most n, which sizes grids and buckets).
+struct KeyCount {
+    u32 n;
+    const u64 *counted;
+    __device__ __forceinline__ u32 get() const { return counted ? (u32)min((u64)n, *counted) : n; }
+};
 
 __device__ __forceinline__ u32 pad16(u32 i) { return i + (i >> 4); }
 constexpr u32 SAMPLE_WORDS = BK_SAMPLES + BK_SAMPLES / 16, BUCKET_WORDS = BK_CAP + BK_CAP / 16;
@@ -290,42 +299,43 @@ __device__ __forceinline__ void write_bounds(K (&v)[BK_KPT], K *buf, u32 m, u32 
 // the whole input; 1: the coarse step; 2: CTA c, the boundaries inside coarse
 // bucket c, whose number follows its size.  A sample is one random key out of
 // each of equally long stretches, so that neither a regular pattern nor a
-// sorted input biases it.
+// sorted input biases it.  (Nothing to do for the keys of one bucket: the bucket
+// sort takes them from the input.)
 template <int STEP>
-__global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u64 *__restrict__ src, u32 n,
-                                                                        u32 buckets, u32 coarse_cap, u32 *ctl,
-                                                                        u64 *__restrict__ bounds)
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u64 *__restrict__ src, KeyCount n,
+                                                                        u32 buckets, u32 coarse_cap, u32 *head,
+                                                                        u32 *arrays, u64 *__restrict__ bounds)
 {
     extern __shared__ __align__(16) u64 split_buf[];
     __shared__ u32 scratch[33];
     __shared__ BitMoves moves[2];
-    u32 cnt = n, nb = buckets;
+    u32 cnt = n.get(), nb = buckets;
+    if (cnt <= BK_CAP) return;
     if (STEP == 2) {
         const u32 c = blockIdx.x;
         // this coarse bucket's first fine bucket: the numbers of those before it, summed
         u32 mine = 0, all = 0;
         for (u32 i = threadIdx.x; i < buckets; i += SPLIT_THREADS) {
-            const u32 f = (min(ctl[C_COARSE + i], coarse_cap) + BK_TARGET - 1) / BK_TARGET;
+            const u32 f = (min(arrays[A_COARSE + i], coarse_cap) + BK_TARGET - 1) / BK_TARGET;
             all += f;
             mine += i < c ? f : 0;
         }
         u32 base, total;
         block_exclusive_scan<u32>(mine, scratch, &base);
         block_exclusive_scan<u32>(all, scratch, &total);
-        cnt = min(ctl[C_COARSE + c], coarse_cap);
+        cnt = min(arrays[A_COARSE + c], coarse_cap);
         nb = (cnt + BK_TARGET - 1) / BK_TARGET;
         if (threadIdx.x == 0) {
-            ctl[C_BASE + c] = base;
-            ctl[C_NUM + c] = nb;
-            if (c == 0) ctl[C_BUCKETS] = total;
+            arrays[A_BASE + c] = base;
+            arrays[A_NUM + c] = nb;
+            if (c == 0) head[H_BUCKETS] = total;
         }
         if (nb <= 1) return;
         src += (u64)c * coarse_cap;
         bounds += (u64)c * BK_FAN;
-    } else if (STEP == 0 && threadIdx.x == 0) {
-        ctl[C_BASE] = 0;
-        ctl[C_NUM] = nb;
-        ctl[C_BUCKETS] = nb;
+    } else if (STEP == 0) {
+        nb = (cnt + BK_TARGET - 1) / BK_TARGET;
+        if (threadIdx.x == 0) head[H_BUCKETS] = nb;
     }
     const u32 m = min(min(nb * (STEP == 1 ? 64u : STEP == 2 ? 32u : 24u), BK_SAMPLES), cnt);
     if (threadIdx.x < 4) scratch[threadIdx.x] = threadIdx.x < 2 ? 0xffffffffu : 0u;
@@ -388,18 +398,21 @@ struct PartSmem {
 // the only step's fine buckets).
 template <bool FINE>
 __global__ void __launch_bounds__(PART_THREADS, 4)
-    bucket_partition_kernel(const u64 *__restrict__ src, u32 n, u32 src_cap, u32 tiles, u32 buckets,
-                            const u64 *__restrict__ bounds, u32 *ctl, u32 counters, u64 *__restrict__ dst, u32 dst_cap)
+    bucket_partition_kernel(const u64 *__restrict__ src, KeyCount n, u32 src_cap, u32 tiles, u32 buckets,
+                            const u64 *__restrict__ bounds, u32 *head, u32 *arrays, u32 counters,
+                            u64 *__restrict__ dst, u32 dst_cap)
 {
     extern __shared__ __align__(16) unsigned char part_smem[];
     PartSmem &S = *reinterpret_cast<PartSmem *>(part_smem);
     const u32 t = threadIdx.x;
     const u32 c = FINE ? blockIdx.x / tiles : 0, tile = FINE ? blockIdx.x % tiles : blockIdx.x;
-    const u32 cnt = FINE ? min(ctl[C_COARSE + c], src_cap) : n;
+    const u32 all = n.get();
+    const u32 cnt = FINE ? min(arrays[A_COARSE + c], src_cap) : all;
     const u32 start = tile * BK_TILE;
-    if (start >= cnt) return;
-    const u32 nb = FINE ? ctl[C_NUM + c] : buckets;
-    const u32 base = FINE ? ctl[C_BASE + c] : 0;
+    if (start >= cnt || all <= BK_CAP) return;
+    // buckets 0: the only step, whose buckets follow the number of keys
+    const u32 nb = FINE ? arrays[A_NUM + c] : buckets ? buckets : head[H_BUCKETS];
+    const u32 base = FINE ? arrays[A_BASE + c] : 0;
     if (FINE) {
         src += (u64)c * src_cap;
         bounds += (u64)c * BK_FAN;
@@ -436,7 +449,7 @@ __global__ void __launch_bounds__(PART_THREADS, 4)
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             num[q] = S.count[2 * t + q];
-            g[q] = num[q] ? atomicAdd(ctl + counters + base + 2 * t + q, num[q]) : 0;
+            g[q] = num[q] ? atomicAdd(arrays + counters + base + 2 * t + q, num[q]) : 0;
         }
         u32 total;
         u32 first = block_exclusive_scan<u32>(num[0] + num[1], S.scan, &total);
@@ -447,7 +460,7 @@ __global__ void __launch_bounds__(PART_THREADS, 4)
             u32 delta = 0xFFFFFFFFu;
             if (num[q]) {
                 if (g[q] + num[q] <= dst_cap) delta = (base + b) * dst_cap + g[q] - first;
-                else atomicOr(ctl + C_FLAGS, BK_OVERFLOW);
+                else atomicOr(head + H_FLAGS, BK_OVERFLOW);
             }
             S.delta[b] = delta;
             first += num[q];
@@ -486,7 +499,7 @@ struct BucketSmem {
 // their offset by look-back, write.  EMIT turns a sorted key into the u64.
 template <bool UNIQUE, bool DIRECT, typename K, class Emit>
 __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh, u32 cnt, u32 tile, u32 tiles, u32 *look,
-                                              u32 *ctl, u64 *__restrict__ out, u32 count_empties, BucketSmem &S, Emit emit)
+                                              u32 *head, u64 *__restrict__ out, u32 count_empties, BucketSmem &S, Emit emit)
 {
     constexpr u32 ALL = 0xffffffffu;
     constexpr u32 AGG = 1u << 30, PRE = 2u << 30;
@@ -520,7 +533,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
         if (!DIRECT) {
             if (tile > 0) {
                 if (UNIQUE && lane == 0) st_relaxed(look + tile, AGG | total);
-                prefix = warp_lookback_sum<u32>(look, (int)tile - 1, ctl + C_FLAGS, SPIN_LIMIT);
+                prefix = warp_lookback_sum<u32>(look, (int)tile - 1, head + H_FLAGS, SPIN_LIMIT);
             }
             if (lane == 0) st_relaxed(look + tile, PRE | (prefix + total));
         }
@@ -528,7 +541,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
         if (lane == 0) {
             S.prefix = prefix;
             S.kept = total;
-            if (tile + 1 == tiles) *(u64 *)(ctl + C_COUNT) = prefix + total;
+            if (tile + 1 == tiles) *(u64 *)(head + H_COUNT) = prefix + total;
         }
     }
     __syncthreads();
@@ -549,14 +562,14 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
     }
     if (UNIQUE && count_empties) {
         empty = __reduce_add_sync(ALL, empty);
-        if (lane == 0 && empty) atomicAdd((unsigned long long *)(ctl + C_EMPTIES), (unsigned long long)empty);
+        if (lane == 0 && empty) atomicAdd((unsigned long long *)(head + H_EMPTIES), (unsigned long long)empty);
     }
 }
 
 // One bucket: sorted, repeats dropped with UNIQUE, written at the sum of the
 // counts of the buckets before it.  Buckets are taken in ticket order, so every
-// predecessor that a look-back waits for is already running.  DIRECT: the
-// input itself is the only bucket.
+// predecessor that a look-back waits for is already running.  An input that
+// fits one bucket is taken as it is (DIRECT: known on the host).
 //
 // The keys of a bucket share their high cells, and the constant bits of the
 // others (fixed cells, the top bits of small tiles) hold no order: in buckets
@@ -566,21 +579,23 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
 // are where the high words agree); the others are sorted as they are.
 template <bool UNIQUE, bool DIRECT>
 __global__ void __launch_bounds__(BUCKET_THREADS, 4)
-    bucket_sort_kernel(const u64 *__restrict__ src, u32 n, u32 counters, u32 words, u32 *ctl, u64 *__restrict__ out,
-                       u32 count_empties)
+    bucket_sort_kernel(const u64 *__restrict__ input, KeyCount n, const u64 *__restrict__ slots, u32 counters, u32 words,
+                       u32 *head, u32 *arrays, u64 *__restrict__ out, u32 count_empties)
 {
     constexpr u32 ALL = 0xffffffffu;
     __shared__ BucketSmem S;
     const u32 t = threadIdx.x;
-    if (t == 0 && !DIRECT) S.tile = atomicAdd(ctl + C_TICKET, 1u);
+    if (t == 0 && !DIRECT) S.tile = atomicAdd(head + H_TICKET, 1u);
     if (t < 4) S.and_or[t] = t < 2 ? ALL : 0u;
+    const u32 all = n.get();
+    const bool whole = DIRECT || all <= BK_CAP;
     __syncthreads();
-    const u32 tile = DIRECT ? 0 : S.tile, tiles = DIRECT ? 1 : ctl[C_BUCKETS];
-    if (!DIRECT && (tile >= tiles || ctl[C_FLAGS])) return;
-    const u32 cnt = DIRECT ? n : ctl[counters + tile];
-    u32 *look = ctl + words;
+    const u32 tile = DIRECT ? 0 : S.tile, tiles = whole ? 1 : head[H_BUCKETS];
+    if (!DIRECT && (tile >= tiles || head[H_FLAGS])) return;
+    const u32 cnt = whole ? all : arrays[counters + tile];
+    u32 *look = arrays + words;
     if (!UNIQUE && t == 0 && tile > 0) st_relaxed(look + tile, (1u << 30) | cnt);
-    if (!DIRECT) src += (u64)tile * BK_CAP;
+    const u64 *src = whole ? input : slots + (u64)tile * BK_CAP;
     u64 k[BK_KPT];
     u64 a = KEY_MAX, o = 0;
     const bool on = (t & ~31u) * BK_KPT < cnt;
@@ -608,7 +623,7 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
         u32 v[BK_KPT];
 #pragma unroll
         for (int i = 0; i < BK_KPT; i++) v[i] = (u32)k[i];  // KEY_MAX beyond cnt
-        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, ctl, out, count_empties, S,
+        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
                                       [=](u32 x) { return make64(high, x); });
     } else if (low + __popc(vary_hi) <= 32) {
         if (t == 0) plan_moves(vary_lo, &S.lo);
@@ -621,10 +636,10 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
 #pragma unroll
             for (int i = 0; i < BK_KPT; i++) v[i] = warp_key(i) < cnt ? narrow_key(k[i], lo, hi, low) : ALL;
         }
-        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, ctl, out, count_empties, S,
+        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
                                       [&](u32 x) { return wide_key(x, S.lo, S.hi, low) | fixed; });
     } else {
-        finish_bucket<UNIQUE, DIRECT>(k, S.wide, S.last64, cnt, tile, tiles, look, ctl, out, count_empties, S,
+        finish_bucket<UNIQUE, DIRECT>(k, S.wide, S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
                                       [](u64 x) { return x; });
     }
 }
@@ -635,8 +650,9 @@ void BucketWorkspace::release(cudaStream_t s)
     dev_free(ctl.p, s);
     dev_free(coarse.p, s);
     dev_free(fine.p, s);
+    dev_free(bounds.p, s);
     ctl = DevBuf<u32>{};
-    coarse = fine = DevBuf<u64>{};
+    coarse = fine = bounds = DevBuf<u64>{};
 }
 
 static bool attributes()
@@ -653,37 +669,109 @@ static bool attributes()
     return done;
 }
 
-template <bool UNIQUE>
-static void launch_buckets(const u64 *src, u32 grid, u32 counters, u32 words, u32 *ctl, u64 *out, bool empties,
-                           cudaStream_t s)
-{
-    bucket_sort_kernel<UNIQUE, false><<<grid, BUCKET_THREADS, 0, s>>>(src, 0, counters, words, ctl, out, empties);
-}
-
 // Sizes of one call.  Two steps from 512 x 1800 keys on: coarse buckets of
 // equal expected size, their space seven sigma above it (a coarse bucket is
 // bounded by 64 samples, or by 8192 / coarse).
-struct BucketPlan {
-    u32 one = 0;          // buckets of the one-step form (0: two steps)
-    u32 coarse = 0, coarse_cap = 0;
-    u32 grid = 0;         // upper bound of the fine buckets
-};
-
 static bool plan_buckets(u64 n, BucketPlan *p)
 {
-    if (n <= (u64)BK_FAN * BK_TARGET) {
-        p->one = p->grid = (u32)((n + BK_TARGET - 1) / BK_TARGET);
-        return true;
+    *p = BucketPlan{};
+    p->n = n;
+    if (n > BUCKET_SORT_KEYS) return false;
+    if (n <= BK_CAP) {
+        p->grid = 1;
+    } else if (n <= (u64)BK_FAN * BK_TARGET) {
+        p->grid = (u32)((n + BK_TARGET - 1) / BK_TARGET);
+    } else {
+        u32 c = (u32)std::ceil(std::sqrt((double)n / BK_TARGET));
+        if (c > BK_COARSE) c = BK_COARSE;
+        const double per = std::min(64.0, (double)BK_SAMPLES / c);
+        const u64 cap = ((u64)((double)n / c * (1.0 + 7.0 / std::sqrt(per))) + 63) / 64 * 64;
+        if (cap > (u64)BK_FAN * BK_TARGET) return false;  // more buckets than one step tells apart
+        p->coarse = c;
+        p->coarse_cap = (u32)cap;
+        p->grid = (u32)(n / BK_TARGET) + c;
     }
-    u32 c = (u32)std::ceil(std::sqrt((double)n / BK_TARGET));
-    if (c > BK_COARSE) c = BK_COARSE;
-    const double per = std::min(64.0, (double)BK_SAMPLES / c);
-    const u64 cap = ((u64)((double)n / c * (1.0 + 7.0 / std::sqrt(per))) + 63) / 64 * 64;
-    if (cap > (u64)BK_FAN * BK_TARGET) return false;  // more buckets than one step tells apart
-    p->coarse = c;
-    p->coarse_cap = (u32)cap;
-    p->grid = (u32)(n / BK_TARGET) + c;
+    p->words = A_FINE + 2 * p->grid;
     return true;
+}
+
+bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s)
+{
+    u64 words = BUCKET_HEADS * BUCKET_HEAD_WORDS, fine = 0, coarse = 0, bounds = 0;
+    for (int i = 0; i < calls; i++) {
+        BucketPlan &p = plans[i];
+        if (!plan_buckets(n[i], &p)) return false;
+        p.arrays_at = words;
+        words += (p.words + 1) / 2 * 2;
+        if (p.n <= BK_CAP) continue;
+        fine = std::max(fine, (u64)p.grid * BK_CAP);
+        coarse = std::max(coarse, (u64)p.coarse * p.coarse_cap);
+        bounds = std::max(bounds, (u64)BK_FAN * (p.coarse + 1));
+    }
+    w.used_words = words;
+    auto room = [&](auto &b, u64 want) { return (b.p && b.cap >= want) || !want || grow(b, want * 5 / 4, s); };
+    if (!w.host && !CGB_CUDA(cudaHostAlloc((void **)&w.host, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4, cudaHostAllocDefault)))
+        return false;
+    return room(w.ctl, words) && room(w.bounds, bounds) && room(w.fine, fine) && room(w.coarse, coarse) && attributes();
+}
+
+bool bucket_clear(BucketWorkspace &w, cudaStream_t s)
+{
+    return CGB_CUDA(cudaMemsetAsync(w.ctl.p, 0, w.used_words * sizeof(u32), s));
+}
+
+template <bool UNIQUE>
+static void launch_sort(const BucketPlan &p, const u64 *keys, KeyCount kc, u64 *out, bool empties, u32 *head, u32 *arrays,
+                        BucketWorkspace &w, cudaStream_t s)
+{
+    if (p.n <= BK_CAP && !kc.counted)
+        bucket_sort_kernel<UNIQUE, true><<<1, BUCKET_THREADS, 0, s>>>(keys, kc, nullptr, A_FINE, A_FINE + p.grid, head,
+                                                                      arrays, out, empties);
+    else
+        bucket_sort_kernel<UNIQUE, false><<<p.grid, BUCKET_THREADS, 0, s>>>(keys, kc, w.fine.p, A_FINE, A_FINE + p.grid,
+                                                                            head, arrays, out, empties);
+}
+
+int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,
+                   BucketWorkspace &w, cudaStream_t s)
+{
+    const u32 split_smem = SAMPLE_WORDS * sizeof(u64);
+    u32 *head = w.ctl.p + slot * BUCKET_HEAD_WORDS, *arrays = w.ctl.p + p.arrays_at;
+    const KeyCount kc{(u32)p.n, counted};
+    const u32 tiles = (u32)((p.n + BK_TILE - 1) / BK_TILE);
+    int np = 1;
+    if (p.n > BK_CAP && !p.coarse) {
+        bucket_split_kernel<0><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, 0, 0, head, arrays, w.bounds.p);
+        bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(
+            keys, kc, 0, 1, 0, w.bounds.p, head, arrays, A_FINE, w.fine.p, BK_CAP);
+        np = 2;
+    } else if (p.coarse) {
+        const u32 fine_tiles = (p.coarse_cap + BK_TILE - 1) / BK_TILE;
+        u64 *fine_bounds = w.bounds.p + BK_FAN;
+        bucket_split_kernel<1><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, p.coarse, 0, head, arrays, w.bounds.p);
+        bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(
+            keys, kc, 0, 1, p.coarse, w.bounds.p, head, arrays, A_COARSE, w.coarse.p, p.coarse_cap);
+        bucket_split_kernel<2><<<p.coarse, SPLIT_THREADS, split_smem, s>>>(w.coarse.p, kc, p.coarse, p.coarse_cap, head,
+                                                                           arrays, fine_bounds);
+        bucket_partition_kernel<true><<<p.coarse * fine_tiles, PART_THREADS, sizeof(PartSmem), s>>>(
+            w.coarse.p, kc, p.coarse_cap, fine_tiles, 0, fine_bounds, head, arrays, A_FINE, w.fine.p, BK_CAP);
+        np = 3;
+    }
+    if (unique) launch_sort<true>(p, keys, kc, out, empties, head, arrays, w, s);
+    else launch_sort<false>(p, keys, kc, out, false, head, arrays, w, s);
+    kstats().launches += np == 1 ? 0 : np == 2 ? 2 : 4;
+    return np;
+}
+
+BucketResult bucket_result(const BucketWorkspace &w, int slot)
+{
+    const u32 *h = w.host + slot * BUCKET_HEAD_WORDS;
+    BucketResult r;
+    r.error = h[H_FLAGS] & ~BK_OVERFLOW;
+    r.overflow = (h[H_FLAGS] & BK_OVERFLOW) != 0;
+    memcpy(&r.count, h + H_COUNT, 8);
+    memcpy(&r.empties, h + H_EMPTIES, 8);
+    return r;
 }
 
 bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 *empties, int *passes,
@@ -691,66 +779,25 @@ bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 
 {
     *done = false;
     BucketPlan p;
-    if (n < 2 || n > BUCKET_SORT_KEYS || (n > BK_CAP && !plan_buckets(n, &p))) return true;
-    if (!attributes()) return false;
-    if (!w.host && !CGB_CUDA(cudaHostAlloc((void **)&w.host, 32, cudaHostAllocDefault))) return false;
-    const bool direct = n <= BK_CAP;
-    const u32 words = C_FINE + p.grid, total_words = words + p.grid;
-    // boundaries behind the control words
-    const u64 bounds_at = (total_words + 1) / 2 * 2, bound_words = 2ull * BK_FAN * (p.coarse + 1);
     // without room for the buckets the caller's digit passes take over
-    if ((!w.ctl.p || w.ctl.cap < bounds_at + bound_words) && !grow(w.ctl, (bounds_at + bound_words) * 5 / 4, s)) return true;
-    if (!direct) {
-        const u64 fine = (u64)p.grid * BK_CAP, coarse = (u64)p.coarse * p.coarse_cap;
-        if ((!w.fine.p || w.fine.cap < fine) && !grow(w.fine, fine * 5 / 4, s)) return true;
-        if (coarse && (!w.coarse.p || w.coarse.cap < coarse) && !grow(w.coarse, coarse * 5 / 4, s)) return true;
-    }
-    const u32 split_smem = SAMPLE_WORDS * sizeof(u64);
-    u32 *ctl = w.ctl.p;
-    u64 *bounds = (u64 *)(ctl + bounds_at);
-    const u64 *src = keys;
-    if (!CGB_CUDA(cudaMemsetAsync(ctl, 0, (direct ? C_COARSE : total_words) * sizeof(u32), s))) return false;
+    if (n < 2 || !bucket_prepare(&n, 1, &p, w, s)) return true;
+    if (!bucket_clear(w, s)) return false;
     kclock().begin(s, &kstats().onesweep_ms);
-    int np = 1;
-    if (direct) {
-        if (unique) bucket_sort_kernel<true, true><<<1, BUCKET_THREADS, 0, s>>>(keys, (u32)n, 0, 0, ctl, out, empties != nullptr);
-        else bucket_sort_kernel<false, true><<<1, BUCKET_THREADS, 0, s>>>(keys, (u32)n, 0, 0, ctl, out, 0);
-    } else {
-        if (p.one) {
-            bucket_split_kernel<0><<<1, SPLIT_THREADS, split_smem, s>>>(src, (u32)n, p.one, 0, ctl, bounds);
-            bucket_partition_kernel<false><<<(u32)((n + BK_TILE - 1) / BK_TILE), PART_THREADS, sizeof(PartSmem), s>>>(
-                src, (u32)n, 0, 1, p.one, bounds, ctl, C_FINE, w.fine.p, BK_CAP);
-            np = 2;
-        } else {
-            const u32 tiles = (p.coarse_cap + BK_TILE - 1) / BK_TILE;
-            bucket_split_kernel<1><<<1, SPLIT_THREADS, split_smem, s>>>(src, (u32)n, p.coarse, 0, ctl, bounds);
-            bucket_partition_kernel<false><<<(u32)((n + BK_TILE - 1) / BK_TILE), PART_THREADS, sizeof(PartSmem), s>>>(
-                src, (u32)n, 0, 1, p.coarse, bounds, ctl, C_COARSE, w.coarse.p, p.coarse_cap);
-            u64 *fine_bounds = bounds + BK_FAN;
-            bucket_split_kernel<2><<<p.coarse, SPLIT_THREADS, split_smem, s>>>(w.coarse.p, 0, p.coarse, p.coarse_cap, ctl,
-                                                                               fine_bounds);
-            bucket_partition_kernel<true><<<p.coarse * tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-                w.coarse.p, 0, p.coarse_cap, tiles, 0, fine_bounds, ctl, C_FINE, w.fine.p, BK_CAP);
-            kstats().launches += 2;
-            np = 3;
-        }
-        if (unique) launch_buckets<true>(w.fine.p, p.grid, C_FINE, words, ctl, out, empties != nullptr, s);
-        else launch_buckets<false>(w.fine.p, p.grid, C_FINE, words, ctl, out, false, s);
-        kstats().launches += 2;
-    }
+    const int np = bucket_enqueue(p, 0, keys, nullptr, out, unique, empties != nullptr, w, s);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError()) ||
-        !CGB_CUDA(cudaMemcpyAsync(w.host, ctl, 32, cudaMemcpyDeviceToHost, s)) || !CGB_CUDA(cudaStreamSynchronize(s)))
+        !CGB_CUDA(cudaMemcpyAsync(w.host, w.ctl.p, BUCKET_HEAD_WORDS * 4, cudaMemcpyDeviceToHost, s)) ||
+        !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
     kclock().flush();
-    const u32 flags = w.host[C_FLAGS];
-    if (flags & ~BK_OVERFLOW) {
-        set_error("bucket_sort: device error " + err_string(flags & ~BK_OVERFLOW));
+    const BucketResult r = bucket_result(w, 0);
+    if (r.error) {
+        set_error("bucket_sort: device error " + err_string(r.error));
         return false;
     }
-    if (flags) return true;
-    memcpy(n_out, w.host + C_COUNT, 8);
-    if (empties) memcpy(empties, w.host + C_EMPTIES, 8);
+    if (r.overflow) return true;
+    *n_out = r.count;
+    if (empties) *empties = r.empties;
     kstats().onesweep_bytes += 16 * n * np;
     kstats().onesweep_launches += np;
     if (passes) *passes = np;

@@ -122,6 +122,7 @@ struct GenBuffers {
     // move step's unique pass; unknown after a sliced move step
     static constexpr u64 UNKNOWN = ~0ull;
     u64 moved_empties = UNKNOWN, prev_empties = 0;
+    double spawn_ratio = 16;   // spawns per board of S in the last layer step
 };
 
 struct Engine {
@@ -157,6 +158,10 @@ struct Engine {
     bool move_layer(const u64 *d_in, u64 n, GenTimes *tm);
     bool spawn_streams(GenTimes *tm);   // g.u2, g.u4: the sorted unique 2- and 4-spawns of g.moved
     bool spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm);
+    // layers of at most so many boards to move take quick_step: above, kernels
+    // of a millisecond hide the waits
+    static constexpr u64 QUICK_BOARDS = 1u << 21;
+    bool quick_step(GenTimes *tm, bool *moved_done, bool *done);
     bool next_inputs(GenTimes *tm);     // g.S from the spawns of g.moved and g.prev
     bool sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
                           u64 *empties = nullptr);

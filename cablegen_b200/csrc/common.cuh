@@ -54,12 +54,14 @@ KernelStats &kstats();
 class KClock {
   public:
     void begin(cudaStream_t s, double *acc);
+    void next(cudaStream_t s, double *acc);  // end and begin with one event
     void end(cudaStream_t s);
     void flush();  // call after the stream has been synchronised
   private:
     struct Pending {
         cudaEvent_t a, b;
         double *acc;
+        bool last;  // b is not the next entry's a
     };
     cudaEvent_t take();
     std::vector<cudaEvent_t> free_;

@@ -18,6 +18,7 @@
 #include "engine.h"
 #include "cgb_engine.h"
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include <unordered_map>
 
@@ -90,8 +91,17 @@ void KClock::end(cudaStream_t s)
     if (!open_) return;
     cudaEvent_t b = take();
     cudaEventRecord(b, s);
-    pend_.push_back({open_, b, open_acc_});
+    pend_.push_back({open_, b, open_acc_, true});
     open_ = nullptr;
+}
+void KClock::next(cudaStream_t s, double *acc)
+{
+    cudaEvent_t b = take();
+    cudaEventRecord(b, s);
+    pend_.push_back({open_, b, open_acc_, false});
+    open_ = b;
+    open_acc_ = acc;
+    kstats().launches++;
 }
 void KClock::flush()
 {
@@ -99,7 +109,7 @@ void KClock::flush()
         float ms = 0;
         if (cudaEventElapsedTime(&ms, p.a, p.b) == cudaSuccess && p.acc) *p.acc += ms;
         free_.push_back(p.a);
-        free_.push_back(p.b);
+        if (p.last) free_.push_back(p.b);
     }
     pend_.clear();
 }
@@ -511,6 +521,89 @@ bool Engine::next_inputs(GenTimes *tm)
     return true;
 }
 
+// One layer step without a wait inside: every size but |S| stays on the device,
+// where the next kernel reads it, and the sizes come back in one copy at the end.
+// A small layer's kernels take 10-20 us each, and three waits with their launches
+// behind them cost as much again.  The spawns' room is a guess from the last layer;
+// where it or a bucket overflows, *done stays false or only the moved layer is
+// taken, and the step with waits does the rest.
+bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
+{
+    *moved_done = *done = false;
+    cudaStream_t s = stream;
+    GenBuffers &g = gen;
+    const u64 n = g.S.n;
+    if (n == 0 || n > QUICK_BOARDS || g.u4.n || !bucket_sorts() || 4 * n > max_sort_keys) return true;
+    const u64 room = std::max<u64>(1 << 14, (u64)(1.5 * (double)n * g.spawn_ratio));
+    if (room > max_sort_keys) return true;
+    const u64 sizes[2] = {4 * n, room};
+    BucketPlan plans[2];
+    if (!reserve(g.a, 4 * n, s) || !reserve(g.b, 4 * n, s) || !reserve(g.c[0], room, s) || !reserve(g.c[1], room, s))
+        return false;
+    BucketWorkspace &w = ws.buckets;
+    if (!bucket_prepare(sizes, 2, plans, w, s)) return true;
+    // the third head: counts of moves, raw moves and spawns, error word
+    constexpr u32 OWN = 2 * BUCKET_HEAD_WORDS;
+    u64 *own = (u64 *)(w.ctl.p + OWN);
+    u32 *err = w.ctl.p + OWN + 6;
+    u32 *const h0 = w.ctl.p;
+    SpawnSource two{g.b.p, 4 * n, 1, 0, (u64 *)(h0 + BUCKET_COUNT_AT)}, four{g.prev.p, g.prev.n, 2, 0};
+    if (!bucket_clear(w, s)) return false;
+    kclock().begin(s, &kstats().expand_ms);
+    if (!expand_moves_enqueue(g.S.p, n, g.a.p, 4 * n, rt, prune_params(), own, own + 1, err, s, filter, plan)) return false;
+    kclock().next(s, &kstats().onesweep_ms);
+    const int np0 = bucket_enqueue(plans[0], 0, g.a.p, own, g.b.p, true, true, w, s);
+    kclock().next(s, &kstats().spawn_ms);
+    if (!expand_next_enqueue(two, four, g.c[0].p, room, own + 2, err, s, plan)) return false;
+    kclock().next(s, &kstats().onesweep_ms);
+    const int np1 = bucket_enqueue(plans[1], 1, g.c[0].p, own + 2, g.c[1].p, true, false, w, s);
+    kclock().end(s);
+    if (!CGB_CUDA(cudaGetLastError()) ||
+        !CGB_CUDA(cudaMemcpyAsync(w.host, w.ctl.p, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4, cudaMemcpyDeviceToHost, s)) ||
+        !sync())
+        return false;
+    kclock().flush();
+    const BucketResult moves = bucket_result(w, 0), next = bucket_result(w, 1);
+    u64 counts[3];
+    memcpy(counts, w.host + OWN, sizeof counts);
+    const u32 e = w.host[OWN + 6] & ~ERR_CAPACITY, bad = e | moves.error | next.error;
+    if (bad) {
+        set_error("layer step: device error " + err_string(bad));
+        return false;
+    }
+    if (moves.overflow) return true;
+    KernelStats &k = kstats();
+    auto sorted = [&](u64 keys, int passes) {
+        k.onesweep_bytes += 16 * keys * passes;
+        k.onesweep_launches += passes;
+        if (tm) {
+            tm->sorted_keys += keys;
+            tm->sort_passes += (u64)passes * keys;
+        }
+    };
+    k.expand_bytes += 8 * (n + counts[0]);
+    k.moves_raw += counts[1];
+    k.moves_kept += counts[0];
+    sorted(counts[0], np0);
+    std::swap(g.b, g.moved);
+    g.moved.n = moves.count;
+    g.moved_empties = moves.empties;
+    *moved_done = true;
+    const u64 total = g.moved_empties + g.prev_empties;
+    g.spawn_ratio = std::max(1.0, (double)total / (double)n);
+    if (total > room || next.overflow) return true;
+    if (counts[2] != total) {
+        set_error("layer step: " + std::to_string(counts[2]) + " spawns written, " + std::to_string(total) + " expected");
+        return false;
+    }
+    k.spawn_bytes += 8 * (g.moved.n + g.prev.n + total);
+    sorted(total, np1);
+    std::swap(g.S, g.c[1]);
+    g.S.n = next.count;
+    *done = true;
+    return true;
+}
+
 bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, LayerSink &sink, GenTimes *tm,
                       const u64 *h_carry, u64 n_carry)
 {
@@ -522,12 +615,14 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
     g.S.n = n_init;
     g.u4.n = n_carry;
     g.prev.n = g.prev_empties = 0;
+    g.spawn_ratio = 16;
     // canonical layer boards share the 0xf mask of the canonical first board (fixed
     // formation cells); the kernels check every board against it
     plan = (n_init && !filter.fid) ? make_canon_plan(canonical(h_initial[0]), rules.free_formation != 0) : CanonPlan{};
     bool ok = true;
     for (int layer = start; layer <= end && ok; layer += 2) {
-        ok = move_layer(g.S.p, g.S.n, tm) && next_inputs(tm);
+        bool moved = false, next = false;
+        ok = quick_step(tm, &moved, &next) && (moved || move_layer(g.S.p, g.S.n, tm)) && (next || next_inputs(tm));
         if (!ok) break;
         if (tm) tm->boards += g.moved.n;
         const bool carry = sink.wants_carry();

@@ -42,12 +42,37 @@ void drop(DevBuf<T> &b, cudaStream_t s)
 
 // ---- bucket sort (bucketsort.cu) ------------------------------------------
 constexpr u64 BUCKET_SORT_KEYS = 160ull << 20;  // the most keys one call takes (512 x 512 buckets hold them)
+constexpr u32 BUCKET_HEADS = 3, BUCKET_HEAD_WORDS = 16;  // heads: two sorts, and words of the caller's own
 struct BucketWorkspace {
-    DevBuf<u32> ctl;           // control words, bucket counts, look-back words, boundaries
+    DevBuf<u32> ctl;           // the heads, then each sort's bucket counts and look-back words
+    DevBuf<u64> bounds;        // bucket boundaries
     DevBuf<u64> coarse, fine;  // the buckets
-    u32 *host = nullptr;       // pinned copy of the first control words
+    u64 used_words = 0;
+    u32 *host = nullptr;       // pinned copy of the heads
     void release(cudaStream_t s);
 };
+constexpr u32 BUCKET_COUNT_AT = 4;  // head word of the 64-bit number of keys written
+struct BucketPlan {
+    u64 n = 0;              // keys at most
+    u32 coarse = 0, coarse_cap = 0;  // two steps: coarse buckets and their space
+    u32 grid = 0;           // buckets at most
+    u64 words = 0, arrays_at = 0;
+};
+struct BucketResult {
+    u64 count = 0, empties = 0;
+    u32 error = 0;
+    bool overflow = false;  // nothing was written: the digit passes take the input
+};
+// The parts of bucket_sort, for callers that put several sorts into one stream
+// without a wait: plans and room for `calls` sorts of at most n[i] keys (false:
+// too many keys or no memory), one clear of all control words, the launches of
+// one sort (the number of keys read from *counted where that is not null;
+// returns the passes), and, once the heads have been copied to w.host, the result.
+bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s);
+bool bucket_clear(BucketWorkspace &w, cudaStream_t s);
+int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,
+                   BucketWorkspace &w, cudaStream_t s);
+BucketResult bucket_result(const BucketWorkspace &w, int slot);
 // out[0, *n_out) = keys[0, n) ascending, without repeats when `unique`; out must
 // not alias keys, which are only read.  empties (optional): the empty cells over
 // the keys kept.  *done = false (and nothing written) where the sort by buckets
@@ -78,6 +103,7 @@ int sort_plan(const u32 *hist_host, u64 n, int *digits);
 bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s,
                SortStats *stats = nullptr);
 // reports device errors a sort left behind (when no unique_keys follows)
+bool bucket_sorts();  // whether the "sort_variant" option lets the bucket sort run
 bool sort_check(SortWorkspace &ws, cudaStream_t s);
 // sort_keys then unique_keys, in one pass over the buckets where they apply:
 // *out points at keys or tmp
@@ -115,6 +141,10 @@ bool partition_by_formation(const u64 *in, u64 n, u64 *out, const unsigned char 
 bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const DeviceRowTable &t,
                   const PruneParams &p, Counters &c, cudaStream_t s, FormationFilter ff = FormationFilter{},
                   const CanonPlan &plan = CanonPlan{});
+// its launch alone: the counts (results, and legal unpruned moves before the
+// repeats went) and errors are added to *count, *raw and *err
+bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceRowTable &t, const PruneParams &p,
+                          u64 *count, u64 *raw, u32 *err, cudaStream_t s, FormationFilter ff, const CanonPlan &plan);
 // number of empty cells over all boards (exact size of the spawn streams)
 bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s);
 // one spawn stream: every empty cell of a set of boards filled with `value`
@@ -123,7 +153,12 @@ struct SpawnSource {
     u64 n = 0;
     u32 value = 1;  // 1: a 2 tile, 2: a 4 tile
     u64 total = 0;  // empty cells over the boards
+    const u64 *counted = nullptr;  // where a kernel before this one left the number of boards (n at most)
 };
+// the launch of expand_next alone: the count and errors are added to *count and
+// *err; nothing is written beyond cap
+bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u64 cap, u64 *count, u32 *err,
+                         cudaStream_t s, const CanonPlan &plan);
 // the canonical spawns of both sources, a.total + b.total of them, in one array
 // and without a wait: the kernel's count and error word land in h_check (pinned,
 // 2 words), for check_spawns once the stream has been waited for

@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(256) expand_next_kernel(SpawnSource a, SpawnSo
 {
     __shared__ u32 scan_scratch[33];
     __shared__ u64 base_sh;
+    if (a.counted) a.n = min(a.n, *a.counted);
     // whole blocks of 256 boards of a, then of b
     const u64 blocks_a = (a.n + 255) / 256, blocks = blocks_a + (b.n + 255) / 256;
     for (u64 block = blockIdx.x; block < blocks; block += gridDim.x) {
@@ -390,11 +391,9 @@ static bool check(Counters &c, cudaStream_t s, const char *what)
     return true;
 }
 
-bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const DeviceRowTable &t,
-                  const PruneParams &p, Counters &c, cudaStream_t s, FormationFilter ff, const CanonPlan &plan)
+bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceRowTable &t, const PruneParams &p,
+                          u64 *count, u64 *raw, u32 *err, cudaStream_t s, FormationFilter ff, const CanonPlan &plan)
 {
-    *n_out = 0;
-    if (n == 0) return true;
     static bool attr = false;
     if (!attr) {
         const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -405,9 +404,6 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
             return false;
         attr = true;
     }
-    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d + 5, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
     // the prune table of these parameters, in device memory until they change
     static PruneTable *d_prune = nullptr;
     static PruneParams have{-1, -1, -1, -1};
@@ -426,15 +422,26 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
     const u32 window = (u32)std::max<u64>(1, std::min<u64>((u64)g_move_window, n / (sms * EXP_THREADS * 2)));
     const u64 chunks = (n + (u64)window * EXP_THREADS - 1) / ((u64)window * EXP_THREADS);
     const int grid = (int)std::min<u64>(chunks, sms);
-    kclock().begin(s, &kstats().expand_ms);
     const auto kernel = plan.form == CANON_ONE        ? expand_moves_kernel<CANON_ONE>
                         : plan.form == CANON_DIAGONAL ? expand_moves_kernel<CANON_DIAGONAL>
                         : plan.form == CANON_MIRROR   ? expand_moves_kernel<CANON_MIRROR>
                                                       : expand_moves_kernel<CANON_LIST>;
-    kernel<<<grid, EXP_THREADS, EXP_SMEM, s>>>(in, n, out, cap, c.d, t.move, p, d_prune, c.err, ff, plan, c.d + 5,
-                                               window);
+    kernel<<<grid, EXP_THREADS, EXP_SMEM, s>>>(in, n, out, cap, count, t.move, p, d_prune, err, ff, plan, raw, window);
+    return CGB_CUDA(cudaGetLastError());
+}
+
+bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const DeviceRowTable &t,
+                  const PruneParams &p, Counters &c, cudaStream_t s, FormationFilter ff, const CanonPlan &plan)
+{
+    *n_out = 0;
+    if (n == 0) return true;
+    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s))) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(c.d + 5, 0, sizeof(u64), s))) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
+    kclock().begin(s, &kstats().expand_ms);
+    const bool ok = expand_moves_enqueue(in, n, out, cap, t, p, c.d, c.d + 5, c.err, s, ff, plan);
     kclock().end(s);
-    if (!CGB_CUDA(cudaGetLastError())) return false;
+    if (!ok) return false;
     u64 raw = 0;
     if (!read_count_checked(n_out, c, 0, s, "expand_moves", &raw)) return false;
     kclock().flush();
@@ -460,24 +467,31 @@ bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s)
     return true;
 }
 
+bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u64 cap, u64 *count, u32 *err,
+                         cudaStream_t s, const CanonPlan &plan)
+{
+    const u64 blocks = (a.n + 255) / 256 + (b.n + 255) / 256;
+    if (blocks == 0) return true;
+    const int grid = (int)std::min<u64>(blocks, (u64)sm_count() * 8);
+    const auto kernel = plan.form == CANON_ONE        ? expand_next_kernel<CANON_ONE>
+                        : plan.form == CANON_DIAGONAL ? expand_next_kernel<CANON_DIAGONAL>
+                        : plan.form == CANON_MIRROR   ? expand_next_kernel<CANON_MIRROR>
+                                                      : expand_next_kernel<CANON_LIST>;
+    kernel<<<grid, 256, 0, s>>>(a, b, out, cap, count, err, plan);
+    return CGB_CUDA(cudaGetLastError());
+}
+
 bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters &c, cudaStream_t s,
                  const CanonPlan &plan, u64 *h_check)
 {
     // the count and, 32 words on, the error word
     if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s)) || !CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s)))
         return false;
-    const u64 blocks = (a.n + 255) / 256 + (b.n + 255) / 256, cap = a.total + b.total;
-    if (blocks) {
-        const int grid = (int)std::min<u64>(blocks, (u64)sm_count() * 8);
-        kclock().begin(s, &kstats().spawn_ms);
-        const auto kernel = plan.form == CANON_ONE        ? expand_next_kernel<CANON_ONE>
-                            : plan.form == CANON_DIAGONAL ? expand_next_kernel<CANON_DIAGONAL>
-                            : plan.form == CANON_MIRROR   ? expand_next_kernel<CANON_MIRROR>
-                                                          : expand_next_kernel<CANON_LIST>;
-        kernel<<<grid, 256, 0, s>>>(a, b, out, cap, c.d, c.err, plan);
-        kclock().end(s);
-        if (!CGB_CUDA(cudaGetLastError())) return false;
-    }
+    const u64 cap = a.total + b.total;
+    kclock().begin(s, &kstats().spawn_ms);
+    const bool ok = expand_next_enqueue(a, b, out, cap, c.d, c.err, s, plan);
+    kclock().end(s);
+    if (!ok) return false;
     if (!CGB_CUDA(cudaMemcpyAsync(h_check, c.d, sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
         !CGB_CUDA(cudaMemcpyAsync(h_check + 1, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s)))
         return false;

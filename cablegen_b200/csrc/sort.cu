@@ -1051,6 +1051,8 @@ int sort_plan(const u32 *hist_host, u64 n, int *digits)
     return np;
 }
 
+bool bucket_sorts() { return g_sort_variant == 4; }
+
 static bool digit_sort(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s,
                        SortStats *stats);
 
@@ -1059,7 +1061,7 @@ bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cuda
     *sorted = keys;
     if (stats) *stats = SortStats{};
     if (n <= 1) return true;
-    if (g_sort_variant == 4) {
+    if (bucket_sorts()) {
         bool done = false;
         int passes = 0;
         u64 m = 0;
@@ -1080,7 +1082,7 @@ bool sort_unique_keys(u64 *keys, u64 *tmp, u64 n, u64 **out, u64 *n_out, SortWor
                       SortStats *stats, u64 *empties)
 {
     if (stats) *stats = SortStats{};
-    if (g_sort_variant == 4 && !ws.err_dirty) {
+    if (bucket_sorts() && !ws.err_dirty) {
         bool done = false;
         int passes = 0;
         if (!bucket_sort(keys, n, tmp, true, n_out, empties, &passes, ws.buckets, s, &done)) return false;

@@ -88,6 +88,9 @@ struct AsyncOut {
             if (s.busy && !CGB_CUDA(cudaStreamWaitEvent(main, s.done, 0))) return false;
         return true;
     }
+    // the older of the two requests: its callback runs while the work enqueued
+    // since then keeps the device busy
+    bool finish_older() { return finish(slot[next]); }
     bool drain() { return finish(slot[next]) && finish(slot[next ^ 1]); }
 };
 

@@ -55,7 +55,8 @@ constexpr u32 BK_OVERFLOW = 1u << 16;   // a bucket ran full (beside the ERR_* b
 
 // control words of one sort (u32 indexes): its head, and its arrays, which start
 // with the counts of the coarse buckets
-constexpr u32 H_TICKET = 0, H_FLAGS = 1, H_BUCKETS = 2, H_COUNT = BUCKET_COUNT_AT, H_EMPTIES = 6;
+constexpr u32 H_TICKET = 0, H_FLAGS = 1, H_BUCKETS = 2, H_COUNT = BUCKET_COUNT_AT, H_EMPTIES = 6, H_ZEROS = 8,
+              H_ONES = 10;  // bits that are 0 (1) in some key, each low word first
 constexpr u32 A_COARSE = 0, A_BASE = A_COARSE + BK_COARSE, A_NUM = A_BASE + BK_COARSE, A_FINE = A_NUM + BK_COARSE;
 
 // The number of keys of a call: known on the host, or counted by a kernel before
@@ -616,6 +617,10 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
         for (int i = 0; i < BK_KPT; i++) k[i] = KEY_MAX;
     }
     __syncthreads();
+    if (UNIQUE && t < 4) {
+        const u32 bits = t < 2 ? ~S.and_or[t] : S.and_or[t];
+        if (bits & ~ld_relaxed(head + H_ZEROS + t)) atomicOr(head + H_ZEROS + t, bits);
+    }
     const u32 vary_lo = S.and_or[0] ^ S.and_or[2], vary_hi = S.and_or[1] ^ S.and_or[3];
     const u32 low = __popc(vary_lo);
     if (vary_hi == 0) {
@@ -771,11 +776,15 @@ BucketResult bucket_result(const BucketWorkspace &w, int slot)
     r.overflow = (h[H_FLAGS] & BK_OVERFLOW) != 0;
     memcpy(&r.count, h + H_COUNT, 8);
     memcpy(&r.empties, h + H_EMPTIES, 8);
+    memcpy(&r.bits.all, h + H_ZEROS, 8);
+    memcpy(&r.bits.any, h + H_ONES, 8);
+    r.bits.all = ~r.bits.all;
+    r.bits.known = r.count > 0;
     return r;
 }
 
 bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 *empties, int *passes,
-                 BucketWorkspace &w, cudaStream_t s, bool *done)
+                 BucketWorkspace &w, cudaStream_t s, bool *done, KeyBits *bits)
 {
     *done = false;
     BucketPlan p;
@@ -798,6 +807,7 @@ bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 
     if (r.overflow) return true;
     *n_out = r.count;
     if (empties) *empties = r.empties;
+    if (bits) *bits = r.bits;
     kstats().onesweep_bytes += 16 * n * np;
     kstats().onesweep_launches += np;
     if (passes) *passes = np;

@@ -122,7 +122,19 @@ struct GenBuffers {
     // move step's unique pass; unknown after a sliced move step
     static constexpr u64 UNKNOWN = ~0ull;
     u64 moved_empties = UNKNOWN, prev_empties = 0;
+    KeyBits moved_bits;        // AND and OR of the moved layer, where its sort gave them
     double spawn_ratio = 16;   // spawns per board of S in the last layer step
+};
+
+// device memory of the calls that solve or look up one layer, kept for the next
+// such call up to KEEP bytes an index: allocating and freeing hundreds of MB costs
+// a call more than its copies and launches
+struct OneShot {
+    static constexpr u64 KEEP = 1ull << 30;
+    DevBuf<u64> ws;          // winstates
+    IndexStorage index[2];   // the s+2 and s+4 tables' indexes
+    bool busy = false;       // a call is using it
+    bool drop(cudaStream_t s);  // gives it all back; false if there was nothing to give
 };
 
 struct Engine {
@@ -164,13 +176,15 @@ struct Engine {
     bool quick_step(GenTimes *tm, bool *moved_done, bool *done);
     bool next_inputs(GenTimes *tm);     // g.S from the spawns of g.moved and g.prev
     bool sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
-                          u64 *empties = nullptr);
+                          u64 *empties = nullptr, KeyBits *bits = nullptr);
     bool join(DevBuf<u64> &acc, DevBuf<u64> &run, u64 n);
     // layers start..end from the input set of layer `start`; h_carry = the
     // 4-spawns of layer start-2 still to merge into layer start+2's input
     // (empty for a fresh sweep, the checkpointed set when resuming)
     bool generate(const u64 *h_initial, u64 n_init, int start, int end, LayerSink &sink, GenTimes *tm,
                   const u64 *h_carry = nullptr, u64 n_carry = 0);
+    OneShot one_shot;
+    void end_one_shot();     // keeps what may be kept
     void release_buffers();
 };
 

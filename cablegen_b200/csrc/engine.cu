@@ -127,6 +127,12 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
 {
     *p = nullptr;
     if (bytes == 0) bytes = 256;
+    auto over_cap = [&] {
+        std::lock_guard<std::mutex> g(g_mem_mu);
+        return g_dev_mem_cap && g_mem_held + bytes > g_dev_mem_cap;
+    };
+    // what one-layer calls keep goes first
+    if (over_cap()) Engine::get().one_shot.drop(s);
     {
         std::lock_guard<std::mutex> g(g_mem_mu);
         if (g_dev_mem_cap && g_mem_held + bytes > g_dev_mem_cap) {
@@ -142,6 +148,7 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
         // freed blocks of other sizes may still sit in the pool: return them
         // to the device and retry once
         cudaGetLastError();
+        Engine::get().one_shot.drop(s);
         cudaStreamSynchronize(s);
         int dev = 0;
         cudaGetDevice(&dev);
@@ -371,12 +378,12 @@ static bool reserve(DevBuf<u64> &b, u64 n, cudaStream_t s)
 // sort + unique of n raw keys in x (y = scratch); returns the buffer holding
 // the unique keys (the other one is left free)
 bool Engine::sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
-                              u64 *empties)
+                              u64 *empties, KeyBits *bits)
 {
     cudaStream_t s = stream;
     u64 *u = x.p;
     SortStats st;
-    if (!sort_unique_keys(x.p, y.p, n, &u, nu, ws, s, &st, empties)) return false;
+    if (!sort_unique_keys(x.p, y.p, n, &u, nu, ws, s, &st, empties, bits)) return false;
     if (tm) {
         tm->sorted_keys += n;
         tm->sort_passes += (u64)st.passes * n;
@@ -416,6 +423,7 @@ bool Engine::move_layer(const u64 *d_in, u64 n, GenTimes *tm)
     const u64 m0 = chunked ? slice : n;
     if (chunked) g.moved.n = 0;
     g.moved_empties = GenBuffers::UNKNOWN;
+    g.moved_bits = KeyBits{};
     for (u64 off = 0; off < n || (n == 0 && off == 0); off += m0) {
         const u64 m = std::min(m0, n - off);
         if (!reserve(g.a, 4 * m0, s) || !reserve(g.b, 4 * m0, s)) return false;
@@ -423,7 +431,7 @@ bool Engine::move_layer(const u64 *d_in, u64 n, GenTimes *tm)
         if (!expand_moves(d_in + off, m, g.a.p, 4 * m, &nr, rt, prune_params(), ctr, s, filter, plan)) return false;
         u64 nu = 0, empties = 0;
         DevBuf<u64> *u = nullptr;
-        if (!sort_unique_step(g.a, g.b, nr, &nu, &u, tm, chunked ? nullptr : &empties)) return false;
+        if (!sort_unique_step(g.a, g.b, nr, &nu, &u, tm, chunked ? nullptr : &empties, chunked ? nullptr : &g.moved_bits)) return false;
         if (!chunked) {
             std::swap(*u, g.moved);   // the layer; the old layer buffer becomes scratch
             g.moved.n = nu;
@@ -588,6 +596,7 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
     std::swap(g.b, g.moved);
     g.moved.n = moves.count;
     g.moved_empties = moves.empties;
+    g.moved_bits = moves.bits;
     *moved_done = true;
     const u64 total = g.moved_empties + g.prev_empties;
     g.spawn_ratio = std::max(1.0, (double)total / (double)n);
@@ -637,12 +646,34 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
     return ok;
 }
 
+bool OneShot::drop(cudaStream_t s)
+{
+    if (busy || !(ws.p || index[0].p || index[1].p)) return false;
+    cgb::drop(ws, s);
+    for (IndexStorage &x : index) {
+        dev_free(x.p, s);
+        x = IndexStorage{};
+    }
+    return true;
+}
+
+void Engine::end_one_shot()
+{
+    one_shot.busy = false;
+    for (IndexStorage &x : one_shot.index)
+        if (x.bytes > OneShot::KEEP) {
+            dev_free(x.p, stream);
+            x = IndexStorage{};
+        }
+}
+
 void Engine::release_buffers()
 {
     GenBuffers &g = gen;
     for (DevBuf<u64> *b : {&g.a, &g.b, &g.c[0], &g.c[1], &g.S, &g.u2, &g.u4, &g.moved, &g.prev, &g.t})
         drop(*b, stream);
     ws.buckets.release(stream);
+    one_shot.drop(stream);
 }
 
 }  // namespace cgb

@@ -41,6 +41,11 @@ void drop(DevBuf<T> &b, cudaStream_t s)
 }
 
 // ---- bucket sort (bucketsort.cu) ------------------------------------------
+// AND and OR over a set of keys
+struct KeyBits {
+    u64 all = 0, any = 0;
+    bool known = false;
+};
 constexpr u64 BUCKET_SORT_KEYS = 160ull << 20;  // the most keys one call takes (512 x 512 buckets hold them)
 constexpr u32 BUCKET_HEADS = 3, BUCKET_HEAD_WORDS = 16;  // heads: two sorts, and words of the caller's own
 struct BucketWorkspace {
@@ -60,6 +65,7 @@ struct BucketPlan {
 };
 struct BucketResult {
     u64 count = 0, empties = 0;
+    KeyBits bits;           // of the keys (unique sorts)
     u32 error = 0;
     bool overflow = false;  // nothing was written: the digit passes take the input
 };
@@ -79,7 +85,7 @@ BucketResult bucket_result(const BucketWorkspace &w, int slot);
 // does not apply: too many keys, no memory for the buckets, or keys that repeat
 // too often.
 bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 *empties, int *passes,
-                 BucketWorkspace &w, cudaStream_t s, bool *done);
+                 BucketWorkspace &w, cudaStream_t s, bool *done, KeyBits *bits = nullptr);
 
 // ---- sort / unique / merge (sort.cu) ------------------------------------
 struct SortWorkspace {
@@ -108,7 +114,7 @@ bool sort_check(SortWorkspace &ws, cudaStream_t s);
 // sort_keys then unique_keys, in one pass over the buckets where they apply:
 // *out points at keys or tmp
 bool sort_unique_keys(u64 *keys, u64 *tmp, u64 n, u64 **out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
-                      SortStats *stats = nullptr, u64 *empties = nullptr);
+                      SortStats *stats = nullptr, u64 *empties = nullptr, KeyBits *bits = nullptr);
 // out must not alias in
 // empties (optional): the number of empty cells over the kept keys
 bool unique_keys(const u64 *in, u64 n, u64 *out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
@@ -203,6 +209,8 @@ struct LayerIndex {
     const void *slots = nullptr;  // cap slots of {u64 key, u64 value bits}; key 0 = empty
     u64 cap = 0;
     CompactHash ch;               // ch.on: cap (a power of two) 8-byte slots instead
+    bool unchecked = false;       // begun, its error word not looked at yet
+    int slot = 0;                 // which error word
 };
 
 // device storage owned by one index (reused across layers)
@@ -220,7 +228,23 @@ u64 hash_capacity(u64 n);
 bool solve_prepare();  // one-time kernel attributes (call before a capture)
 bool build_hash_enqueue(LayerIndex &ix, int vbytes, void *slots, u64 cap, u32 *err, cudaStream_t s);
 
-// builds ix (keys/vals/n already set) of the requested kind; vbytes = 8 or 4
+// builds ix (keys/vals/n already set) of the requested kind; vbytes = 8 or 4.
+// index_begin launches the build: kernels behind it on the stream may use ix;
+// index_finish waits for it and, where a build gave up (an overflow list or a
+// probe distance ran out), builds the index another way (*again, if given: what
+// used ix since has to run once more).  Indexes between the two have slots of
+// their own.  bits: AND and OR of the keys, or unknown
+constexpr int INDEX_SLOTS = 2;
+bool index_begin(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c, cudaStream_t s,
+                 const KeyBits &bits = KeyBits{}, int slot = 0);
+bool index_finish(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s, bool *again = nullptr);
+// AND and OR of two sets of keys (bits[0], bits[1]) and a key to be read with them
+// (into bits[2].any; first may be null), behind one wait
+struct KeySet {
+    const u64 *keys = nullptr;
+    u64 n = 0;
+};
+bool key_bits(const KeySet &a, const KeySet &b, KeyBits *bits, const u64 *first, Counters &c, cudaStream_t s);
 bool build_index(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c,
                  cudaStream_t s);
 // the value of each of m boards (canonicalised first when canon) in an indexed
@@ -237,6 +261,13 @@ bool solve_layer_f64(const u64 *keys, u64 n, double *out, const LayerIndex &t2, 
 bool solve_layer_f32(const u64 *keys, u64 n, float *out, const LayerIndex &t2, const LayerIndex &t4,
                      const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
                      const CanonPlan &plan = CanonPlan{});
+
+// the same without a wait; the probes are counted on the device until
+// solve_collect (after which the stream is idle) adds them to the statistics
+bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
+                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
+                        const CanonPlan &plan);
+bool solve_collect(Counters &c, cudaStream_t s);
 
 // ---- resident layers ------------------------------------------------------
 // Resident layers of a sweep.  Layers are appended during generation and

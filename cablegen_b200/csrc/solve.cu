@@ -421,7 +421,7 @@ constexpr int item_smem() { return TABLE_BYTES_S + ITEM_WARPS * (ITEM_MAX * 2 + 
 template <typename V, int FORM>
 __global__ void __launch_bounds__(ITEM_THREADS, 1)
     solve_items_kernel(const u64 *__restrict__ keys, u64 n, V *__restrict__ out, DevTable<V> t2, DevTable<V> t4,
-                       SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan)
+                       SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan, u32 per)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     stage_table_s(smem, g_move);
@@ -430,10 +430,10 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
     unsigned short *items = (unsigned short *)(smem + TABLE_BYTES_S) + warp * ITEM_MAX;  // (lane << 4) | cell
     V *best_sh = (V *)(smem + TABLE_BYTES_S + ITEM_WARPS * ITEM_MAX * 2) + warp * 64;   // [2][32]
     u32 probes = 0;
-    const u64 stride = (u64)gridDim.x * ITEM_THREADS;
-    for (u64 base = (u64)blockIdx.x * ITEM_THREADS + warp * 32; base < n; base += stride) {
+    const u64 stride = (u64)gridDim.x * ITEM_WARPS * per;
+    for (u64 base = ((u64)blockIdx.x * ITEM_WARPS + warp) * per; base < n; base += stride) {
         const u64 i = base + lane;
-        const bool active = i < n;
+        const bool active = lane < (int)per && i < n;
         const u64 b = active ? keys[i] : 0;
         const bool sat = active && satisfied(b, r);
         u64 e = (active && !sat) ? empty_mask(b) : 0;
@@ -511,21 +511,23 @@ __global__ void hash_build_kernel(const u64 *__restrict__ keys, const V *__restr
     }
 }
 
-__global__ void key_bits_kernel(const u64 *__restrict__ keys, u64 n, unsigned long long *and_or)
+// AND and OR over the keys, as the bits that are 0 in some key (bits[0]) and 1 in
+// some key (bits[1]), which start at zero
+__global__ void key_bits_kernel(const u64 *__restrict__ keys, u64 n, unsigned long long *bits)
 {
-    u64 a = ~0ull, o = 0;
+    u64 z = 0, o = 0;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
         const u64 k = keys[i];
-        a &= k;
+        z |= ~k;
         o |= k;
     }
     for (int d = 16; d; d >>= 1) {
-        a &= __shfl_xor_sync(0xffffffffu, a, d);
+        z |= __shfl_xor_sync(0xffffffffu, z, d);
         o |= __shfl_xor_sync(0xffffffffu, o, d);
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAnd(and_or, (unsigned long long)a);
-        atomicOr(and_or + 1, (unsigned long long)o);
+        atomicOr(bits, (unsigned long long)z);
+        atomicOr(bits + 1, (unsigned long long)o);
     }
 }
 
@@ -640,9 +642,10 @@ __global__ void __launch_bounds__(512) region_build_kernel(const ulonglong2 *__r
 }
 
 // the overflow keys, inserted into the finished table by the atomic linear probe
-__global__ void overflow_insert_kernel(const ulonglong2 *__restrict__ over, u32 n, ulonglong2 *slots, u64 cap,
-                                       u32 *err)
+__global__ void overflow_insert_kernel(const ulonglong2 *__restrict__ over, const u32 *n_over, u32 max_over,
+                                       ulonglong2 *slots, u64 cap, u32 *err)
 {
+    const u32 n = min(*n_over, max_over);
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const ulonglong2 e = over[i];
         u64 s = home_pair(e.x, cap);
@@ -680,53 +683,65 @@ static bool ensure_storage(IndexStorage &st, u64 bytes, cudaStream_t s)
     return true;
 }
 
-int g_hash_compact = 1;  // FP32 hash tables in 8-byte slots where the keys allow it
-
-// plans and builds the 8-byte-slot index of an FP32 layer: AND/OR of the keys
-// give the constant bytes; the table is the power of two at or above twice the
-// layer; the tag holds the remainder bits (at most 26) and the probe distance.
-// Leaves ix.kind == INDEX_BISECT (nothing built) when the keys vary in too many
-// bytes or a key would sit further from home than the tag can say.
-static bool build_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStream_t s)
+bool key_bits(const KeySet &a, const KeySet &b, KeyBits *bits, const u64 *first, Counters &c, cudaStream_t s)
 {
-    unsigned long long init[2] = {~0ull, 0ull};
-    if (!CGB_CUDA(cudaMemcpyAsync(c.d + 3, init, 16, cudaMemcpyHostToDevice, s))) return false;
-    key_bits_kernel<<<grid_for(ix.n, 256, 8), 256, 0, s>>>(ix.keys, ix.n, (unsigned long long *)(c.d + 3));
-    u64 ao[2];
-    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(ao, c.d + 3, 16, cudaMemcpyDeviceToHost, s)) ||
+    // device words 16..19: the two sets' bits, 20: the first key of *first
+    static u64 *host = nullptr;
+    if (!host && !CGB_CUDA(cudaHostAlloc((void **)&host, 5 * sizeof(u64), cudaHostAllocDefault))) return false;
+    u64 *d = c.d + 16;
+    if (!CGB_CUDA(cudaMemsetAsync(d, 0, 4 * sizeof(u64), s))) return false;
+    if (first && !CGB_CUDA(cudaMemcpyAsync(d + 4, first, sizeof(u64), cudaMemcpyDeviceToDevice, s))) return false;
+    if (a.n) key_bits_kernel<<<grid_for(a.n, 256, 8), 256, 0, s>>>(a.keys, a.n, (unsigned long long *)d);
+    if (b.n) key_bits_kernel<<<grid_for(b.n, 256, 8), 256, 0, s>>>(b.keys, b.n, (unsigned long long *)(d + 2));
+    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(host, d, 5 * sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
         !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
+    for (int i = 0; i < 2; i++)
+        if (i ? b.n : a.n) bits[i] = KeyBits{~host[2 * i], host[2 * i + 1], true};
+    if (first) bits[2].any = host[4];
+    return true;
+}
+
+int g_hash_compact = 1;  // FP32 hash tables in 8-byte slots where the keys allow it
+
+// a begun build's error word, on the device and its pinned copy, by ix.slot
+static u32 *h_index_err = nullptr;
+static u32 *index_err(const LayerIndex &ix, Counters &c) { return (u32 *)(c.d + 40 + ix.slot); }
+
+// launches the build of the 8-byte-slot index of an FP32 layer: AND/OR of the keys
+// give the constant bytes; the table is the power of two at or above twice the
+// layer; the tag holds the remainder bits (at most 26) and the probe distance.
+// Leaves ix.kind == INDEX_BISECT (nothing launched) when the keys vary in too
+// many bytes.
+static bool begin_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStream_t s, KeyBits bits)
+{
+    if (!bits.known && !key_bits(KeySet{ix.keys, ix.n}, KeySet{}, &bits, nullptr, c, s)) return false;
     int cbits = 0;
-    const CompactHash ch = plan_compact(ao[0], ao[1], ix.n, &cbits);
+    const CompactHash ch = plan_compact(bits.all, bits.any, ix.n, &cbits);
     if (!ch.on) return true;
     const u64 cap = 1ull << cbits;
     if (!ensure_storage(st, cap * 8, s)) return false;
     if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 8, s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, sizeof(u32), s))) return false;
     kclock().begin(s, &kstats().index_ms);
     compact_build_kernel<<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const float *)ix.vals, ix.n,
-                                                                 (unsigned long long *)st.p, ch, cap, c.err);
+                                                                 (unsigned long long *)st.p, ch, cap, index_err(ix, c));
     kclock().end(s);
-    u32 e = 0;
-    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(&e, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaStreamSynchronize(s)))
+    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(h_index_err + ix.slot, index_err(ix, c), sizeof(u32), cudaMemcpyDeviceToHost, s)))
         return false;
-    kclock().flush();
-    if (e) return true;  // a probe ran past what the tag can hold: 16-byte slots instead
     ix.kind = INDEX_HASH;
     ix.slots = st.p;
     ix.cap = cap;
     ix.ch = ch;
-    kstats().index_builds++;
-    kstats().compact_index_builds++;
+    ix.unchecked = true;
     return true;
 }
 
 int g_region_build = 1;  // 16-byte-slot indexes of 2^16..2^28 keys built region by region
 
-// the region-partitioned build (above); leaves ix.kind == INDEX_BISECT when the
-// overflow list ran out (the caller then builds with the atomic form)
-static bool build_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s)
+// launches the region-partitioned build (above); the overflow keys are inserted
+// by a kernel that reads their number, so nothing is waited for in between
+static bool begin_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s)
 {
     const u64 n = ix.n;
     const u64 cap = hash_capacity(n);
@@ -736,48 +751,57 @@ static bool build_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
     const double mean = (double)n * BUILD_REGION / (double)cap;
     const u32 bcap = (u32)((mean + 8.0 * sqrt(mean) + 64.0 + 15.0) / 16.0) * 16u;
     if (!ensure_storage(st, cap * 16, s)) return false;
-    // scratch: the cursors (u32), the region buckets, the overflow list
+    // scratch: the cursors and the overflow count (u32), the region buckets, the overflow list
     const u64 bytes = 4ull * nreg + 64 + 16ull * nreg * bcap + 16ull * max_over;
     void *scratch = nullptr;
     if (!dev_alloc(&scratch, bytes, s)) return false;
-    u32 *cursor = (u32 *)scratch;
-    ulonglong2 *tmp = (ulonglong2 *)(((uintptr_t)(cursor + nreg) + 15) & ~(uintptr_t)15);
+    u32 *cursor = (u32 *)scratch, *n_over = cursor + nreg;
+    ulonglong2 *tmp = (ulonglong2 *)(((uintptr_t)(n_over + 1) + 15) & ~(uintptr_t)15);
     ulonglong2 *over = tmp + (u64)nreg * bcap;
-    bool ok = CGB_CUDA(cudaMemsetAsync(cursor, 0, 4ull * nreg, s)) &&
-              CGB_CUDA(cudaMemsetAsync(c.d + 6, 0, sizeof(u64), s)) && CGB_CUDA(cudaMemsetAsync(c.err, 0, 4, s));
-    u32 *n_over = (u32 *)(c.d + 6);
+    bool ok = CGB_CUDA(cudaMemsetAsync(cursor, 0, 4ull * nreg + 4, s)) && CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, 4, s));
     if (ok) {
         kclock().begin(s, &kstats().index_ms);
         const int grid = grid_for((n + 3) / 4, 256, 8);
         if (vbytes == 8)
             region_scatter_kernel<double><<<grid, 256, 0, s>>>(ix.keys, (const double *)ix.vals, n, cap, bcap,
-                                                                cursor, tmp, over, max_over, n_over, c.err);
+                                                                cursor, tmp, over, max_over, n_over, index_err(ix, c));
         else
             region_scatter_kernel<float><<<grid, 256, 0, s>>>(ix.keys, (const float *)ix.vals, n, cap, bcap,
-                                                               cursor, tmp, over, max_over, n_over, c.err);
+                                                               cursor, tmp, over, max_over, n_over, index_err(ix, c));
         region_build_kernel<<<std::min<u32>(nreg, (u32)NUM_SMS_B200 * 4), 512, 0, s>>>(
-            tmp, cursor, bcap, nreg, cap, (ulonglong2 *)st.p, over, max_over, n_over, c.err);
+            tmp, cursor, bcap, nreg, cap, (ulonglong2 *)st.p, over, max_over, n_over, index_err(ix, c));
+        overflow_insert_kernel<<<NUM_SMS_B200, 256, 0, s>>>(over, n_over, max_over, (ulonglong2 *)st.p, cap, index_err(ix, c));
         kclock().end(s);
         kstats().launches += 2;
-        ok = CGB_CUDA(cudaGetLastError());
-    }
-    u32 h[2] = {0, 0};  // overflow count, error word
-    ok = ok && CGB_CUDA(cudaMemcpyAsync(&h[0], n_over, 4, cudaMemcpyDeviceToHost, s)) &&
-         CGB_CUDA(cudaMemcpyAsync(&h[1], c.err, 4, cudaMemcpyDeviceToHost, s)) && CGB_CUDA(cudaStreamSynchronize(s));
-    kclock().flush();
-    if (ok && h[1] == 0 && h[0]) {
-        kclock().begin(s, &kstats().index_ms);
-        overflow_insert_kernel<<<std::max<u32>(1, std::min<u32>((h[0] + 255) / 256, 1024)), 256, 0, s>>>(
-            over, h[0], (ulonglong2 *)st.p, cap, c.err);
-        kclock().end(s);
-        kstats().launches++;
-        ok = CGB_CUDA(cudaGetLastError()) && CGB_CUDA(cudaMemcpyAsync(&h[1], c.err, 4, cudaMemcpyDeviceToHost, s)) &&
-             CGB_CUDA(cudaStreamSynchronize(s));
-        kclock().flush();
+        ok = CGB_CUDA(cudaGetLastError()) &&
+             CGB_CUDA(cudaMemcpyAsync(h_index_err + ix.slot, index_err(ix, c), sizeof(u32), cudaMemcpyDeviceToHost, s));
     }
     dev_free(scratch, s);
     if (!ok) return false;
-    if (h[1]) return true;  // the overflow list ran out: the atomic build instead
+    ix.kind = INDEX_HASH;
+    ix.slots = st.p;
+    ix.cap = cap;
+    ix.unchecked = true;
+    return true;
+}
+
+// launches the atomic build into a zeroed table, which cannot fail: the table
+// has more slots than keys
+static bool begin_atomic(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s)
+{
+    // load factor <= g_hash_load_pct: capacity rounded up to a multiple of 64 slots
+    const u64 cap = hash_capacity(ix.n);
+    if (!ensure_storage(st, cap * 16, s)) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 16, s))) return false;
+    kclock().begin(s, &kstats().index_ms);
+    if (vbytes == 8)
+        hash_build_kernel<double><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const double *)ix.vals, ix.n,
+                                                                         (ulonglong2 *)st.p, cap, index_err(ix, c));
+    else
+        hash_build_kernel<float><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const float *)ix.vals, ix.n,
+                                                                        (ulonglong2 *)st.p, cap, index_err(ix, c));
+    kclock().end(s);
+    if (!CGB_CUDA(cudaGetLastError())) return false;
     ix.kind = INDEX_HASH;
     ix.slots = st.p;
     ix.cap = cap;
@@ -785,52 +809,29 @@ static bool build_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
     return true;
 }
 
-bool build_index(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c,
-                 cudaStream_t s)
+bool index_begin(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c, cudaStream_t s,
+                 const KeyBits &bits, int slot)
 {
+    ix.slot = slot;
     ix.kind = INDEX_BISECT;
     ix.bucket = nullptr;
     ix.slots = nullptr;
     ix.cap = 0;
+    ix.unchecked = false;
     if (ix.n == 0 || kind == INDEX_BISECT) return true;
     ix.ch = CompactHash{};
+    if (!h_index_err) {
+        void *h = nullptr;
+        if (!CGB_CUDA(cudaHostAlloc(&h, INDEX_SLOTS * sizeof(u32), cudaHostAllocDefault))) return false;
+        h_index_err = (u32 *)h;
+    }
     if (kind == INDEX_HASH && vbytes == 4 && g_hash_compact && ix.n >= 64) {
-        if (!build_compact(ix, st, c, s)) return false;
+        if (!begin_compact(ix, st, c, s, bits)) return false;
         if (ix.kind == INDEX_HASH) return true;
     }
-    if (kind == INDEX_HASH && g_region_build && ix.n >= (1u << 16) && ix.n <= (1u << 28)) {
-        if (!build_regions(ix, vbytes, st, c, s)) return false;
-        if (ix.kind == INDEX_HASH) return true;
-    }
-    if (kind == INDEX_HASH) {
-        // load factor <= g_hash_load_pct: capacity rounded up to a multiple of 64 slots
-        const u64 cap = hash_capacity(ix.n);
-        if (!ensure_storage(st, cap * 16, s)) return false;
-        if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 16, s))) return false;
-        if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
-        kclock().begin(s, &kstats().index_ms);
-        if (vbytes == 8)
-            hash_build_kernel<double><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(
-                ix.keys, (const double *)ix.vals, ix.n, (ulonglong2 *)st.p, cap, c.err);
-        else
-            hash_build_kernel<float><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(
-                ix.keys, (const float *)ix.vals, ix.n, (ulonglong2 *)st.p, cap, c.err);
-        kclock().end(s);
-        if (!CGB_CUDA(cudaGetLastError())) return false;
-        u32 e = 0;
-        if (!CGB_CUDA(cudaMemcpyAsync(&e, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s))) return false;
-        if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
-        kclock().flush();
-        if (e) {
-            set_error("build_index: device error " + err_string(e));
-            return false;
-        }
-        ix.kind = INDEX_HASH;
-        ix.slots = st.p;
-        ix.cap = cap;
-        kstats().index_builds++;
-        return true;
-    }
+    if (kind == INDEX_HASH && g_region_build && ix.n >= (1u << 16) && ix.n <= (1u << 28))
+        return begin_regions(ix, vbytes, st, c, s);
+    if (kind == INDEX_HASH) return begin_atomic(ix, vbytes, st, c, s);
     // INDEX_BUCKET
     if (ix.n < 64 || bucket_bits <= 0) return true;
     u64 first, last;
@@ -839,21 +840,49 @@ bool build_index(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int buc
     if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
     const u64 x = first ^ last;
     const int prefix = x ? __builtin_clzll(x) : 64;
-    int bits = bucket_bits;
-    if (bits > 64 - prefix) bits = 64 - prefix;
-    if (bits <= 0) return true;
-    const u64 need = ((1ull << bits) + 1) * sizeof(u32);
+    int nb = bucket_bits;
+    if (nb > 64 - prefix) nb = 64 - prefix;
+    if (nb <= 0) return true;
+    const u64 need = ((1ull << nb) + 1) * sizeof(u32);
     if (!ensure_storage(st, need, s)) return false;
     kclock().begin(s, &kstats().index_ms);
-    bucket_offsets_kernel<<<grid_for(ix.n + 1, 256, 16), 256, 0, s>>>(ix.keys, ix.n, (u32 *)st.p, prefix, bits);
+    bucket_offsets_kernel<<<grid_for(ix.n + 1, 256, 16), 256, 0, s>>>(ix.keys, ix.n, (u32 *)st.p, prefix, nb);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
     ix.kind = INDEX_BUCKET;
     ix.bucket = (const u32 *)st.p;
     ix.prefix = prefix;
-    ix.bits = bits;
+    ix.bits = nb;
     ix.prefix_value = prefix ? first >> (64 - prefix) : 0;
     return true;
+}
+
+bool index_finish(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s, bool *again)
+{
+    if (!ix.unchecked) return true;
+    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
+    kclock().flush();
+    ix.unchecked = false;
+    if (h_index_err[ix.slot] == 0) {
+        kstats().index_builds++;
+        if (ix.ch.on) kstats().compact_index_builds++;
+        return true;
+    }
+    // a probe ran past what the tag can hold: 16-byte slots; their overflow list ran
+    // out: the atomic build
+    if (again) *again = true;
+    const bool was_compact = ix.ch.on != 0;
+    ix.ch = CompactHash{};
+    ix.kind = INDEX_BISECT;
+    if (was_compact && g_region_build && ix.n >= (1u << 16) && ix.n <= (1u << 28))
+        return begin_regions(ix, vbytes, st, c, s) && index_finish(ix, vbytes, st, c, s);
+    return begin_atomic(ix, vbytes, st, c, s);
+}
+
+bool build_index(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c,
+                 cudaStream_t s)
+{
+    return index_begin(ix, kind, vbytes, st, bucket_bits, c, s) && index_finish(ix, vbytes, st, c, s);
 }
 
 template <typename V>
@@ -915,36 +944,49 @@ static void enqueue_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, 
                             : plan.form == CANON_DIAGONAL ? solve_items_kernel<V, CANON_DIAGONAL>
                             : plan.form == CANON_MIRROR   ? solve_items_kernel<V, CANON_MIRROR>
                                                           : solve_items_kernel<V, CANON_LIST>;
-        kernel<<<grid_for(n, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
-            keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan);
+        // a warp takes `per` boards at a time: 32, fewer where the layer does not
+        // give every warp of the chip that many, so that it spreads over the SMs and
+        // one round of pairs serves a warp (2600 2x4 boards: 27 -> 18 us)
+        u32 per = 4;
+        while (per < 32 && (u64)per * ITEM_WARPS * NUM_SMS_B200 < n) per *= 2;
+        kernel<<<grid_for((n + per - 1) / per * 32, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
+            keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan, per);
     } else {
         solve_direct_kernel<V><<<grid_for(n, DIRECT_THREADS, 1), DIRECT_THREADS, TABLE_BYTES_S, s>>>(
             keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan);
     }
 }
 
-template <class V>
-static bool launch_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, const LayerIndex &t4,
-                         const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
-                         const CanonPlan &plan)
+constexpr int PROBES_AT = 12;  // counter word of the probes not collected yet
+
+bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
+                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
+                        const CanonPlan &plan)
 {
     if (n == 0) return true;
     if (!solve_attrs()) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d + 2, 0, sizeof(u64), s))) return false;
     kclock().begin(s, &kstats().solve_ms);
-    enqueue_solve<V>(keys, n, out, t2, t4, r, rt, c.d + 2, s, plan);
+    if (vbytes == 4) enqueue_solve<float>(keys, n, (float *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan);
+    else enqueue_solve<double>(keys, n, (double *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    u64 probes = 0;
-    if (!CGB_CUDA(cudaMemcpyAsync(&probes, c.d + 2, sizeof(u64), cudaMemcpyDeviceToHost, s))) return false;
-    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
-    kclock().flush();
     KernelStats &k = kstats();
     k.solve_launches++;
     k.solve_boards += n;
+    k.solve_bytes += (8 + vbytes) * n;  // keys in, values out; the probes' sectors follow
+    return true;
+}
+
+bool solve_collect(Counters &c, cudaStream_t s)
+{
+    u64 probes = 0;
+    if (!CGB_CUDA(cudaMemcpyAsync(&probes, c.d + PROBES_AT, sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
+        !CGB_CUDA(cudaMemsetAsync(c.d + PROBES_AT, 0, sizeof(u64), s)) || !CGB_CUDA(cudaStreamSynchronize(s)))
+        return false;
+    kclock().flush();
+    KernelStats &k = kstats();
     k.lookups += probes;
-    // keys in, values out, one key sector and one value sector per probe
-    k.solve_bytes += (8 + sizeof(V)) * n + 64 * probes;
+    k.solve_bytes += 64 * probes;  // one key sector and one value sector per probe
     return true;
 }
 
@@ -998,13 +1040,13 @@ bool build_hash_enqueue(LayerIndex &ix, int vbytes, void *slots, u64 cap, u32 *e
 bool solve_layer_f64(const u64 *keys, u64 n, double *out, const LayerIndex &t2, const LayerIndex &t4,
                      const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s, const CanonPlan &plan)
 {
-    return launch_solve<double>(keys, n, out, t2, t4, r, rt, c, s, plan);
+    return n == 0 || (solve_layer_launch(keys, n, out, 8, t2, t4, r, rt, c, s, plan) && solve_collect(c, s));
 }
 
 bool solve_layer_f32(const u64 *keys, u64 n, float *out, const LayerIndex &t2, const LayerIndex &t4,
                      const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s, const CanonPlan &plan)
 {
-    return launch_solve<float>(keys, n, out, t2, t4, r, rt, c, s, plan);
+    return n == 0 || (solve_layer_launch(keys, n, out, 4, t2, t4, r, rt, c, s, plan) && solve_collect(c, s));
 }
 
 // ---- batch lookup (lookup(), src/solve.c:108-164, for many boards) --------

@@ -1079,13 +1079,14 @@ bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cuda
 }
 
 bool sort_unique_keys(u64 *keys, u64 *tmp, u64 n, u64 **out, u64 *n_out, SortWorkspace &ws, cudaStream_t s,
-                      SortStats *stats, u64 *empties)
+                      SortStats *stats, u64 *empties, KeyBits *bits)
 {
     if (stats) *stats = SortStats{};
+    if (bits) *bits = KeyBits{};
     if (bucket_sorts() && !ws.err_dirty) {
         bool done = false;
         int passes = 0;
-        if (!bucket_sort(keys, n, tmp, true, n_out, empties, &passes, ws.buckets, s, &done)) return false;
+        if (!bucket_sort(keys, n, tmp, true, n_out, empties, &passes, ws.buckets, s, &done, bits)) return false;
         if (done) {
             *out = tmp;
             if (stats) {

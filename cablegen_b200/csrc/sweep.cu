@@ -30,6 +30,7 @@ struct Layer {
     LayerStore::Handle h;
     bool live;
     const u64 *host = nullptr;  // host copy of the keys (host_layers), when kept
+    KeyBits bits;               // AND and OR of the keys
 };
 
 // device -> host copy on the I/O stream after the main stream's work so far;
@@ -86,6 +87,7 @@ struct StoreSink : LayerSink {
         // the engine's layer buffer is reused by the next layer step: keep an
         // exact-size copy in the store (8 B/board)
         Layer L{sum, {}, true};
+        L.bits = Engine::get().gen.moved_bits;
         if (!store.push(n, s, &L.h)) return false;
         u64 *keys = store.ptr(L.h, s);
         if (!keys) return false;
@@ -137,6 +139,7 @@ struct Chain {
         const u64 *keys = nullptr;
         void *vals = nullptr;
         u64 n = 0;
+        KeyBits bits;
         IndexStorage store;
         LayerIndex ix;
     };
@@ -164,17 +167,17 @@ struct Chain {
         cur.vb = layer_vbytes(cur.sum);
         if (cur.vb == 4 && !(narrow(e, t2, s) && narrow(e, t4, s))) return false;
         if (!dev_alloc(&cur.vals, cur.n * cur.vb + 8, s)) return false;
-        if (cur.vb == 4)
-            return solve_layer_f32(cur.keys, cur.n, (float *)cur.vals, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan);
-        return solve_layer_f64(cur.keys, cur.n, (double *)cur.vals, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan);
+        return solve_layer_launch(cur.keys, cur.n, cur.vals, cur.vb, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan);
     }
-    bool index(Engine &e, cudaStream_t s)
+    // launches the index build of the solved layer; finish_index waits for it
+    bool begin_index(Engine &e, cudaStream_t s)
     {
         cur.ix.keys = cur.keys;
         cur.ix.vals = cur.vals;
         cur.ix.n = cur.n;
-        return build_index(cur.ix, e.index_kind, cur.vb, cur.store, e.bucket_bits, e.ctr, s);
+        return index_begin(cur.ix, e.index_kind, cur.vb, cur.store, e.bucket_bits, e.ctr, s, cur.bits);
     }
+    bool finish_index(Engine &e, cudaStream_t s) { return index_finish(cur.ix, cur.vb, cur.store, e.ctr, s); }
     void rotate(cudaStream_t s)
     {
         if (t4.vals) dev_free(t4.vals, s);
@@ -303,6 +306,7 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
             c.cur.sum = sum;
             c.cur.keys = keys;
             c.cur.n = n;
+            c.cur.bits = it != by_sum.end() ? sink.layers[it->second].bits : KeyBits{};
             ok = ok && c.solve(e, rules, s);
         }
         if (!ok) break;
@@ -357,7 +361,11 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
             }
             if (!ok) break;
         }
-        for (auto &c : chains) ok = ok && c.index(e, s);
+        // the index build runs while the callback of the table before this one does;
+        // two chains share the build's error word, so each finishes its own at once
+        for (auto &c : chains) ok = ok && c.begin_index(e, s) && (chains.size() == 1 || c.finish_index(e, s));
+        if (ok && enqueued) ok = out.finish_older();
+        for (auto &c : chains) ok = ok && c.finish_index(e, s);
         if (!ok) break;
         // the s+4 layer is no longer needed by anyone.  When this layer's table
         // was enqueued, the copies still in flight are this layer's and the
@@ -375,6 +383,7 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
     }
     if (ok) ok = out.drain();
     out.fence_main();
+    if (!solve_collect(e.ctr, s)) ok = false;
     for (auto &c : chains) c.release(s);
     sink.store.clear(s);
     dev_free(d_ws, s);

@@ -332,11 +332,11 @@ extern "C" int cgb_solve_layer(const uint64_t *d_keys, uint64_t n, void *d_out, 
 {
     CGB_TRY(ensure_rules_for_api());
     cudaStream_t s = E().stream;
-    std::vector<u64> ws = expand_winstates(h_winstates, n_winstates);
-    u64 *d_ws = nullptr;
-    CGB_TRY(dev_alloc((void **)&d_ws, ws.size() * 8 + 8, s));
-    if (!ws.empty())
-        CGB_TRY(CGB_CUDA(cudaMemcpyAsync(d_ws, ws.data(), ws.size() * 8, cudaMemcpyHostToDevice, s)));
+    const std::vector<u64> ws = expand_winstates(h_winstates, n_winstates);
+    OneShot &o = E().one_shot;
+    o.busy = true;
+    bool ok = o.ws.cap >= ws.size() + 1 || grow(o.ws, 2 * ws.size() + 64, s);
+    if (ok && !ws.empty()) ok = CGB_CUDA(cudaMemcpyAsync(o.ws.p, ws.data(), ws.size() * 8, cudaMemcpyHostToDevice, s));
     LayerIndex t2, t4;
     t2.keys = d_k2;
     t2.vals = d_v2;
@@ -344,30 +344,30 @@ extern "C" int cgb_solve_layer(const uint64_t *d_keys, uint64_t n, void *d_out, 
     t4.keys = d_k4;
     t4.vals = d_v4;
     t4.n = n4;
-    const int vb = precision == 32 ? 4 : 8;
-    IndexStorage st2, st4;
-    bool ok = build_index(t2, E().index_kind, vb, st2, E().bucket_bits, E().ctr, s) &&
-              build_index(t4, E().index_kind, vb, st4, E().bucket_bits, E().ctr, s);
-    const SolveRules r = make_solve_rules(E().rules, d_ws, (int)ws.size());
-    // the images that can be canonical follow the 0xf mask of the first board
+    const int vb = precision == 32 ? 4 : 8, kind = E().index_kind;
+    // one wait for what the host has to know first: the images that can be canonical
+    // follow the 0xf mask of the first board; FP32 tables' keys decide their slots
+    KeyBits bits[3];
     CanonPlan plan;
     if (ok && n) {
-        u64 first = 0;
-        ok = CGB_CUDA(cudaMemcpyAsync(&first, d_keys, 8, cudaMemcpyDeviceToHost, s)) &&
-             CGB_CUDA(cudaStreamSynchronize(s));
-        plan = make_canon_plan(first, E().rules.free_formation != 0);
+        const KeySet none;
+        const bool want = vb == 4 && kind == INDEX_HASH;
+        ok = key_bits(want ? KeySet{d_k2, n2} : none, want ? KeySet{d_k4, n4} : none, bits, d_keys, E().ctr, s);
+        plan = make_canon_plan(bits[2].any, E().rules.free_formation != 0);
     }
-    if (ok) {
-        if (precision == 32)
-            ok = solve_layer_f32(d_keys, n, (float *)d_out, t2, t4, r, E().rt, E().ctr, s, plan);
-        else
-            ok = solve_layer_f64(d_keys, n, (double *)d_out, t2, t4, r, E().rt, E().ctr, s, plan);
-    }
-    dev_free(d_ws, s);
-    dev_free(st2.p, s);
-    dev_free(st4.p, s);
+    const SolveRules r = make_solve_rules(E().rules, o.ws.p, (int)ws.size());
+    // and one at the end, for the solve and both builds' error words
+    ok = ok && index_begin(t2, kind, vb, o.index[0], E().bucket_bits, E().ctr, s, bits[0], 0) &&
+         index_begin(t4, kind, vb, o.index[1], E().bucket_bits, E().ctr, s, bits[1], 1);
+    bool again = false;
+    do {
+        ok = ok && solve_layer_launch(d_keys, n, d_out, vb, t2, t4, r, E().rt, E().ctr, s, plan);
+        again = false;
+        ok = ok && solve_collect(E().ctr, s) && index_finish(t2, vb, o.index[0], E().ctr, s, &again) &&
+             index_finish(t4, vb, o.index[1], E().ctr, s, &again);
+    } while (ok && again);
+    E().end_one_shot();
     CGB_TRY(ok);
-    CGB_TRY(E().sync());
     return 0;
 }
 
@@ -394,10 +394,11 @@ int cgb_lookup_batch(const uint64_t *d_keys, const void *d_vals, uint64_t n, int
     if (search) {
         CGB_TRY(lookup_sorted(ix, vb, d_boards, m, canonicalize != 0, d_out, s));
     } else {
-        IndexStorage st;
+        IndexStorage &st = E().one_shot.index[0];
+        E().one_shot.busy = true;
         const bool ok = build_index(ix, E().index_kind, vb, st, E().bucket_bits, E().ctr, s) &&
                         lookup_batch(ix, vb, d_boards, m, canonicalize != 0, d_out, s);
-        dev_free(st.p, s);
+        E().end_one_shot();
         CGB_TRY(ok);
     }
     CGB_TRY(E().sync());

@@ -5,13 +5,13 @@
 // step.  An LSD radix sort moves every key once per varying byte (six times
 // for an LL board) and pays a fixed latency per pass, so both large and small
 // streams are slow.  Here a key moves two or three times whatever its width:
-//   1. split:     one CTA sorts a sample of the input (64 keys per bucket) and
+//   1. split:     one CTA sorts a sample of the input (20 to 64 keys per bucket) and
 //                 keeps the bucket boundaries;
-//   2. partition: each tile of 8192 keys finds its keys' buckets by binary
+//   2. partition: each tile of 4096 keys finds its keys' buckets by binary
 //                 search over the boundaries in shared memory, ranks them with
 //                 shared-memory counters, reserves its space in every bucket
 //                 with one global add and writes the buckets' parts coalesced;
-//                 above 512 buckets this runs twice: coarse buckets first, then
+//                 above 400 buckets this runs twice: coarse buckets first, then
 //                 every coarse bucket by boundaries of its own;
 //   3. bucket:    one CTA per bucket (at most 4096 keys, 1800 on average) sorts
 //                 it in shared memory -- 16 keys per thread through a register
@@ -42,6 +42,8 @@ constexpr u32 BK_TARGET = 1800;   // keys per bucket aimed at
 constexpr u32 BK_CAP = 4096;      // keys a bucket holds; 2.27 x the target: with 32 samples per bucket a
                                   // size is off by 18 % (one sigma), so this is seven sigma
 constexpr u32 BK_FAN = 512;       // buckets of one partition step
+constexpr u32 BK_ONE_STEP = 400 * BK_TARGET;  // keys up to which one step is taken: 8192 samples bound 400
+                                              // buckets as well as 20 each do (2.27 x the size: one in a million)
 constexpr u32 BK_COARSE = 512;    // coarse buckets of the two-step form
 constexpr u32 BK_TILE = 4096;     // keys per partition CTA
 constexpr int BK_KPT = 16;        // keys per thread, every kernel
@@ -296,13 +298,14 @@ __device__ __forceinline__ void write_bounds(K (&v)[BK_KPT], K *buf, u32 m, u32 
     }
 }
 
-// Boundaries from a sorted sample.  STEP 0: the only step, `buckets` buckets of
-// the whole input; 1: the coarse step; 2: CTA c, the boundaries inside coarse
-// bucket c, whose number follows its size.  A sample is one random key out of
+// Boundaries from a sorted sample.  FINE false: of the whole input, into buckets
+// of the target size where one step does (BK_ONE_STEP), else into `buckets`
+// coarse buckets; true: CTA c, the boundaries inside coarse bucket c, whose number
+// follows its size.  A sample is one random key out of
 // each of equally long stretches, so that neither a regular pattern nor a
 // sorted input biases it.  (Nothing to do for the keys of one bucket: the bucket
 // sort takes them from the input.)
-template <int STEP>
+template <bool FINE>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u64 *__restrict__ src, KeyCount n,
                                                                         u32 buckets, u32 coarse_cap, u32 *head,
                                                                         u32 *arrays, u64 *__restrict__ bounds)
@@ -311,8 +314,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u6
     __shared__ u32 scratch[33];
     __shared__ BitMoves moves[2];
     u32 cnt = n.get(), nb = buckets;
-    if (cnt <= BK_CAP) return;
-    if (STEP == 2) {
+    const bool one_step = cnt <= BK_ONE_STEP;
+    if (cnt <= BK_CAP || (FINE && one_step)) return;
+    if (FINE) {
         const u32 c = blockIdx.x;
         // this coarse bucket's first fine bucket: the numbers of those before it, summed
         u32 mine = 0, all = 0;
@@ -334,11 +338,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u6
         if (nb <= 1) return;
         src += (u64)c * coarse_cap;
         bounds += (u64)c * BK_FAN;
-    } else if (STEP == 0) {
+    } else if (one_step) {
         nb = (cnt + BK_TARGET - 1) / BK_TARGET;
         if (threadIdx.x == 0) head[H_BUCKETS] = nb;
     }
-    const u32 m = min(min(nb * (STEP == 1 ? 64u : STEP == 2 ? 32u : 24u), BK_SAMPLES), cnt);
+    const u32 m = min(min(nb * (FINE ? 32u : one_step ? 24u : 64u), BK_SAMPLES), cnt);
     if (threadIdx.x < 4) scratch[threadIdx.x] = threadIdx.x < 2 ? 0xffffffffu : 0u;
     __syncthreads();
     u64 k[BK_KPT];
@@ -395,13 +399,13 @@ struct PartSmem {
 
 // One tile of a partition step.  FINE: the tile belongs to coarse bucket
 // blockIdx.x / tiles and goes to that bucket's fine buckets; else the input is
-// the source and the destination is the coarse buckets (or, with `fine_dst`,
-// the only step's fine buckets).
+// the source and goes to the coarse buckets, or to the fine ones where one step
+// does.
 template <bool FINE>
 __global__ void __launch_bounds__(PART_THREADS, 4)
     bucket_partition_kernel(const u64 *__restrict__ src, KeyCount n, u32 src_cap, u32 tiles, u32 buckets,
-                            const u64 *__restrict__ bounds, u32 *head, u32 *arrays, u32 counters,
-                            u64 *__restrict__ dst, u32 dst_cap)
+                            const u64 *__restrict__ bounds, u32 *head, u32 *arrays, u64 *coarse, u32 coarse_cap,
+                            u64 *fine)
 {
     extern __shared__ __align__(16) unsigned char part_smem[];
     PartSmem &S = *reinterpret_cast<PartSmem *>(part_smem);
@@ -410,9 +414,12 @@ __global__ void __launch_bounds__(PART_THREADS, 4)
     const u32 all = n.get();
     const u32 cnt = FINE ? min(arrays[A_COARSE + c], src_cap) : all;
     const u32 start = tile * BK_TILE;
-    if (start >= cnt || all <= BK_CAP) return;
-    // buckets 0: the only step, whose buckets follow the number of keys
-    const u32 nb = FINE ? arrays[A_NUM + c] : buckets ? buckets : head[H_BUCKETS];
+    const bool one_step = all <= BK_ONE_STEP;
+    if (start >= cnt || all <= BK_CAP || (FINE && one_step)) return;
+    const bool to_fine = FINE || one_step;
+    u64 *dst = to_fine ? fine : coarse;
+    const u32 dst_cap = to_fine ? BK_CAP : coarse_cap, counters = to_fine ? A_FINE : A_COARSE;
+    const u32 nb = FINE ? arrays[A_NUM + c] : one_step ? head[H_BUCKETS] : buckets;
     const u32 base = FINE ? arrays[A_BASE + c] : 0;
     if (FINE) {
         src += (u64)c * src_cap;
@@ -666,15 +673,14 @@ static bool attributes()
     if (done) return true;
     const int part = (int)sizeof(PartSmem), split = (int)(SAMPLE_WORDS * sizeof(u64));
     const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    done = CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<0>, smem, split)) &&
-           CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<1>, smem, split)) &&
-           CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<2>, smem, split)) &&
+    done = CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<false>, smem, split)) &&
+           CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<true>, smem, split)) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<false>, smem, part)) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<true>, smem, part));
     return done;
 }
 
-// Sizes of one call.  Two steps from 512 x 1800 keys on: coarse buckets of
+// Sizes of one call.  Two steps above BK_ONE_STEP keys: coarse buckets of
 // equal expected size, their space seven sigma above it (a coarse bucket is
 // bounded by 64 samples, or by 8192 / coarse).
 static bool plan_buckets(u64 n, BucketPlan *p)
@@ -684,7 +690,7 @@ static bool plan_buckets(u64 n, BucketPlan *p)
     if (n > BUCKET_SORT_KEYS) return false;
     if (n <= BK_CAP) {
         p->grid = 1;
-    } else if (n <= (u64)BK_FAN * BK_TARGET) {
+    } else if (n <= BK_ONE_STEP) {
         p->grid = (u32)((n + BK_TARGET - 1) / BK_TARGET);
     } else {
         u32 c = (u32)std::ceil(std::sqrt((double)n / BK_TARGET));
@@ -745,21 +751,19 @@ int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *co
     const KeyCount kc{(u32)p.n, counted};
     const u32 tiles = (u32)((p.n + BK_TILE - 1) / BK_TILE);
     int np = 1;
-    if (p.n > BK_CAP && !p.coarse) {
-        bucket_split_kernel<0><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, 0, 0, head, arrays, w.bounds.p);
+    if (p.n > BK_CAP) {
+        bucket_split_kernel<false><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, p.coarse, 0, head, arrays, w.bounds.p);
         bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-            keys, kc, 0, 1, 0, w.bounds.p, head, arrays, A_FINE, w.fine.p, BK_CAP);
+            keys, kc, 0, 1, p.coarse, w.bounds.p, head, arrays, w.coarse.p, p.coarse_cap, w.fine.p);
         np = 2;
-    } else if (p.coarse) {
+    }
+    if (p.coarse) {
         const u32 fine_tiles = (p.coarse_cap + BK_TILE - 1) / BK_TILE;
         u64 *fine_bounds = w.bounds.p + BK_FAN;
-        bucket_split_kernel<1><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, p.coarse, 0, head, arrays, w.bounds.p);
-        bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-            keys, kc, 0, 1, p.coarse, w.bounds.p, head, arrays, A_COARSE, w.coarse.p, p.coarse_cap);
-        bucket_split_kernel<2><<<p.coarse, SPLIT_THREADS, split_smem, s>>>(w.coarse.p, kc, p.coarse, p.coarse_cap, head,
-                                                                           arrays, fine_bounds);
+        bucket_split_kernel<true><<<p.coarse, SPLIT_THREADS, split_smem, s>>>(w.coarse.p, kc, p.coarse, p.coarse_cap, head,
+                                                                              arrays, fine_bounds);
         bucket_partition_kernel<true><<<p.coarse * fine_tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-            w.coarse.p, kc, p.coarse_cap, fine_tiles, 0, fine_bounds, head, arrays, A_FINE, w.fine.p, BK_CAP);
+            w.coarse.p, kc, p.coarse_cap, fine_tiles, 0, fine_bounds, head, arrays, nullptr, 0, w.fine.p);
         np = 3;
     }
     if (unique) launch_sort<true>(p, keys, kc, out, empties, head, arrays, w, s);

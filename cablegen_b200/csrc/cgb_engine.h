@@ -144,9 +144,6 @@ struct Engine {
     DeviceRowTable rt;
     SortWorkspace ws;
     Counters ctr;
-    // pinned words the spawn expansion's count and error word are copied into
-    // without a wait (checked after the sort that follows)
-    u64 *h_spawn_check = nullptr;
     cgb_rules rules{};
     int index_kind = INDEX_HASH;  // lookup structure of solved layers
     int bucket_bits = 22;         // INDEX_BUCKET: bucket count = 2^bits

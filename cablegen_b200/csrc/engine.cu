@@ -332,17 +332,12 @@ bool Engine::init(int dev)
     // that fails returns the cache to the device and retries (dev_alloc)
     u64 keep = ~0ull;
     if (!CGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep))) return false;
-    if (!h_spawn_check) {
-        void *h = nullptr;
-        if (!CGB_CUDA(cudaHostAlloc(&h, 2 * sizeof(u64), cudaHostAllocDefault))) return false;
-        h_spawn_check = (u64 *)h;
-        h_spawn_check[0] = h_spawn_check[1] = 0;
-    }
     if (!ctr.d) {
         void *p;
         if (!CGB_CUDA(cudaMalloc(&p, 64 * sizeof(u64)))) return false;
         ctr.d = (u64 *)p;
-        ctr.err = (u32 *)(ctr.d + 32);
+        ctr.err = (u32 *)(ctr.d + Counters::ERR);
+        if (!CGB_CUDA(cudaHostAlloc((void **)&ctr.host, Counters::HEAD * sizeof(u64), cudaHostAllocDefault))) return false;
         if (!CGB_CUDA(cudaMemset(p, 0, 64 * sizeof(u64)))) return false;
     }
     ready = true;
@@ -472,11 +467,11 @@ bool Engine::spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm)
         }
         for (auto &x : g.c)
             if (!reserve(x, cap, s)) return false;
-        if (!expand_next(part, SpawnSource{}, g.c[0].p, ctr, s, plan, h_spawn_check)) return false;
+        if (!expand_next(part, SpawnSource{}, g.c[0].p, ctr, s, plan)) return false;
         u64 nu = 0;
         DevBuf<u64> *u = nullptr;
         if (!sort_unique_step(g.c[0], g.c[1], part.total, &nu, &u, tm)) return false;
-        if (!check_spawns(h_spawn_check, part.total)) return false;
+        if (!check_spawns(ctr, part.total)) return false;
         if (!join(acc, *u, nu)) return false;
         if (chunked && tm) tm->chunks++;
         off += part.n;
@@ -512,11 +507,11 @@ bool Engine::next_inputs(GenTimes *tm)
     if (total <= std::min(max_sort_keys, BUCKET_SORT_KEYS)) {
         for (auto &x : g.c)
             if (!reserve(x, total, s)) return false;
-        if (!expand_next(two, four, g.c[0].p, ctr, s, plan, h_spawn_check)) return false;
+        if (!expand_next(two, four, g.c[0].p, ctr, s, plan)) return false;
         u64 nu = 0;
         DevBuf<u64> *u = nullptr;
         if (!sort_unique_step(g.c[0], g.c[1], total, &nu, &u, tm)) return false;
-        if (total && !check_spawns(h_spawn_check, total)) return false;
+        if (total && !check_spawns(ctr, total)) return false;
         std::swap(g.S, *u);
         g.S.n = nu;
     } else if (!spawn_into(two, g.S, tm) || !spawn_into(four, g.S, tm)) {

@@ -89,10 +89,13 @@ bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 
 
 // ---- sort / unique / merge (sort.cu) ------------------------------------
 struct SortWorkspace {
-    static constexpr int SMALL_WORDS = 8192;
-    u32 *small = nullptr;       // histograms, tile counters, error word, counts
-    u32 *lookback = nullptr;    // decoupled look-back state
-    u64 lookback_bytes = 0;
+    // histograms, bin offsets, tile counters, error word, counts; the decoupled
+    // look-back state follows in the same allocation, so one clear covers both
+    static constexpr int SMALL_WORDS = 4128;
+    u32 *small = nullptr;
+    u32 *lookback = nullptr;
+    u64 lookback_words = 0;
+    u32 *host = nullptr;        // pinned copy of the small words
     bool err_dirty = false;     // a sort left its errors in the word for unique to report
     BucketWorkspace buckets;
     bool reserve(u64 words, cudaStream_t s);
@@ -135,8 +138,12 @@ void build_row_table(int free_formation, int ignore_f, unsigned short *move, u32
 bool upload_row_table(DeviceRowTable &t, int free_formation, int ignore_f, cudaStream_t s);
 
 struct Counters {
-    u64 *d = nullptr;   // device words: [0] output count, [1] spawn total, [2..] scratch
-    u32 *err = nullptr; // device error word
+    // device words: [0] output count, [1] spawn total, [5] raw moves, [6] error word,
+    // [12] probes, [16..20] key bits, [40..] indexes' error words
+    static constexpr int ERR = 6, HEAD = 7;
+    u64 *d = nullptr;
+    u32 *err = nullptr;   // d + ERR
+    u64 *host = nullptr;  // pinned copy of the first HEAD words
 };
 
 // move + prune + canonicalise every board; out needs room for 4n boards
@@ -166,11 +173,11 @@ struct SpawnSource {
 bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u64 cap, u64 *count, u32 *err,
                          cudaStream_t s, const CanonPlan &plan);
 // the canonical spawns of both sources, a.total + b.total of them, in one array
-// and without a wait: the kernel's count and error word land in h_check (pinned,
-// 2 words), for check_spawns once the stream has been waited for
+// and without a wait: the counters land in c.host, for check_spawns once the
+// stream has been waited for
 bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters &c, cudaStream_t s,
-                 const CanonPlan &plan, u64 *h_check);
-bool check_spawns(const u64 *h_check, u64 expect);
+                 const CanonPlan &plan);
+bool check_spawns(const Counters &c, u64 expect);
 // canonical 2-spawn and 4-spawn of every empty cell of every board
 bool expand_spawns(const u64 *in, u64 n, u64 *out2, u64 *out4, u64 cap, u64 *n_out, Counters &c,
                    cudaStream_t s, const CanonPlan &plan = CanonPlan{});

@@ -355,40 +355,22 @@ static int sm_count()
     return sms;
 }
 
-static bool read_word(u64 *dst, const u64 *src, cudaStream_t s)
+// the counters start at zero ...
+static bool clear_counters(Counters &c, cudaStream_t s)
 {
-    if (!CGB_CUDA(cudaMemcpyAsync(dst, src, sizeof(u64), cudaMemcpyDeviceToHost, s))) return false;
-    return CGB_CUDA(cudaStreamSynchronize(s));
+    return CGB_CUDA(cudaMemsetAsync(c.d, 0, Counters::HEAD * sizeof(u64), s));
 }
-
-// one copy for a count word and the error word (Counters keeps the error word
-// 32 words after the counts)
-static bool read_count_checked(u64 *dst, Counters &c, int idx, cudaStream_t s, const char *what,
-                               u64 *raw = nullptr)
+// ... and come back in one copy
+static bool fetch_counters(Counters &c, cudaStream_t s)
 {
-    u64 words[33];
-    if (!CGB_CUDA(cudaMemcpyAsync(words, c.d, sizeof words, cudaMemcpyDeviceToHost, s))) return false;
-    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
-    const u32 e = (u32)words[32];
-    if (e) {
-        set_error(std::string(what) + ": device error " + err_string(e));
-        return false;
-    }
-    *dst = words[idx];
-    if (raw) *raw = words[5];
-    return true;
+    return CGB_CUDA(cudaMemcpyAsync(c.host, c.d, Counters::HEAD * sizeof(u64), cudaMemcpyDeviceToHost, s));
 }
-
-static bool check(Counters &c, cudaStream_t s, const char *what)
+static bool read_counters(Counters &c, cudaStream_t s, const char *what)
 {
-    u32 e = 0;
-    if (!CGB_CUDA(cudaMemcpyAsync(&e, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s))) return false;
-    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
-    if (e) {
-        set_error(std::string(what) + ": device error " + err_string(e));
-        return false;
-    }
-    return true;
+    if (!fetch_counters(c, s) || !CGB_CUDA(cudaStreamSynchronize(s))) return false;
+    const u32 e = (u32)c.host[Counters::ERR];
+    if (e) set_error(std::string(what) + ": device error " + err_string(e));
+    return e == 0;
 }
 
 bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceRowTable &t, const PruneParams &p,
@@ -435,18 +417,16 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
 {
     *n_out = 0;
     if (n == 0) return true;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d + 5, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
+    if (!clear_counters(c, s)) return false;
     kclock().begin(s, &kstats().expand_ms);
     const bool ok = expand_moves_enqueue(in, n, out, cap, t, p, c.d, c.d + 5, c.err, s, ff, plan);
     kclock().end(s);
     if (!ok) return false;
-    u64 raw = 0;
-    if (!read_count_checked(n_out, c, 0, s, "expand_moves", &raw)) return false;
+    if (!read_counters(c, s, "expand_moves")) return false;
+    *n_out = c.host[0];
     kclock().flush();
     kstats().expand_bytes += 8 * (n + *n_out);
-    kstats().moves_raw += raw;
+    kstats().moves_raw += c.host[5];
     kstats().moves_kept += *n_out;
     return true;
 }
@@ -455,13 +435,14 @@ bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s)
 {
     *total = 0;
     if (n == 0) return true;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d + 1, 0, sizeof(u64), s))) return false;
+    if (!clear_counters(c, s)) return false;
     const int grid = (int)std::min<u64>((n + 255) / 256, (u64)sm_count() * 8);
     kclock().begin(s, &kstats().spawn_ms);
     count_spawns_kernel<<<grid, 256, 0, s>>>(in, n, c.d + 1);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    if (!read_word(total, c.d + 1, s)) return false;
+    if (!read_counters(c, s, "count_spawns")) return false;
+    *total = c.host[1];
     kclock().flush();
     kstats().spawn_bytes += 8 * n;
     return true;
@@ -482,32 +463,26 @@ bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u
 }
 
 bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters &c, cudaStream_t s,
-                 const CanonPlan &plan, u64 *h_check)
+                 const CanonPlan &plan)
 {
-    // the count and, 32 words on, the error word
-    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s)) || !CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s)))
-        return false;
     const u64 cap = a.total + b.total;
+    if (!clear_counters(c, s)) return false;
     kclock().begin(s, &kstats().spawn_ms);
     const bool ok = expand_next_enqueue(a, b, out, cap, c.d, c.err, s, plan);
     kclock().end(s);
-    if (!ok) return false;
-    if (!CGB_CUDA(cudaMemcpyAsync(h_check, c.d, sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaMemcpyAsync(h_check + 1, c.err, sizeof(u32), cudaMemcpyDeviceToHost, s)))
-        return false;
     kstats().spawn_bytes += 8 * (a.n + b.n) + 8 * cap;
-    return true;
+    return ok && fetch_counters(c, s);
 }
 
-bool check_spawns(const u64 *h_check, u64 expect)
+bool check_spawns(const Counters &c, u64 expect)
 {
-    const u32 e = (u32)h_check[1];
+    const u32 e = (u32)c.host[Counters::ERR];
     if (e) {
         set_error(std::string("expand_next: device error ") + err_string(e));
         return false;
     }
-    if (h_check[0] != expect) {
-        set_error("expand_next: " + std::to_string(h_check[0]) + " spawns written, " + std::to_string(expect) +
+    if (c.host[0] != expect) {
+        set_error("expand_next: " + std::to_string(c.host[0]) + " spawns written, " + std::to_string(expect) +
                   " expected");
         return false;
     }
@@ -519,14 +494,14 @@ bool expand_spawns(const u64 *in, u64 n, u64 *out2, u64 *out4, u64 cap, u64 *n_o
 {
     *n_out = 0;
     if (n == 0) return true;
-    if (!CGB_CUDA(cudaMemsetAsync(c.d, 0, sizeof(u64), s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(c.err, 0, sizeof(u32), s))) return false;
+    if (!clear_counters(c, s)) return false;
     const int grid = (int)std::min<u64>((n + 255) / 256, (u64)sm_count() * 8);
     kclock().begin(s, &kstats().spawn_ms);
     expand_spawns_kernel<<<grid, 256, 0, s>>>(in, n, out2, out4, cap, c.d, c.err, plan);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    if (!read_count_checked(n_out, c, 0, s, "expand_spawns")) return false;
+    if (!read_counters(c, s, "expand_spawns")) return false;
+    *n_out = c.host[0];
     kclock().flush();
     kstats().spawn_bytes += 8 * n + 16 * *n_out;
     return true;

@@ -991,32 +991,56 @@ static inline u32 ceil_div(u64 a, u64 b) { return (u32)((a + b - 1) / b); }
 // user), one per tile for unique, four per tile for a merge
 bool SortWorkspace::reserve(u64 words, cudaStream_t s)
 {
-    const u64 need = (words + 64) * sizeof(u32);
-    if (need <= lookback_bytes && small) return true;
-    if (lookback) cudaFreeAsync(lookback, s);
-    lookback = nullptr;
-    if (!small) {
-        if (!CGB_CUDA(cudaMallocAsync((void **)&small, SMALL_WORDS * sizeof(u32), s))) return false;
+    if (!host && !CGB_CUDA(cudaHostAlloc((void **)&host, SMALL_WORDS * sizeof(u32), cudaHostAllocDefault))) return false;
+    if (small && words + 64 <= lookback_words) return true;
+    const u64 want = words + words / 4 + 64;
+    u32 *p = nullptr;
+    if (!CGB_CUDA(cudaMallocAsync((void **)&p, (SMALL_WORDS + want) * sizeof(u32), s))) return false;
+    if (small) {
+        // an earlier sort may have left errors for the next call to report
+        if (!CGB_CUDA(cudaMemcpyAsync(p, small, SMALL_WORDS * sizeof(u32), cudaMemcpyDeviceToDevice, s))) return false;
+        cudaFreeAsync(small, s);
     }
-    if (!CGB_CUDA(cudaMallocAsync((void **)&lookback, need, s))) return false;
-    lookback_bytes = need;
+    small = p;
+    lookback = p + SMALL_WORDS;
+    lookback_words = want;
     return true;
 }
 
 void SortWorkspace::release(cudaStream_t s)
 {
-    if (lookback) cudaFreeAsync(lookback, s);
     if (small) cudaFreeAsync(small, s);
     lookback = nullptr;
     small = nullptr;
-    lookback_bytes = 0;
+    lookback_words = 0;
     buckets.release(s);
 }
 
-// small words: [0,2048) histograms, [2048,2064) tile counters, 2064 err, 2065 count,
-// 2066-2067 a 64-bit count (8-byte aligned)
-static constexpr int W_HIST = 0, W_CTR = 2048, W_ERR = 2064, W_COUNT = 2065, W_COUNT64 = 2066, W_EMPTIES = 2068,
-                     W_OFFS = 4096;
+// small words: [0,2048) histograms, [2048,4096) bin offsets, [4096,4112) tile
+// counters, then the error word, a count, a 64-bit count and the empty-cell sum
+static constexpr int W_HIST = 0, W_OFFS = 2048, W_CTR = 4096, W_ERR = 4112, W_COUNT = 4113, W_COUNT64 = 4114,
+                     W_EMPTIES = 4116;
+
+// zeroes the tile counters, counts and `words` look-back words, and the error
+// word unless an earlier sort left errors in it for this call to report
+static bool clear_state(SortWorkspace &ws, u64 words, cudaStream_t s)
+{
+    int from = W_CTR;
+    if (ws.err_dirty) {
+        if (!CGB_CUDA(cudaMemsetAsync(ws.small + W_CTR, 0, (W_ERR - W_CTR) * sizeof(u32), s))) return false;
+        from = W_COUNT;
+        ws.err_dirty = false;
+    }
+    return CGB_CUDA(cudaMemsetAsync(ws.small + from, 0, (SortWorkspace::SMALL_WORDS - from + words) * sizeof(u32), s));
+}
+
+// the error word and the counts on the host
+static bool fetch_state(SortWorkspace &ws, cudaStream_t s)
+{
+    return CGB_CUDA(cudaMemcpyAsync(ws.host + W_ERR, ws.small + W_ERR, (W_EMPTIES + 2 - W_ERR) * sizeof(u32),
+                                    cudaMemcpyDeviceToHost, s)) &&
+           CGB_CUDA(cudaStreamSynchronize(s));
+}
 
 static bool check_err(SortWorkspace &ws, cudaStream_t s, const char *what)
 {
@@ -1119,13 +1143,13 @@ static bool digit_sort(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &
     kclock().end(s);
     kstats().hist_bytes += 8 * n;
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    u32 hist[8 * RADIX];
+    const u32 *hist = ws.host + W_HIST;
     if (g_sort_variant >= 3) {
         digit_offsets_kernel<<<8, RADIX, 0, s>>>(ws.small + W_HIST, ws.small + W_OFFS);
         kstats().launches++;
         if (!CGB_CUDA(cudaGetLastError())) return false;
     }
-    if (!CGB_CUDA(cudaMemcpyAsync(hist, ws.small + W_HIST, sizeof(hist), cudaMemcpyDeviceToHost, s))) return false;
+    if (!CGB_CUDA(cudaMemcpyAsync(ws.host + W_HIST, ws.small + W_HIST, 8 * RADIX * sizeof(u32), cudaMemcpyDeviceToHost, s))) return false;
     if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
     int digits[8];
     const int np = sort_plan(hist, n, digits);
@@ -1199,30 +1223,23 @@ bool unique_keys(const u64 *in, u64 n, u64 *out, u64 *n_out, SortWorkspace &ws, 
     }
     if (!ws.reserve((n + UNQ_TILE - 1) / UNQ_TILE + 1, s)) return false;
     const u32 tiles = ceil_div(n, UNQ_TILE);
-    if (!CGB_CUDA(cudaMemsetAsync(ws.small + W_CTR, 0, (W_ERR - W_CTR) * sizeof(u32), s))) return false;
-    // the count, the 64-bit count slot and the empty-cell sum start at zero
-    if (!CGB_CUDA(cudaMemsetAsync(ws.small + W_COUNT, 0, (W_EMPTIES + 2 - W_COUNT) * sizeof(u32), s))) return false;
-    if (!ws.err_dirty && !CGB_CUDA(cudaMemsetAsync(ws.small + W_ERR, 0, sizeof(u32), s))) return false;
-    ws.err_dirty = false;
-    if (!CGB_CUDA(cudaMemsetAsync(ws.lookback, 0, (u64)tiles * sizeof(u32), s))) return false;
+    if (!clear_state(ws, tiles, s)) return false;
     kclock().begin(s, &kstats().unique_ms);
     unique_kernel<<<tiles, UNQ_THREADS, 0, s>>>(in, (u32)n, out, ws.lookback, ws.small + W_CTR,
                                                 ws.small + W_COUNT, ws.small + W_ERR,
                                                 empties ? (unsigned long long *)(ws.small + W_EMPTIES) : nullptr);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    u32 ec[W_EMPTIES + 2 - W_ERR];  // error word, count, (64-bit count), empty-cell sum
-    if (!CGB_CUDA(cudaMemcpyAsync(ec, ws.small + W_ERR, sizeof(ec), cudaMemcpyDeviceToHost, s))) return false;
-    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
+    if (!fetch_state(ws, s)) return false;
     kclock().flush();
-    if (ec[0]) {
-        set_error(std::string("sort/unique: device error ") + err_string(ec[0]));
+    if (ws.host[W_ERR]) {
+        set_error(std::string("sort/unique: device error ") + err_string(ws.host[W_ERR]));
         return false;
     }
-    const u32 cnt = ec[1];
+    const u32 cnt = ws.host[W_COUNT];
     kstats().unique_bytes += 8 * (n + cnt);
     *n_out = cnt;
-    if (empties) memcpy(empties, &ec[W_EMPTIES - W_ERR], sizeof(u64));
+    if (empties) memcpy(empties, ws.host + W_EMPTIES, sizeof(u64));
     return true;
 }
 
@@ -1242,17 +1259,8 @@ bool merge_unique(const u64 *a, u64 na, const u64 *b, u64 nb, u64 *out, u64 *n_o
     // 64-bit look-back words, then the splits (both fit in the u32 look-back area)
     u64 *lb = (u64 *)ws.lookback;
     u64 *splits = lb + ((u64)tiles + 1);
-    // tile counters and counts start at zero; the error word too, unless sorts
-    // before this merge left errors in it (reported below with the merge's own)
-    if (ws.err_dirty) {
-        if (!CGB_CUDA(cudaMemsetAsync(ws.small + W_CTR, 0, (W_ERR - W_CTR) * sizeof(u32), s)) ||
-            !CGB_CUDA(cudaMemsetAsync(ws.small + W_COUNT, 0, (W_COUNT64 + 2 - W_COUNT) * sizeof(u32), s)))
-            return false;
-    } else if (!CGB_CUDA(cudaMemsetAsync(ws.small + W_CTR, 0, (W_COUNT64 + 2 - W_CTR) * sizeof(u32), s))) {
-        return false;
-    }
-    ws.err_dirty = false;
-    if (!CGB_CUDA(cudaMemsetAsync(lb, 0, ((u64)tiles + 1) * sizeof(u64), s))) return false;
+    // errors that sorts before this merge left are reported below with its own
+    if (!clear_state(ws, 2 * ((u64)tiles + 1), s)) return false;
     kclock().begin(s, &kstats().merge_ms);
     merge_partition_kernel<<<ceil_div(tiles + 1, 256), 256, 0, s>>>(a, na, b, nb, splits, tiles);
     merge_unique_kernel<<<tiles, MRG_THREADS, 0, s>>>(a, na, b, nb, splits, out, lb, ws.small + W_CTR,
@@ -1260,16 +1268,14 @@ bool merge_unique(const u64 *a, u64 na, const u64 *b, u64 nb, u64 *out, u64 *n_o
     kclock().end(s);
     kstats().launches++;
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    u32 ec[4];  // error word, (count u32 unused), 64-bit count
-    if (!CGB_CUDA(cudaMemcpyAsync(ec, ws.small + W_ERR, 4 * sizeof(u32), cudaMemcpyDeviceToHost, s))) return false;
-    if (!CGB_CUDA(cudaStreamSynchronize(s))) return false;
+    if (!fetch_state(ws, s)) return false;
     kclock().flush();
-    if (ec[0]) {
-        set_error(std::string("merge_unique: device error ") + err_string(ec[0]));
+    if (ws.host[W_ERR]) {
+        set_error(std::string("merge_unique: device error ") + err_string(ws.host[W_ERR]));
         return false;
     }
     u64 cnt;
-    memcpy(&cnt, &ec[2], 8);
+    memcpy(&cnt, ws.host + W_COUNT64, 8);
     kstats().merge_bytes += 8 * (total + cnt);
     *n_out = cnt;
     return true;
@@ -1310,11 +1316,11 @@ bool partition_by_formation(const u64 *in, u64 n, u64 *out, const unsigned char 
                                                           ws.lookback, ws.small + W_CTR, ws.small + W_ERR);
     kstats().launches += 2;
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    u32 e = 0;
-    if (!CGB_CUDA(cudaMemcpyAsync(counts, ws.small + W_HIST, 256 * sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaMemcpyAsync(&e, ws.small + W_ERR, sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
-        !CGB_CUDA(cudaStreamSynchronize(s)))
+    if (!CGB_CUDA(cudaMemcpyAsync(ws.host + W_HIST, ws.small + W_HIST, 256 * sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
+        !fetch_state(ws, s))
         return false;
+    memcpy(counts, ws.host + W_HIST, 256 * sizeof(u32));
+    const u32 e = ws.host[W_ERR];
     ws.err_dirty = false;
     if (e) {
         set_error("partition_by_formation: device error " + err_string(e));

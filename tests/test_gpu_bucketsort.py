@@ -1,5 +1,5 @@
 """The sort by sampled buckets (csrc/bucketsort.cu) against numpy at the sizes where it changes
-form -- one bucket (up to 4096 keys), one partition step (up to 512 x 1800 keys), two steps -- for
+form -- one bucket (up to 4096 keys), one partition step (up to 400 x 1800 keys), two steps -- for
 keys whose buckets differ in the low word alone, in at most 32 bits of both words, and in more; keys
 with repeats; and inputs it hands on to the digit passes (a bucket that cannot hold its repeats)."""
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-ONE, TWO = 4096, 512 * 1800
+ONE, TWO = 4096, 400 * 1800
 
 
 def keys(kind, n):

@@ -295,6 +295,53 @@ __host__ __device__ __forceinline__ bool prune_by_table(u64 b, const PruneTable 
     return thrice || slc >= 6 || (long long)small > t.stsl + 64 || large > t.ltc;
 }
 
+// The same predicate from one u64 per byte, for smallest_large from 5 up: fields
+// for the small-tile weight (sl + 5 bits), the number of large tiles (6 bits) and
+// the copies of every large value (5 bits each), 81 - 4 sl bits in all.  The sum
+// over a board's eight bytes holds all counts; one added constant carries every
+// field that is over its limit into the field's top bit, and one AND tells.  A
+// third of the shared-memory traffic of prune_by_table and half its operations.
+struct PackedPrune {
+    u64 w[256];
+    u64 add, test;
+    u32 on;
+};
+
+inline void build_packed_prune(const PruneParams &p, PackedPrune *t)
+{
+    *t = PackedPrune{};
+    const long long sl = p.smallest_large, limit = p.stsl + 64;
+    if (sl < 5 || sl > 14 || limit < 0 || p.ltc < 0) return;
+    const int sb = (int)sl + 5, nf = 14 - (int)sl;  // small field's bits, count fields
+    const int large_at = sb, count_at = sb + 6;
+    for (int b = 0; b < 256; b++)
+        for (int x : {b >> 4, b & 15}) {
+            if (x < sl) t->w[b] += 1ull << x;
+            else if (x < 14) t->w[b] += (1ull << large_at) + (1ull << (count_at + 5 * (x - (int)sl)));
+        }
+    // over its limit <=> the field plus (top bit - 1 - limit) reaches the top bit; a
+    // limit that no board can pass adds nothing
+    const long long small_top = 1ll << (sb - 1);
+    t->test = (1ull << (sb - 1)) | (1ull << (large_at + 5));
+    if (limit < small_top) t->add += (u64)(small_top - 1 - limit);
+    if (p.ltc < 32) t->add += (u64)(31 - p.ltc) << large_at;
+    for (int i = 0; i < nf; i++) {  // three copies of a value, six of smallest_large
+        t->add += (u64)(16 - (i == 0 ? 6 : 3)) << (count_at + 5 * i);
+        t->test |= 16ull << (count_at + 5 * i);
+    }
+    t->on = 1;
+}
+
+// tab: w of every byte value, `stride` words apart
+__host__ __device__ __forceinline__ bool prune_packed(u64 b, const u64 *tab, u32 stride, u64 add, u64 test)
+{
+    const u32 hi = (u32)(b >> 32), lo = (u32)b;
+    u64 sum = add;
+#pragma unroll
+    for (int i = 0; i < 4; i++) sum += tab[((hi >> (8 * i)) & 0xFFu) * stride] + tab[((lo >> (8 * i)) & 0xFFu) * stride];
+    return (sum & test) != 0;
+}
+
 // contains tile x?  (src/generate.c:89-96 returns the negation)
 __host__ __device__ __forceinline__ bool has_tile(u64 b, int x)
 {

@@ -114,8 +114,30 @@ constexpr int MOVE_SET = 8192;
 // sweep to tile sum 600 a window of 4 kept 10.5 % fewer moves (sort -44 ms
 // per step) but the fuller set's longer probes cost the expansion 108 ms more
 int g_move_window = 1;
+// The prune tables: both forms in device memory; in shared memory either
+// prune_by_table's, or eight interleaved copies of the packed one, a copy for
+// every eighth lane, so that of 16 lanes only two can meet on a bank.  Measured
+// on 4M LL boards: 270 us for the whole kernel with prune_by_table, 211 us packed.
+struct PruneTables {
+    PruneTable table;
+    PackedPrune packed;
+};
+constexpr int PACKED_COPIES = 8;
 constexpr int PRUNE_BYTES = ((int)sizeof(PruneTable) + 15) / 16 * 16;
-constexpr int EXP_SMEM = TABLE_BYTES + MOVE_SET * 8 + PRUNE_BYTES;
+constexpr int PACKED_BYTES = 256 * PACKED_COPIES * 8;
+constexpr int EXP_SMEM = TABLE_BYTES + MOVE_SET * 8 + (PRUNE_BYTES > PACKED_BYTES ? PRUNE_BYTES : PACKED_BYTES);
+
+// a board's prune verdict; smem is the staged form
+struct Pruner {
+    const unsigned char *smem;
+    u64 add, test;
+    bool packed;
+    __device__ __forceinline__ bool operator()(u64 b) const
+    {
+        if (packed) return prune_packed(b, (const u64 *)smem + (threadIdx.x & (PACKED_COPIES - 1)), PACKED_COPIES, add, test);
+        return prune_by_table(b, *(const PruneTable *)smem);
+    }
+};
 
 // probes before a key is kept without a slot (a repeat that gets this far is
 // kept too: the sort's unique drops it)
@@ -138,7 +160,7 @@ __device__ __forceinline__ bool set_insert(unsigned long long *set, u64 key)
 // images; FORM -1: over all eight) and checked against the CTA's set; returns
 // the mask of results to write
 template <int FORM>
-__device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const PruneParams &pp, const PruneTable &pt,
+__device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const PruneParams &pp, const Pruner &prunes,
                                            const CanonPlan &plan, unsigned long long *set, u64 r[4], u32 *raw)
 {
     u64 v[4];
@@ -150,7 +172,7 @@ __device__ __forceinline__ u32 board_moves(const RowTable &t, u64 b, const Prune
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         u64 m;
-        if (move_left(t, v[k], &m) == 2 && !(pp.enabled && popc64(empty_mask(m)) != empties && prune_by_table(m, pt))) {
+        if (move_left(t, v[k], &m) == 2 && !(pp.enabled && popc64(empty_mask(m)) != empties && prunes(m))) {
             r[k] = canon_planned<FORM>(m, plan, k);
             (*raw)++;
             if (set_insert(set, r[k])) mask |= 1u << k;
@@ -163,7 +185,7 @@ template <int FORM>
 __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 *__restrict__ in, u64 n,
                                                                       u64 *__restrict__ out, u64 cap,
                                                                       u64 *out_count, const unsigned short *g_move,
-                                                                      PruneParams pp, const PruneTable *g_prune,
+                                                                      PruneParams pp, const PruneTables *g_prune,
                                                                       u32 *err, FormationFilter ff, CanonPlan plan,
                                                                       u64 *raw_count, u32 window)
 {
@@ -171,10 +193,20 @@ __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 
     __shared__ u32 scan_scratch[33];
     __shared__ u64 base_sh;
     // the prune table next to the row table; both staged before the barrier in stage_table
-    PruneTable *pt = (PruneTable *)(smem + TABLE_BYTES + MOVE_SET * 8);
-    if (pp.enabled)
-        for (int i = threadIdx.x; i < PRUNE_BYTES / 16; i += EXP_THREADS)
-            ((uint4 *)pt)[i] = __ldg((const uint4 *)g_prune + i);
+    Pruner prunes{smem + TABLE_BYTES + MOVE_SET * 8, 0, 0, false};
+    if (pp.enabled) {
+        const PackedPrune &k = g_prune->packed;
+        prunes.add = k.add;
+        prunes.test = k.test;
+        prunes.packed = k.on != 0;
+        if (prunes.packed) {
+            for (int i = threadIdx.x; i < 256 * PACKED_COPIES; i += EXP_THREADS)
+                ((u64 *)(smem + TABLE_BYTES + MOVE_SET * 8))[i] = __ldg(k.w + i / PACKED_COPIES);
+        } else {
+            for (int i = threadIdx.x; i < PRUNE_BYTES / 16; i += EXP_THREADS)
+                ((uint4 *)(smem + TABLE_BYTES + MOVE_SET * 8))[i] = __ldg((const uint4 *)&g_prune->table + i);
+        }
+    }
     stage_table(smem, g_move);
     const RowTable t{(const unsigned short *)smem};
     unsigned long long *set = (unsigned long long *)(smem + TABLE_BYTES);
@@ -197,9 +229,9 @@ __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 
         if (idx < n) {
             // boards of a formation that has reached its last layer stop here
             const bool live = !ff.fid || __ldg(ff.active + __ldg(ff.fid + fixed_pattern(b)));
-            if (live && !(pp.enabled && prune_by_table(b, *pt))) {
-                if (planned) mask = board_moves<FORM>(t, b, pp, *pt, plan, set, r, &raw);
-                else mask = board_moves<-1>(t, b, pp, *pt, plan, set, r, &raw);
+            if (live && !(pp.enabled && prunes(b))) {
+                if (planned) mask = board_moves<FORM>(t, b, pp, prunes, plan, set, r, &raw);
+                else mask = board_moves<-1>(t, b, pp, prunes, plan, set, r, &raw);
             }
         }
         const u32 cnt = __popc(mask);
@@ -387,12 +419,14 @@ bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceR
         attr = true;
     }
     // the prune table of these parameters, in device memory until they change
-    static PruneTable *d_prune = nullptr;
+    static PruneTables *d_prune = nullptr;
     static PruneParams have{-1, -1, -1, -1};
     if (p.enabled && (!d_prune || have.stsl != p.stsl || have.ltc != p.ltc || have.smallest_large != p.smallest_large)) {
-        static PruneTable h;
-        build_prune_table(p, &h);
-        if (!d_prune && !CGB_CUDA(cudaMalloc((void **)&d_prune, PRUNE_BYTES))) return false;
+        static PruneTables h;
+        build_prune_table(p, &h.table);
+        build_packed_prune(p, &h.packed);
+        // (room for the last 16 bytes of the staged copy)
+        if (!d_prune && !CGB_CUDA(cudaMalloc((void **)&d_prune, sizeof(PruneTables) + 16))) return false;
         if (!CGB_CUDA(cudaMemcpyAsync(d_prune, &h, sizeof h, cudaMemcpyHostToDevice, s)) ||
             !CGB_CUDA(cudaStreamSynchronize(s)))
             return false;

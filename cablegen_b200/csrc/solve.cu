@@ -562,12 +562,19 @@ __global__ void compact_build_kernel(const u64 *__restrict__ keys, const float *
 // inserted afterwards into the finished table with the atomic probe from its
 // home slot; the slots a placed key skipped were taken when it was placed and
 // stay taken, so every key stays reachable by the linear probe from its home.
-constexpr u32 BUILD_REGION = 2048;
+constexpr u32 BUILD_REGION = 1024;
+// u32 words from one region's cursor to the next: a sector each, which spreads
+// the atomic adds over the L2 slices
+constexpr u32 CURSOR_PAD = 8;
 
 // Each region owns a bucket of `bcap` pairs in the scratch (the mean count of
 // a region plus eight standard deviations and a margin, so that a bucket runs
 // full almost never); a pair that finds its bucket full joins the overflow
 // list.  Four keys per thread per step keep four cursor atomics in flight.
+// Measured over 12.2M keys (two LL layers, FP64, scatter and build): cursors side
+// by side and 2048-slot regions in CTAs of 512 threads 506 us, a sector per cursor
+// 477 us, and 1024-slot regions in CTAs of 256, whose clearing, filling and
+// writing overlap more, 465 us; eight keys per step gave nothing.
 template <typename V>
 __global__ void __launch_bounds__(256) region_scatter_kernel(const u64 *__restrict__ keys, const V *__restrict__ vals,
                                                              u64 n, u64 cap, u32 bcap, u32 *cursor,
@@ -589,7 +596,7 @@ __global__ void __launch_bounds__(256) region_scatter_kernel(const u64 *__restri
 #pragma unroll
         for (int u = 0; u < U; u++) {
             r[u] = (u32)(home_pair(key[u], cap) / BUILD_REGION);
-            p[u] = i0 + u * stride < n ? atomicAdd(cursor + r[u], 1u) : 0u;
+            p[u] = i0 + u * stride < n ? atomicAdd(cursor + r[u] * CURSOR_PAD, 1u) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -606,7 +613,7 @@ __global__ void __launch_bounds__(256) region_scatter_kernel(const u64 *__restri
     }
 }
 
-__global__ void __launch_bounds__(512) region_build_kernel(const ulonglong2 *__restrict__ tmp,
+__global__ void __launch_bounds__(256) region_build_kernel(const ulonglong2 *__restrict__ tmp,
                                                            const u32 *__restrict__ cursor, u32 bcap, u32 nreg,
                                                            u64 cap, ulonglong2 *slots, ulonglong2 *overflow,
                                                            u32 max_over, u32 *n_over, u32 *err)
@@ -617,7 +624,7 @@ __global__ void __launch_bounds__(512) region_build_kernel(const ulonglong2 *__r
         __syncthreads();
         const u64 base = (u64)r * BUILD_REGION;
         const u32 len = (u32)min((u64)BUILD_REGION, cap - base);
-        const u32 cnt = min(cursor[r], bcap);
+        const u32 cnt = min(cursor[r * CURSOR_PAD], bcap);
         const ulonglong2 *bucket = tmp + (u64)r * bcap;
         for (u32 j = threadIdx.x; j < cnt; j += blockDim.x) {
             const ulonglong2 e = bucket[j];
@@ -752,13 +759,13 @@ static bool begin_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
     const u32 bcap = (u32)((mean + 8.0 * sqrt(mean) + 64.0 + 15.0) / 16.0) * 16u;
     if (!ensure_storage(st, cap * 16, s)) return false;
     // scratch: the cursors and the overflow count (u32), the region buckets, the overflow list
-    const u64 bytes = 4ull * nreg + 64 + 16ull * nreg * bcap + 16ull * max_over;
+    const u64 bytes = 4ull * nreg * CURSOR_PAD + 64 + 16ull * nreg * bcap + 16ull * max_over;
     void *scratch = nullptr;
     if (!dev_alloc(&scratch, bytes, s)) return false;
-    u32 *cursor = (u32 *)scratch, *n_over = cursor + nreg;
+    u32 *cursor = (u32 *)scratch, *n_over = cursor + (u64)nreg * CURSOR_PAD;
     ulonglong2 *tmp = (ulonglong2 *)(((uintptr_t)(n_over + 1) + 15) & ~(uintptr_t)15);
     ulonglong2 *over = tmp + (u64)nreg * bcap;
-    bool ok = CGB_CUDA(cudaMemsetAsync(cursor, 0, 4ull * nreg + 4, s)) && CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, 4, s));
+    bool ok = CGB_CUDA(cudaMemsetAsync(cursor, 0, 4ull * nreg * CURSOR_PAD + 4, s)) && CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, 4, s));
     if (ok) {
         kclock().begin(s, &kstats().index_ms);
         const int grid = grid_for((n + 3) / 4, 256, 8);
@@ -768,7 +775,7 @@ static bool begin_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
         else
             region_scatter_kernel<float><<<grid, 256, 0, s>>>(ix.keys, (const float *)ix.vals, n, cap, bcap,
                                                                cursor, tmp, over, max_over, n_over, index_err(ix, c));
-        region_build_kernel<<<std::min<u32>(nreg, (u32)NUM_SMS_B200 * 4), 512, 0, s>>>(
+        region_build_kernel<<<std::min<u32>(nreg, (u32)NUM_SMS_B200 * 8), 256, 0, s>>>(
             tmp, cursor, bcap, nreg, cap, (ulonglong2 *)st.p, over, max_over, n_over, index_err(ix, c));
         overflow_insert_kernel<<<NUM_SMS_B200, 256, 0, s>>>(over, n_over, max_over, (ulonglong2 *)st.p, cap, index_err(ix, c));
         kclock().end(s);

@@ -135,8 +135,8 @@ __device__ __forceinline__ void warp_sort(K (&v)[BK_KPT])
             for (int i = 0; i < BK_KPT / 2; i++) {
                 const K a = __shfl_xor_sync(0xffffffffu, v[BK_KPT - 1 - i], 2 * run - 1);
                 const K b = __shfl_xor_sync(0xffffffffu, v[i], 2 * run - 1);
-                v[i] = up ? max(v[i], a) : min(v[i], a);
-                v[BK_KPT - 1 - i] = up ? max(v[BK_KPT - 1 - i], b) : min(v[BK_KPT - 1 - i], b);
+                v[i] = (v[i] < a) != up ? v[i] : a;
+                v[BK_KPT - 1 - i] = (v[BK_KPT - 1 - i] < b) != up ? v[BK_KPT - 1 - i] : b;
             }
         }
 #pragma unroll 1
@@ -145,7 +145,7 @@ __device__ __forceinline__ void warp_sort(K (&v)[BK_KPT])
 #pragma unroll
             for (int i = 0; i < BK_KPT; i++) {
                 const K a = __shfl_xor_sync(0xffffffffu, v[i], d);
-                v[i] = up ? max(v[i], a) : min(v[i], a);
+                v[i] = (v[i] < a) != up ? v[i] : a;  // the smaller of the two, or the larger
             }
         }
 #pragma unroll

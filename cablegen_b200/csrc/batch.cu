@@ -88,7 +88,6 @@ struct BatchSink : LayerSink {
     std::vector<std::vector<Range>> ranges;  // [formation][step]
     int step = 0;
     u64 reserve_bytes = 0;
-    size_t checked_at = 0;  // store chunks at the last free-memory check
 
     bool set_active(cudaStream_t s)
     {
@@ -149,13 +148,11 @@ struct BatchSink : LayerSink {
         step++;
         if (!set_active(s)) return false;
         // keep room for the next steps (older steps move to pinned host memory)
-        // (the device query is not free: ask only when the store took a new chunk)
-        if (store.chunk_count() != checked_at) {
+        if (store.grown()) {
             const u64 want = reserve_bytes + 12 * n * 8;
             const u64 avail = device_available_bytes(e->device);
             // false when nothing is left to spill: carry on, an allocation may still fit
             if (avail < want) store.spill(want - avail, s, out->io);
-            checked_at = store.chunk_count();
         }
         return true;
     }

@@ -799,7 +799,7 @@ bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 
     const int np = bucket_enqueue(p, 0, keys, nullptr, out, unique, empties != nullptr, w, s);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError()) ||
-        !CGB_CUDA(cudaMemcpyAsync(w.host, w.ctl.p, BUCKET_HEAD_WORDS * 4, cudaMemcpyDeviceToHost, s)) ||
+        !words_to_host(w.host, w.ctl.p, BUCKET_HEAD_WORDS, s) ||
         !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
     kclock().flush();

@@ -123,6 +123,48 @@ static std::mutex g_mem_mu;
 static std::unordered_map<void *, u64> g_mem_blocks;
 static u64 g_mem_held = 0;
 
+// Large blocks that were freed, for the next allocation of about their size on
+// the same stream.  The stream-ordered pool under them splits a large free block
+// for any smaller request, so a sweep that frees and allocates blocks of hundreds
+// of MB left it in pieces and made it map new memory, at 1 to 25 ms a time.
+// Bounded in bytes; everything goes back to the pool when an allocation fails,
+// under a memory cap, and with release_blocks().
+struct FreeBlock {
+    void *p;
+    u64 bytes;
+    cudaStream_t s;
+};
+static std::vector<FreeBlock> g_free_blocks;
+static u64 g_free_bytes = 0;
+static constexpr u64 LARGE_BLOCK = 16ull << 20, FREE_BLOCK_BYTES = 8ull << 30;
+
+void release_blocks()
+{
+    std::lock_guard<std::mutex> g(g_mem_mu);
+    for (auto &b : g_free_blocks) cudaFreeAsync(b.p, b.s);
+    g_free_blocks.clear();
+    g_free_bytes = 0;
+}
+// a kept block of bytes .. 1.25 bytes; its size in *bytes
+static void *take_block(u64 *bytes, cudaStream_t s)
+{
+    if (*bytes < LARGE_BLOCK) return nullptr;
+    std::lock_guard<std::mutex> g(g_mem_mu);
+    size_t best = g_free_blocks.size();
+    for (size_t i = 0; i < g_free_blocks.size(); i++) {
+        const FreeBlock &b = g_free_blocks[i];
+        if (b.s == s && b.bytes >= *bytes && b.bytes <= *bytes + *bytes / 4 &&
+            (best == g_free_blocks.size() || b.bytes < g_free_blocks[best].bytes))
+            best = i;
+    }
+    if (best == g_free_blocks.size()) return nullptr;
+    const FreeBlock b = g_free_blocks[best];
+    g_free_blocks.erase(g_free_blocks.begin() + best);
+    g_free_bytes -= b.bytes;
+    *bytes = b.bytes;
+    return b.p;
+}
+
 bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
 {
     *p = nullptr;
@@ -143,12 +185,19 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
             return false;
         }
     }
+    if ((*p = take_block(&bytes, s))) {
+        std::lock_guard<std::mutex> g(g_mem_mu);
+        g_mem_blocks[*p] = bytes;
+        g_mem_held += bytes;
+        return true;
+    }
     cudaError_t e = cudaMallocAsync(p, bytes, s);
     if (e == cudaErrorMemoryAllocation) {
         // freed blocks of other sizes may still sit in the pool: return them
         // to the device and retry once
         cudaGetLastError();
         Engine::get().one_shot.drop(s);
+        release_blocks();
         cudaStreamSynchronize(s);
         int dev = 0;
         cudaGetDevice(&dev);
@@ -177,14 +226,32 @@ void dev_free(void *p, cudaStream_t s)
         std::lock_guard<std::mutex> g(g_mem_mu);
         auto it = g_mem_blocks.find(p);
         if (it != g_mem_blocks.end()) {
-            g_mem_held -= it->second;
+            const u64 bytes = it->second;
+            g_mem_held -= bytes;
             g_mem_blocks.erase(it);
+            // (blocks freed on another stream than the engine's are not allocated there)
+            if (bytes >= LARGE_BLOCK && !g_dev_mem_cap && g_free_bytes + bytes <= FREE_BLOCK_BYTES &&
+                s == Engine::get().stream) {
+                g_free_blocks.push_back({p, bytes, s});
+                g_free_bytes += bytes;
+                return;
+            }
         }
     }
     cudaFreeAsync(p, s);
 }
 
-// free device memory plus what the stream-ordered pool holds cached but unused
+__global__ void words_kernel(u32 *dst, const u32 *src, int words)
+{
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+}
+bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s)
+{
+    words_kernel<<<1, 64, 0, s>>>(pinned, dev, words);
+    return CGB_CUDA(cudaGetLastError());
+}
+
+// free device memory plus what the stream-ordered pool and the kept blocks hold unused
 u64 device_available_bytes(int dev)
 {
     size_t free_b = 0, total_b = 0;
@@ -195,7 +262,8 @@ u64 device_available_bytes(int dev)
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
     }
-    return (u64)free_b + (reserved > used ? reserved - used : 0);
+    std::lock_guard<std::mutex> g(g_mem_mu);
+    return (u64)free_b + (reserved > used ? reserved - used : 0) + g_free_bytes;
 }
 
 // ---- resident layer store ---------------------------------------------------
@@ -204,8 +272,11 @@ bool LayerStore::push(u64 n, cudaStream_t s, Handle *h)
     const u64 need = n ? n : 1;
     if (chunks_.empty() || !chunks_.back().base || chunks_.back().top + need > chunks_.back().cap) {
         Chunk c;
-        c.cap = std::max<u64>(need, chunk_bytes / 8);
+        // the first chunk 64 MB (a small sweep needs no more, and mapping 4 GB takes
+        // 25 ms), each further one as large as all before it, up to chunk_bytes
+        c.cap = std::max<u64>(need, std::min<u64>(chunk_bytes / 8, std::max<u64>(8ull << 20, total)));
         if (!dev_alloc((void **)&c.base, c.cap * 8, s)) return false;
+        total += c.cap;
         chunks_.push_back(std::move(c));
     }
     Chunk &c = chunks_.back();
@@ -337,7 +408,7 @@ bool Engine::init(int dev)
         if (!CGB_CUDA(cudaMalloc(&p, 64 * sizeof(u64)))) return false;
         ctr.d = (u64 *)p;
         ctr.err = (u32 *)(ctr.d + Counters::ERR);
-        if (!CGB_CUDA(cudaHostAlloc((void **)&ctr.host, Counters::HEAD * sizeof(u64), cudaHostAllocDefault))) return false;
+        if (!CGB_CUDA(cudaHostAlloc((void **)&ctr.host, (Counters::HEAD + 1) * sizeof(u64), cudaHostAllocDefault))) return false;
         if (!CGB_CUDA(cudaMemset(p, 0, 64 * sizeof(u64)))) return false;
     }
     ready = true;
@@ -562,7 +633,7 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
     const int np1 = bucket_enqueue(plans[1], 1, g.c[0].p, own + 2, g.c[1].p, true, false, w, s);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError()) ||
-        !CGB_CUDA(cudaMemcpyAsync(w.host, w.ctl.p, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4, cudaMemcpyDeviceToHost, s)) ||
+        !words_to_host(w.host, w.ctl.p, BUCKET_HEADS * BUCKET_HEAD_WORDS, s) ||
         !sync())
         return false;
     kclock().flush();
@@ -660,6 +731,7 @@ void Engine::end_one_shot()
             dev_free(x.p, stream);
             x = IndexStorage{};
         }
+    index_release_scratch(stream);
 }
 
 void Engine::release_buffers()
@@ -669,6 +741,7 @@ void Engine::release_buffers()
         drop(*b, stream);
     ws.buckets.release(stream);
     one_shot.drop(stream);
+    release_blocks();
 }
 
 }  // namespace cgb

@@ -18,6 +18,11 @@ struct DevBuf {
     u64 cap = 0;   // elements allocated
 };
 
+// a few words from the device to pinned memory, visible once the stream has been
+// waited for.  A kernel writes them: a copy would queue in the copy engine behind
+// whatever layers and tables other streams are sending to the host
+bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s);
+
 bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
 void dev_free(void *p, cudaStream_t s);
 template <typename T>
@@ -143,7 +148,7 @@ struct Counters {
     static constexpr int ERR = 6, HEAD = 7;
     u64 *d = nullptr;
     u32 *err = nullptr;   // d + ERR
-    u64 *host = nullptr;  // pinned copy of the first HEAD words
+    u64 *host = nullptr;  // pinned copy of the first HEAD words, then the probes'
 };
 
 // move + prune + canonicalise every board; out needs room for 4n boards
@@ -226,6 +231,11 @@ struct IndexStorage {
     u64 bytes = 0;
 };
 
+// at least `bytes` bytes (what was there is not kept)
+bool ensure_storage(IndexStorage &st, u64 bytes, cudaStream_t s);
+// gives back the scratch that index builds keep for the next
+void index_release_scratch(cudaStream_t s);
+
 // graph-capturable forms (no host round trip): the solve kernel, counting
 // probes into *probes, and the hash index into caller-owned slots
 // (hash_capacity(n) slots of 16 bytes); device errors accumulate in *err
@@ -295,6 +305,15 @@ class LayerStore {
         int chunk = -1;
         u64 off = 0, n = 0;
     };
+    u64 total = 0;                  // boards that all chunks taken so far have room for
+    // whether a chunk of full size has been taken since the last call: before that
+    // there is nothing worth spilling, and the device query that decides costs 2.5 ms
+    bool grown()
+    {
+        const bool yes = total * 8 >= chunk_bytes && chunks_.size() != checked_;
+        if (yes) checked_ = chunks_.size();
+        return yes;
+    }
     bool push(u64 n, cudaStream_t s, Handle *h);      // room for n boards
     u64 *ptr(const Handle &h, cudaStream_t s);         // device address (restores a spilled chunk)
     void release(const Handle &h, cudaStream_t s);     // frees a pushed block
@@ -316,6 +335,7 @@ class LayerStore {
         std::vector<Block> blocks;
     };
     std::vector<Chunk> chunks_;
+    size_t checked_ = 0;
     void drop_chunk(Chunk &c, cudaStream_t s);
 };
 

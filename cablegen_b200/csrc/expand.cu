@@ -395,7 +395,7 @@ static bool clear_counters(Counters &c, cudaStream_t s)
 // ... and come back in one copy
 static bool fetch_counters(Counters &c, cudaStream_t s)
 {
-    return CGB_CUDA(cudaMemcpyAsync(c.host, c.d, Counters::HEAD * sizeof(u64), cudaMemcpyDeviceToHost, s));
+    return words_to_host((u32 *)c.host, (const u32 *)c.d, 2 * Counters::HEAD, s);
 }
 static bool read_counters(Counters &c, cudaStream_t s, const char *what)
 {

@@ -939,6 +939,7 @@ void solve(unsigned start, unsigned end, char *posfmt, char *tablefmt, const sta
     for (Lay *x : {&t2, &t4})
         for (void *p : {(void *)x->keys, x->vals, x->store.p}) cgb::dev_free(p, st);
     cgb::dev_free(d_ws, st);
+    cgb::index_release_scratch(st);
     cudaStreamSynchronize(st);
 }
 

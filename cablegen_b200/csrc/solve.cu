@@ -679,7 +679,7 @@ static int grid_for(u64 n, int threads, int per_sm)
     return (int)std::max<u64>(1, std::min<u64>(need, (u64)sms * per_sm));
 }
 
-static bool ensure_storage(IndexStorage &st, u64 bytes, cudaStream_t s)
+bool ensure_storage(IndexStorage &st, u64 bytes, cudaStream_t s)
 {
     if (st.bytes >= bytes && st.p) return true;
     if (st.p) dev_free(st.p, s);
@@ -700,7 +700,7 @@ bool key_bits(const KeySet &a, const KeySet &b, KeyBits *bits, const u64 *first,
     if (first && !CGB_CUDA(cudaMemcpyAsync(d + 4, first, sizeof(u64), cudaMemcpyDeviceToDevice, s))) return false;
     if (a.n) key_bits_kernel<<<grid_for(a.n, 256, 8), 256, 0, s>>>(a.keys, a.n, (unsigned long long *)d);
     if (b.n) key_bits_kernel<<<grid_for(b.n, 256, 8), 256, 0, s>>>(b.keys, b.n, (unsigned long long *)(d + 2));
-    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(host, d, 5 * sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
+    if (!CGB_CUDA(cudaGetLastError()) || !words_to_host((u32 *)host, (const u32 *)d, 10, s) ||
         !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
     for (int i = 0; i < 2; i++)
@@ -734,7 +734,7 @@ static bool begin_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStr
     compact_build_kernel<<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const float *)ix.vals, ix.n,
                                                                  (unsigned long long *)st.p, ch, cap, index_err(ix, c));
     kclock().end(s);
-    if (!CGB_CUDA(cudaGetLastError()) || !CGB_CUDA(cudaMemcpyAsync(h_index_err + ix.slot, index_err(ix, c), sizeof(u32), cudaMemcpyDeviceToHost, s)))
+    if (!CGB_CUDA(cudaGetLastError()) || !words_to_host(h_index_err + ix.slot, index_err(ix, c), 1, s))
         return false;
     ix.kind = INDEX_HASH;
     ix.slots = st.p;
@@ -743,6 +743,10 @@ static bool begin_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStr
     ix.unchecked = true;
     return true;
 }
+
+// the region-partitioned build's cursors, buckets and overflow list, kept from one
+// build to the next until index_release_scratch
+static IndexStorage region_scratch;
 
 int g_region_build = 1;  // 16-byte-slot indexes of 2^16..2^28 keys built region by region
 
@@ -760,9 +764,8 @@ static bool begin_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
     if (!ensure_storage(st, cap * 16, s)) return false;
     // scratch: the cursors and the overflow count (u32), the region buckets, the overflow list
     const u64 bytes = 4ull * nreg * CURSOR_PAD + 64 + 16ull * nreg * bcap + 16ull * max_over;
-    void *scratch = nullptr;
-    if (!dev_alloc(&scratch, bytes, s)) return false;
-    u32 *cursor = (u32 *)scratch, *n_over = cursor + (u64)nreg * CURSOR_PAD;
+    if (!ensure_storage(region_scratch, bytes, s)) return false;
+    u32 *cursor = (u32 *)region_scratch.p, *n_over = cursor + (u64)nreg * CURSOR_PAD;
     ulonglong2 *tmp = (ulonglong2 *)(((uintptr_t)(n_over + 1) + 15) & ~(uintptr_t)15);
     ulonglong2 *over = tmp + (u64)nreg * bcap;
     bool ok = CGB_CUDA(cudaMemsetAsync(cursor, 0, 4ull * nreg * CURSOR_PAD + 4, s)) && CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, 4, s));
@@ -781,15 +784,20 @@ static bool begin_regions(LayerIndex &ix, int vbytes, IndexStorage &st, Counters
         kclock().end(s);
         kstats().launches += 2;
         ok = CGB_CUDA(cudaGetLastError()) &&
-             CGB_CUDA(cudaMemcpyAsync(h_index_err + ix.slot, index_err(ix, c), sizeof(u32), cudaMemcpyDeviceToHost, s));
+             words_to_host(h_index_err + ix.slot, index_err(ix, c), 1, s);
     }
-    dev_free(scratch, s);
     if (!ok) return false;
     ix.kind = INDEX_HASH;
     ix.slots = st.p;
     ix.cap = cap;
     ix.unchecked = true;
     return true;
+}
+
+void index_release_scratch(cudaStream_t s)
+{
+    dev_free(region_scratch.p, s);
+    region_scratch = IndexStorage{};
 }
 
 // launches the atomic build into a zeroed table, which cannot fail: the table
@@ -986,8 +994,8 @@ bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const Lay
 
 bool solve_collect(Counters &c, cudaStream_t s)
 {
-    u64 probes = 0;
-    if (!CGB_CUDA(cudaMemcpyAsync(&probes, c.d + PROBES_AT, sizeof(u64), cudaMemcpyDeviceToHost, s)) ||
+    u64 &probes = c.host[Counters::HEAD];
+    if (!words_to_host((u32 *)&probes, (const u32 *)(c.d + PROBES_AT), 2, s) ||
         !CGB_CUDA(cudaMemsetAsync(c.d + PROBES_AT, 0, sizeof(u64), s)) || !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
     kclock().flush();

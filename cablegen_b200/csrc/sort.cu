@@ -1037,8 +1037,7 @@ static bool clear_state(SortWorkspace &ws, u64 words, cudaStream_t s)
 // the error word and the counts on the host
 static bool fetch_state(SortWorkspace &ws, cudaStream_t s)
 {
-    return CGB_CUDA(cudaMemcpyAsync(ws.host + W_ERR, ws.small + W_ERR, (W_EMPTIES + 2 - W_ERR) * sizeof(u32),
-                                    cudaMemcpyDeviceToHost, s)) &&
+    return words_to_host(ws.host + W_ERR, ws.small + W_ERR, W_EMPTIES + 2 - W_ERR, s) &&
            CGB_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -1316,7 +1315,7 @@ bool partition_by_formation(const u64 *in, u64 n, u64 *out, const unsigned char 
                                                           ws.lookback, ws.small + W_CTR, ws.small + W_ERR);
     kstats().launches += 2;
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    if (!CGB_CUDA(cudaMemcpyAsync(ws.host + W_HIST, ws.small + W_HIST, 256 * sizeof(u32), cudaMemcpyDeviceToHost, s)) ||
+    if (!words_to_host(ws.host + W_HIST, ws.small + W_HIST, 256, s) ||
         !fetch_state(ws, s))
         return false;
     memcpy(counts, ws.host + W_HIST, 256 * sizeof(u32));

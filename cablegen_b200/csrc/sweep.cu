@@ -59,7 +59,6 @@ struct StoreSink : LayerSink {
     void *user = nullptr;
     AsyncOut *out = nullptr;
     u64 reserve_bytes = 0;
-    size_t checked_at = 0;  // store chunks at the last free-memory check
     int device = 0;
     HostArena *host = nullptr;  // set when layers and tables both go to the host
     u64 host_cap = 0;
@@ -114,13 +113,11 @@ struct StoreSink : LayerSink {
         layers.push_back(L);
         // keep room for the next layer steps: the working set grows with the
         // layer, so the reserve scales with it
-        // (the device query is not free: ask only when the store took a new chunk)
-        if (store.chunk_count() != checked_at) {
+        if (store.grown()) {
             const u64 want = reserve_bytes + 12 * n * 8;
             const u64 avail = device_available_bytes(device);
             // false when nothing is left to spill: carry on, an allocation may still fit
             if (avail < want) store.spill(want - avail, s, out->io);
-            checked_at = store.chunk_count();
         }
         return true;
     }
@@ -138,12 +135,17 @@ struct Chain {
         int vb = 8;  // bytes per value of this layer's table
         const u64 *keys = nullptr;
         void *vals = nullptr;
+        IndexStorage room;      // the memory behind vals
         u64 n = 0;
         KeyBits bits;
         IndexStorage store;
         LayerIndex ix;
     };
     Solved t2, t4, cur;
+    // memory of the layer that left last, for the next one: three layers' tables
+    // take turns in the same blocks.  Allocating and freeing hundreds of MB a layer
+    // left the allocator's pool in pieces, and growing it costs milliseconds.
+    IndexStorage spare_room, spare_store;
 
     int layer_vbytes(int sum) const { return vbytes == 4 && sum > fp64_above ? 8 : vbytes; }
 
@@ -154,7 +156,8 @@ struct Chain {
         void *f = nullptr;
         if (!dev_alloc(&f, x.n * 4 + 8, s)) return false;
         if (x.n && !narrow_values((const double *)x.vals, (float *)f, x.n, s)) return false;
-        dev_free(x.vals, s);
+        dev_free(x.room.p, s);
+        x.room = IndexStorage{f, x.n * 4 + 8};
         x.vals = f;
         x.vb = 4;
         x.ix.keys = x.keys;
@@ -166,7 +169,9 @@ struct Chain {
     {
         cur.vb = layer_vbytes(cur.sum);
         if (cur.vb == 4 && !(narrow(e, t2, s) && narrow(e, t4, s))) return false;
-        if (!dev_alloc(&cur.vals, cur.n * cur.vb + 8, s)) return false;
+        std::swap(cur.room, spare_room);
+        if (!ensure_storage(cur.room, cur.n * cur.vb + 8, s)) return false;
+        cur.vals = cur.room.p;
         return solve_layer_launch(cur.keys, cur.n, cur.vals, cur.vb, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan);
     }
     // launches the index build of the solved layer; finish_index waits for it
@@ -175,23 +180,35 @@ struct Chain {
         cur.ix.keys = cur.keys;
         cur.ix.vals = cur.vals;
         cur.ix.n = cur.n;
+        std::swap(cur.store, spare_store);
         return index_begin(cur.ix, e.index_kind, cur.vb, cur.store, e.bucket_bits, e.ctr, s, cur.bits);
     }
     bool finish_index(Engine &e, cudaStream_t s) { return index_finish(cur.ix, cur.vb, cur.store, e.ctr, s); }
     void rotate(cudaStream_t s)
     {
-        if (t4.vals) dev_free(t4.vals, s);
-        if (t4.store.p) dev_free(t4.store.p, s);
+        keep(t4.room, spare_room, s);
+        keep(t4.store, spare_store, s);
         t4 = t2;
         t2 = cur;
         cur = Solved{};
     }
+    // the larger of a block that is free and the one kept so far
+    void keep(IndexStorage &x, IndexStorage &spare, cudaStream_t s)
+    {
+        if (x.bytes > spare.bytes) std::swap(x, spare);
+        dev_free(x.p, s);
+        x = IndexStorage{};
+    }
     void release(cudaStream_t s)
     {
         for (Solved *x : {&t2, &t4, &cur}) {
-            if (x->vals) dev_free(x->vals, s);
-            if (x->store.p) dev_free(x->store.p, s);
+            dev_free(x->room.p, s);
+            dev_free(x->store.p, s);
             *x = Solved{};
+        }
+        for (IndexStorage *x : {&spare_room, &spare_store}) {
+            dev_free(x->p, s);
+            *x = IndexStorage{};
         }
     }
 };
@@ -385,6 +402,7 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
     out.fence_main();
     if (!solve_collect(e.ctr, s)) ok = false;
     for (auto &c : chains) c.release(s);
+    index_release_scratch(s);
     sink.store.clear(s);
     dev_free(d_ws, s);
     dev_free(d_err, s);

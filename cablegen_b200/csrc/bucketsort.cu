@@ -18,7 +18,8 @@
 //                 network, then merge-path merges -- drops repeats when asked
 //                 (equal keys always share a bucket) and writes at the offset
 //                 that a look-back over the buckets' counts gives.
-// Inputs of up to 4096 keys go straight to step 3 as one bucket.
+// Inputs of up to 16384 keys are one bucket, sorted by one CTA of 1024 threads
+// (of 256 up to 4096 keys).
 //
 // Bounds: the partition is bound by its shared-memory accesses (50 wavefronts
 // per 32 keys: search, counters, staging; 62 % of the peak), the bucket sort by
@@ -51,6 +52,8 @@ constexpr int SPLIT_THREADS = 512;
 constexpr u32 BK_SAMPLES = 8192;
 constexpr int PART_THREADS = 256;
 constexpr int BUCKET_THREADS = 256;
+constexpr int SMALL_THREADS = 1024;
+constexpr u32 BK_SMALL = SMALL_THREADS * BK_KPT;  // keys that one CTA sorts in a single launch
 
 constexpr u64 KEY_MAX = ~0ull;
 constexpr u32 BK_OVERFLOW = 1u << 16;   // a bucket ran full (beside the ERR_* bits)
@@ -70,7 +73,7 @@ struct KeyCount {
 };
 
 __device__ __forceinline__ u32 pad16(u32 i) { return i + (i >> 4); }
-constexpr u32 SAMPLE_WORDS = BK_SAMPLES + BK_SAMPLES / 16, BUCKET_WORDS = BK_CAP + BK_CAP / 16;
+constexpr u32 SAMPLE_WORDS = BK_SAMPLES + BK_SAMPLES / 16;
 
 // ---- sorting inside a CTA ---------------------------------------------------
 // Keys are u64, or u32 where a bucket's keys differ in at most 32 bits.
@@ -491,13 +494,15 @@ __global__ void __launch_bounds__(PART_THREADS, 4)
     }
 }
 
+template <int THREADS>
 struct BucketSmem {
+    static constexpr u32 WORDS = THREADS * BK_KPT + THREADS;  // padded
     union {
-        u64 wide[BUCKET_WORDS];
-        u32 narrow[BUCKET_WORDS];
+        u64 wide[WORDS];
+        u32 narrow[WORDS];
     };
-    u64 last64[BUCKET_THREADS];
-    u32 warp[BUCKET_THREADS / 32];
+    u64 last64[THREADS];
+    u32 warp[THREADS / 32];
     u32 and_or[4];
     BitMoves lo, hi;
     u32 tile, prefix, kept;
@@ -505,9 +510,9 @@ struct BucketSmem {
 
 // Everything after the sort key type is known: sort, flag the keys to keep,
 // their offset by look-back, write.  EMIT turns a sorted key into the u64.
-template <bool UNIQUE, bool DIRECT, typename K, class Emit>
+template <bool UNIQUE, bool DIRECT, int THREADS, typename K, class Emit>
 __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh, u32 cnt, u32 tile, u32 tiles, u32 *look,
-                                              u32 *head, u64 *__restrict__ out, u32 count_empties, BucketSmem &S, Emit emit)
+                                              u32 *head, u64 *__restrict__ out, u32 count_empties, BucketSmem<THREADS> &S, Emit emit)
 {
     constexpr u32 ALL = 0xffffffffu;
     constexpr u32 AGG = 1u << 30, PRE = 2u << 30;
@@ -534,7 +539,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
     if (lane == 31) S.warp[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        const u32 c = lane < BUCKET_THREADS / 32 ? S.warp[lane] : 0u;
+        const u32 c = lane < THREADS / 32 ? S.warp[lane] : 0u;
         const u32 wi = warp_inclusive_scan(c);
         const u32 total = __shfl_sync(ALL, wi, 31);
         u32 prefix = 0;
@@ -545,7 +550,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
             }
             if (lane == 0) st_relaxed(look + tile, PRE | (prefix + total));
         }
-        if (lane < BUCKET_THREADS / 32) S.warp[lane] = wi - c;
+        if (lane < THREADS / 32) S.warp[lane] = wi - c;
         if (lane == 0) {
             S.prefix = prefix;
             S.kept = total;
@@ -563,7 +568,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
     __syncthreads();
     const u32 prefix = S.prefix, num = S.kept;
     u32 empty = 0;
-    for (u32 j = t; j < num; j += BUCKET_THREADS) {
+    for (u32 j = t; j < num; j += THREADS) {
         const u64 key = emit(buf[pad16(j)]);
         out[prefix + j] = key;
         if (UNIQUE && count_empties) empty += zero_nibbles(key);
@@ -585,25 +590,12 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
 // them.  Such a bucket is sorted as u32 keys of those bits alone, where a
 // compare-exchange is two instructions instead of six (the low words as they
 // are where the high words agree); the others are sorted as they are.
-template <bool UNIQUE, bool DIRECT>
-__global__ void __launch_bounds__(BUCKET_THREADS, 4)
-    bucket_sort_kernel(const u64 *__restrict__ input, KeyCount n, const u64 *__restrict__ slots, u32 counters, u32 words,
-                       u32 *head, u32 *arrays, u64 *__restrict__ out, u32 count_empties)
+template <bool UNIQUE, bool DIRECT, int THREADS>
+__device__ __forceinline__ void sort_bucket(const u64 *__restrict__ src, u32 cnt, u32 tile, u32 tiles, u32 *look, u32 *head,
+                                            u64 *__restrict__ out, u32 count_empties, BucketSmem<THREADS> &S)
 {
     constexpr u32 ALL = 0xffffffffu;
-    __shared__ BucketSmem S;
     const u32 t = threadIdx.x;
-    if (t == 0 && !DIRECT) S.tile = atomicAdd(head + H_TICKET, 1u);
-    if (t < 4) S.and_or[t] = t < 2 ? ALL : 0u;
-    const u32 all = n.get();
-    const bool whole = DIRECT || all <= BK_CAP;
-    __syncthreads();
-    const u32 tile = DIRECT ? 0 : S.tile, tiles = whole ? 1 : head[H_BUCKETS];
-    if (!DIRECT && (tile >= tiles || head[H_FLAGS])) return;
-    const u32 cnt = whole ? all : arrays[counters + tile];
-    u32 *look = arrays + words;
-    if (!UNIQUE && t == 0 && tile > 0) st_relaxed(look + tile, (1u << 30) | cnt);
-    const u64 *src = whole ? input : slots + (u64)tile * BK_CAP;
     u64 k[BK_KPT];
     u64 a = KEY_MAX, o = 0;
     const bool on = (t & ~31u) * BK_KPT < cnt;
@@ -635,8 +627,8 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
         u32 v[BK_KPT];
 #pragma unroll
         for (int i = 0; i < BK_KPT; i++) v[i] = (u32)k[i];  // KEY_MAX beyond cnt
-        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
-                                      [=](u32 x) { return make64(high, x); });
+        finish_bucket<UNIQUE, DIRECT, THREADS>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out,
+                                               count_empties, S, [=](u32 x) { return make64(high, x); });
     } else if (low + __popc(vary_hi) <= 32) {
         if (t == 0) plan_moves(vary_lo, &S.lo);
         if (t == 32) plan_moves(vary_hi, &S.hi);
@@ -648,12 +640,51 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
 #pragma unroll
             for (int i = 0; i < BK_KPT; i++) v[i] = warp_key(i) < cnt ? narrow_key(k[i], lo, hi, low) : ALL;
         }
-        finish_bucket<UNIQUE, DIRECT>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
-                                      [&](u32 x) { return wide_key(x, S.lo, S.hi, low) | fixed; });
+        finish_bucket<UNIQUE, DIRECT, THREADS>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out,
+                                               count_empties, S,
+                                               [&](u32 x) { return wide_key(x, S.lo, S.hi, low) | fixed; });
     } else {
-        finish_bucket<UNIQUE, DIRECT>(k, S.wide, S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
-                                      [](u64 x) { return x; });
+        finish_bucket<UNIQUE, DIRECT, THREADS>(k, S.wide, S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
+                                               [](u64 x) { return x; });
     }
+}
+
+template <bool UNIQUE, bool DIRECT>
+__global__ void __launch_bounds__(BUCKET_THREADS, 4)
+    bucket_sort_kernel(const u64 *__restrict__ input, KeyCount n, const u64 *__restrict__ slots, u32 counters, u32 words,
+                       u32 *head, u32 *arrays, u64 *__restrict__ out, u32 count_empties)
+{
+    __shared__ BucketSmem<BUCKET_THREADS> S;
+    const u32 t = threadIdx.x;
+    const u32 all = n.get();
+    if (t == 0 && !DIRECT) S.tile = atomicAdd(head + H_TICKET, 1u);
+    if (t < 4) S.and_or[t] = t < 2 ? 0xffffffffu : 0u;
+    const bool whole = DIRECT || all <= BK_CAP;
+    __syncthreads();
+    const u32 tile = DIRECT ? 0 : S.tile, tiles = whole ? 1 : head[H_BUCKETS];
+    if (!DIRECT && (tile >= tiles || head[H_FLAGS])) return;
+    const u32 cnt = whole ? all : arrays[counters + tile];
+    u32 *look = arrays + words;
+    if (!UNIQUE && t == 0 && tile > 0) st_relaxed(look + tile, (1u << 30) | cnt);
+    const u64 *src = whole ? input : slots + (u64)tile * BK_CAP;
+    sort_bucket<UNIQUE, DIRECT, BUCKET_THREADS>(src, cnt, tile, tiles, look, head, out, count_empties, S);
+}
+
+// Up to 16384 keys in one CTA of 1024 threads: a launch in place of three, whose
+// kernels would each leave the chip idle.  The two sorts of the 149 layers of the
+// 2x4 table (3400 moves and 14000 spawns each): 7.8 -> 6.0 ms.
+template <bool UNIQUE>
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+    small_sort_kernel(const u64 *__restrict__ input, KeyCount n, u32 *head, u64 *__restrict__ out, u32 count_empties)
+{
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    BucketSmem<SMALL_THREADS> &S = *reinterpret_cast<BucketSmem<SMALL_THREADS> *>(small_smem);
+    const u32 cnt = n.get();
+    if (cnt > BK_SMALL && threadIdx.x == 0) head[H_FLAGS] = BK_OVERFLOW;
+    if (cnt == 0 || cnt > BK_SMALL) return;
+    if (threadIdx.x < 4) S.and_or[threadIdx.x] = threadIdx.x < 2 ? 0xffffffffu : 0u;
+    __syncthreads();
+    sort_bucket<UNIQUE, true, SMALL_THREADS>(input, cnt, 0, 1, nullptr, head, out, count_empties, S);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,6 +706,8 @@ static bool attributes()
     const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
     done = CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<false>, smem, split)) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_split_kernel<true>, smem, split)) &&
+           CGB_CUDA(cudaFuncSetAttribute(small_sort_kernel<false>, smem, (int)sizeof(BucketSmem<SMALL_THREADS>))) &&
+           CGB_CUDA(cudaFuncSetAttribute(small_sort_kernel<true>, smem, (int)sizeof(BucketSmem<SMALL_THREADS>))) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<false>, smem, part)) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<true>, smem, part));
     return done;
@@ -706,15 +739,16 @@ static bool plan_buckets(u64 n, BucketPlan *p)
     return true;
 }
 
-bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s)
+bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s, const u64 *likely)
 {
     u64 words = BUCKET_HEADS * BUCKET_HEAD_WORDS, fine = 0, coarse = 0, bounds = 0;
     for (int i = 0; i < calls; i++) {
         BucketPlan &p = plans[i];
         if (!plan_buckets(n[i], &p)) return false;
+        p.small = (likely && likely[i] <= BK_SMALL) || (n[i] > BK_CAP && n[i] <= BK_SMALL);
         p.arrays_at = words;
         words += (p.words + 1) / 2 * 2;
-        if (p.n <= BK_CAP) continue;
+        if (p.n <= BK_CAP || p.small) continue;
         fine = std::max(fine, (u64)p.grid * BK_CAP);
         coarse = std::max(coarse, (u64)p.coarse * p.coarse_cap);
         bounds = std::max(bounds, (u64)BK_FAN * (p.coarse + 1));
@@ -751,6 +785,12 @@ int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *co
     const KeyCount kc{(u32)p.n, counted};
     const u32 tiles = (u32)((p.n + BK_TILE - 1) / BK_TILE);
     int np = 1;
+    if (p.small) {
+        constexpr u32 smem = sizeof(BucketSmem<SMALL_THREADS>);
+        if (unique) small_sort_kernel<true><<<1, SMALL_THREADS, smem, s>>>(keys, kc, head, out, empties);
+        else small_sort_kernel<false><<<1, SMALL_THREADS, smem, s>>>(keys, kc, head, out, 0);
+        return np;
+    }
     if (p.n > BK_CAP) {
         bucket_split_kernel<false><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, p.coarse, 0, head, arrays, w.bounds.p);
         bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(

@@ -123,7 +123,7 @@ struct GenBuffers {
     static constexpr u64 UNKNOWN = ~0ull;
     u64 moved_empties = UNKNOWN, prev_empties = 0;
     KeyBits moved_bits;        // AND and OR of the moved layer, where its sort gave them
-    double spawn_ratio = 16;   // spawns per board of S in the last layer step
+    double spawn_ratio = 16, move_ratio = 4;  // spawns and moves per board of S in the last layer step
 };
 
 // device memory of the calls that solve or look up one layer, kept for the next

@@ -615,7 +615,8 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
     if (!reserve(g.a, 4 * n, s) || !reserve(g.b, 4 * n, s) || !reserve(g.c[0], room, s) || !reserve(g.c[1], room, s))
         return false;
     BucketWorkspace &w = ws.buckets;
-    if (!bucket_prepare(sizes, 2, plans, w, s)) return true;
+    const u64 likely[2] = {(u64)(1.25 * (double)n * g.move_ratio), (u64)(1.25 * (double)n * g.spawn_ratio)};
+    if (!bucket_prepare(sizes, 2, plans, w, s, likely)) return true;
     // the third head: counts of moves, raw moves and spawns, error word
     constexpr u32 OWN = 2 * BUCKET_HEAD_WORDS;
     u64 *own = (u64 *)(w.ctl.p + OWN);
@@ -645,6 +646,7 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
         set_error("layer step: device error " + err_string(bad));
         return false;
     }
+    g.move_ratio = std::max(0.25, (double)counts[0] / (double)n);
     if (moves.overflow) return true;
     KernelStats &k = kstats();
     auto sorted = [&](u64 keys, int passes) {
@@ -691,6 +693,7 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
     g.u4.n = n_carry;
     g.prev.n = g.prev_empties = 0;
     g.spawn_ratio = 16;
+    g.move_ratio = 4;
     // canonical layer boards share the 0xf mask of the canonical first board (fixed
     // formation cells); the kernels check every board against it
     plan = (n_init && !filter.fid) ? make_canon_plan(canonical(h_initial[0]), rules.free_formation != 0) : CanonPlan{};

@@ -64,6 +64,7 @@ struct BucketWorkspace {
 constexpr u32 BUCKET_COUNT_AT = 4;  // head word of the 64-bit number of keys written
 struct BucketPlan {
     u64 n = 0;              // keys at most
+    bool small = false;     // expected to fit one CTA: nothing but its sort is launched
     u32 coarse = 0, coarse_cap = 0;  // two steps: coarse buckets and their space
     u32 grid = 0;           // buckets at most
     u64 words = 0, arrays_at = 0;
@@ -76,10 +77,12 @@ struct BucketResult {
 };
 // The parts of bucket_sort, for callers that put several sorts into one stream
 // without a wait: plans and room for `calls` sorts of at most n[i] keys (false:
-// too many keys or no memory), one clear of all control words, the launches of
+// too many keys or no memory; likely[i], if given: the number to expect, an
+// overflow being reported where a sort was launched for far fewer), one clear of all control words, the launches of
 // one sort (the number of keys read from *counted where that is not null;
 // returns the passes), and, once the heads have been copied to w.host, the result.
-bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s);
+bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s,
+                    const u64 *likely = nullptr);
 bool bucket_clear(BucketWorkspace &w, cudaStream_t s);
 int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,
                    BucketWorkspace &w, cudaStream_t s);

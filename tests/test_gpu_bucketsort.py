@@ -1,5 +1,5 @@
 """The sort by sampled buckets (csrc/bucketsort.cu) against numpy at the sizes where it changes
-form -- one bucket (up to 4096 keys), one partition step (up to 400 x 1800 keys), two steps -- for
+form -- one bucket (up to 4096 and up to 16384 keys), one partition step (up to 400 x 1800 keys), two steps -- for
 keys whose buckets differ in the low word alone, in at most 32 bits of both words, and in more; keys
 with repeats; and inputs it hands on to the digit passes (a bucket that cannot hold its repeats)."""
 import numpy as np
@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-ONE, TWO = 4096, 400 * 1800
+ONE, SMALL, TWO = 4096, 16384, 400 * 1800
 
 
 def keys(kind, n):
@@ -31,7 +31,7 @@ def keys(kind, n):
 
 
 @pytest.mark.parametrize("kind", ["low", "nibbles", "wide", "repeats", "sorted", "heavy"])
-@pytest.mark.parametrize("n", [2, 15, 17, 511, 513, 2049, ONE, ONE + 1, 9001, TWO, TWO + 1, 3_000_017])
+@pytest.mark.parametrize("n", [2, 15, 17, 511, 513, 2049, ONE, ONE + 1, 9001, SMALL, SMALL + 1, TWO, TWO + 1, 3_000_017])
 def test_bucket_sort(cuda, kind, n):
     x = keys(kind, n)
     got, _ = cuda.sort(cuda.to_device(x))

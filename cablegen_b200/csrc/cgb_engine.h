@@ -170,7 +170,7 @@ struct Engine {
     // layers of at most so many boards to move take quick_step: above, kernels
     // of a millisecond hide the waits
     static constexpr u64 QUICK_BOARDS = 1u << 21;
-    bool quick_step(GenTimes *tm, bool *moved_done, bool *done);
+    bool quick_step(GenTimes *tm, bool last, bool *moved_done, bool *done);
     bool next_inputs(GenTimes *tm);     // g.S from the spawns of g.moved and g.prev
     bool sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
                           u64 *empties = nullptr, KeyBits *bits = nullptr);

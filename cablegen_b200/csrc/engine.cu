@@ -600,15 +600,16 @@ bool Engine::next_inputs(GenTimes *tm)
 // A small layer's kernels take 10-20 us each, and three waits with their launches
 // behind them cost as much again.  The spawns' room is a guess from the last layer;
 // where it or a bucket overflows, *done stays false or only the moved layer is
-// taken, and the step with waits does the rest.
-bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
+// taken, and the step with waits does the rest.  After the last layer no input set
+// is wanted.
+bool Engine::quick_step(GenTimes *tm, bool last, bool *moved_done, bool *done)
 {
     *moved_done = *done = false;
     cudaStream_t s = stream;
     GenBuffers &g = gen;
     const u64 n = g.S.n;
     if (n == 0 || n > QUICK_BOARDS || g.u4.n || !bucket_sorts() || 4 * n > max_sort_keys) return true;
-    const u64 room = std::max<u64>(1 << 14, (u64)(1.5 * (double)n * g.spawn_ratio));
+    const u64 room = last ? 1 : std::max<u64>(1 << 14, (u64)(1.5 * (double)n * g.spawn_ratio));
     if (room > max_sort_keys) return true;
     const u64 sizes[2] = {4 * n, room};
     BucketPlan plans[2];
@@ -616,7 +617,7 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
         return false;
     BucketWorkspace &w = ws.buckets;
     const u64 likely[2] = {(u64)(1.25 * (double)n * g.move_ratio), (u64)(1.25 * (double)n * g.spawn_ratio)};
-    if (!bucket_prepare(sizes, 2, plans, w, s, likely)) return true;
+    if (!bucket_prepare(sizes, last ? 1 : 2, plans, w, s, likely)) return true;
     // the third head: counts of moves, raw moves and spawns, error word
     constexpr u32 OWN = 2 * BUCKET_HEAD_WORDS;
     u64 *own = (u64 *)(w.ctl.p + OWN);
@@ -628,10 +629,13 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
     if (!expand_moves_enqueue(g.S.p, n, g.a.p, 4 * n, rt, prune_params(), own, own + 1, err, s, filter, plan)) return false;
     kclock().next(s, &kstats().onesweep_ms);
     const int np0 = bucket_enqueue(plans[0], 0, g.a.p, own, g.b.p, true, true, w, s);
-    kclock().next(s, &kstats().spawn_ms);
-    if (!expand_next_enqueue(two, four, g.c[0].p, room, own + 2, err, s, plan)) return false;
-    kclock().next(s, &kstats().onesweep_ms);
-    const int np1 = bucket_enqueue(plans[1], 1, g.c[0].p, own + 2, g.c[1].p, true, false, w, s);
+    int np1 = 0;
+    if (!last) {
+        kclock().next(s, &kstats().spawn_ms);
+        if (!expand_next_enqueue(two, four, g.c[0].p, room, own + 2, err, s, plan)) return false;
+        kclock().next(s, &kstats().onesweep_ms);
+        np1 = bucket_enqueue(plans[1], 1, g.c[0].p, own + 2, g.c[1].p, true, false, w, s);
+    }
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError()) ||
         !words_to_host(w.host, w.ctl.p, BUCKET_HEADS * BUCKET_HEAD_WORDS, s) ||
@@ -666,6 +670,7 @@ bool Engine::quick_step(GenTimes *tm, bool *moved_done, bool *done)
     g.moved_empties = moves.empties;
     g.moved_bits = moves.bits;
     *moved_done = true;
+    if (last) return *done = true;
     const u64 total = g.moved_empties + g.prev_empties;
     g.spawn_ratio = std::max(1.0, (double)total / (double)n);
     if (total > room || next.overflow) return true;
@@ -699,11 +704,13 @@ bool Engine::generate(const u64 *h_initial, u64 n_init, int start, int end, Laye
     plan = (n_init && !filter.fid) ? make_canon_plan(canonical(h_initial[0]), rules.free_formation != 0) : CanonPlan{};
     bool ok = true;
     for (int layer = start; layer <= end && ok; layer += 2) {
+        // the input set of the layer after the last is made for a checkpoint only
+        const bool carry = sink.wants_carry(), last = layer + 2 > end && !carry;
         bool moved = false, next = false;
-        ok = quick_step(tm, &moved, &next) && (moved || move_layer(g.S.p, g.S.n, tm)) && (next || next_inputs(tm));
+        ok = quick_step(tm, last, &moved, &next) && (moved || move_layer(g.S.p, g.S.n, tm)) &&
+             (next || last || next_inputs(tm));
         if (!ok) break;
         if (tm) tm->boards += g.moved.n;
-        const bool carry = sink.wants_carry();
         if (carry)
             ok = reserve(g.u4, 1, s) && spawn_into(SpawnSource{g.moved.p, g.moved.n, 2, g.moved_empties}, g.u4, tm);
         ok = ok && sink.layer(layer, g.moved.p, g.moved.n, s);

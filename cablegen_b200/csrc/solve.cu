@@ -127,7 +127,7 @@ __device__ __forceinline__ V table_value(const DevTable<V> &t, u64 key)
     }
     if (t.kind == INDEX_HASH) {
         if (t.cap == 0) return V(0);
-        const u64 s = home_pair(key, t.cap);
+        const u64 s = home_slot(key, t.cap);
         const ulonglong2 e = __ldg(t.slots + s);
         if (e.x == key) return from_bits<V>(e.y);
         if (e.x == 0) return V(0);
@@ -231,7 +231,7 @@ __device__ __forceinline__ void probe4(const DevTable<V> &t, const u64 *key, u32
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const bool on = (legal >> j) & 1 && t.cap;
-            s[j] = on ? home_pair(key[j], t.cap) : 0;
+            s[j] = on ? home_slot(key[j], t.cap) : 0;
             e[j] = on ? __ldg(t.slots + s[j]) : make_ulonglong2(0, 0);
         }
 #pragma unroll
@@ -291,7 +291,7 @@ __device__ __forceinline__ V probe1(const DevTable<V> &t, u64 key, bool legal)
     }
     if (t.kind == INDEX_HASH) {
         if (t.cap == 0) return V(0);
-        const u64 s = home_pair(key, t.cap);
+        const u64 s = home_slot(key, t.cap);
         const ulonglong2 e = __ldg(t.slots + s);
         if (e.x == key) return from_bits<V>(e.y);
         if (e.x == 0) return V(0);
@@ -332,7 +332,7 @@ __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int
         probes += (u32)ok2 + (u32)ok4;
         V v2 = V(0), v4 = V(0);
         if (wide) {
-            const u64 s2 = home_pair(c2, t2.cap), s4 = home_pair(c4, t4.cap);
+            const u64 s2 = home_slot(c2, t2.cap), s4 = home_slot(c4, t4.cap);
             ulonglong2 e2 = make_ulonglong2(0, 0), e4 = e2;
             if (ok2) e2 = __ldg(t2.slots + s2);
             if (ok4) e4 = __ldg(t4.slots + s4);
@@ -496,7 +496,7 @@ __global__ void hash_build_kernel(const u64 *__restrict__ keys, const V *__restr
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
         const u64 key = keys[i];
-        u64 s = home_pair(key, cap);
+        u64 s = home_slot(key, cap);
         bool placed = false;
         for (u64 p = 0; p < cap; p++) {
             const u64 prev = atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)key);
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(256) region_scatter_kernel(const u64 *__restri
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            r[u] = (u32)(home_pair(key[u], cap) / BUILD_REGION);
+            r[u] = (u32)(home_slot(key[u], cap) / BUILD_REGION);
             p[u] = i0 + u * stride < n ? atomicAdd(cursor + r[u] * CURSOR_PAD, 1u) : 0u;
         }
 #pragma unroll
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256) region_build_kernel(const ulonglong2 *__r
         for (u32 j = threadIdx.x; j < cnt; j += blockDim.x) {
             const ulonglong2 e = bucket[j];
             bool placed = false;
-            for (u32 sl = (u32)(home_pair(e.x, cap) - base); sl < len; sl++) {
+            for (u32 sl = (u32)(home_slot(e.x, cap) - base); sl < len; sl++) {
                 if (atomicCAS((unsigned long long *)&tab[sl].x, 0ull, (unsigned long long)e.x) == 0ull) {
                     tab[sl].y = e.y;
                     placed = true;
@@ -655,7 +655,7 @@ __global__ void overflow_insert_kernel(const ulonglong2 *__restrict__ over, cons
     const u32 n = min(*n_over, max_over);
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const ulonglong2 e = over[i];
-        u64 s = home_pair(e.x, cap);
+        u64 s = home_slot(e.x, cap);
         bool placed = false;
         for (u64 p = 0; p < cap; p++) {
             if (atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)e.x) == 0ull) {

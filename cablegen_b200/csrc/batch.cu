@@ -89,11 +89,11 @@ struct BatchSink : LayerSink {
     int step = 0;
     u64 reserve_bytes = 0;
 
-    bool set_active(cudaStream_t s)
+    bool before(int sum, cudaStream_t s) override  // sums count 0, 2, 4 ... here
     {
         bool changed = false;
         for (size_t f = 0; f < plans->size(); f++) {
-            const unsigned char a = step < (*plans)[f].steps ? 1 : 0;
+            const unsigned char a = sum / 2 < (*plans)[f].steps ? 1 : 0;
             changed |= active[f] != a;
             active[f] = a;
         }
@@ -146,7 +146,6 @@ struct BatchSink : LayerSink {
                 return false;
         }
         step++;
-        if (!set_active(s)) return false;
         // keep room for the next steps (older steps move to pinned host memory)
         if (store.grown()) {
             const u64 want = reserve_bytes + 12 * n * 8;
@@ -266,7 +265,6 @@ bool run_group(Engine &e, const cgb_batch *b, std::vector<Plan> &plans, cgb_batc
     cudaEvent_t ev[3];
     for (auto &x : ev) cudaEventCreate(&x);
     cudaEventRecord(ev[0], s);
-    if (ok) ok = sink.set_active(s);
     e.filter = FormationFilter{d_tab, d_tab + off_active};
     if (ok && max_steps > 0) ok = e.generate(init.data(), init.size(), 0, 2 * (max_steps - 1), sink, &tm);
     e.filter = FormationFilter{};

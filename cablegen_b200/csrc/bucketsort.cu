@@ -812,9 +812,9 @@ int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *co
     return np;
 }
 
-BucketResult bucket_result(const BucketWorkspace &w, int slot)
+BucketResult bucket_result(const u32 *heads, int slot)
 {
-    const u32 *h = w.host + slot * BUCKET_HEAD_WORDS;
+    const u32 *h = heads + slot * BUCKET_HEAD_WORDS;
     BucketResult r;
     r.error = h[H_FLAGS] & ~BK_OVERFLOW;
     r.overflow = (h[H_FLAGS] & BK_OVERFLOW) != 0;
@@ -843,7 +843,7 @@ bool bucket_sort(const u64 *keys, u64 n, u64 *out, bool unique, u64 *n_out, u64 
         !CGB_CUDA(cudaStreamSynchronize(s)))
         return false;
     kclock().flush();
-    const BucketResult r = bucket_result(w, 0);
+    const BucketResult r = bucket_result(w.host, 0);
     if (r.error) {
         set_error("bucket_sort: device error " + err_string(r.error));
         return false;

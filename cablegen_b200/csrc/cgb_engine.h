@@ -42,7 +42,10 @@ struct GenTimes {
 // receives each generated layer (device pointer, valid on stream s)
 struct LayerSink {
     virtual ~LayerSink() {}
-    // the buffer is reused by the layer after next
+    // called before the first kernel of layer `sum` is launched
+    virtual bool before(int sum, cudaStream_t s) { (void)sum, (void)s; return true; }
+    // the buffer is reused by the layer after next; the next layer's kernels may
+    // have been launched by now (not with wants_carry)
     virtual bool layer(int sum, u64 *d_boards, u64 n, cudaStream_t s) = 0;
     // whether gen.u4 shall hold the layer's 4-spawns (sorted, unique) at the call
     virtual bool wants_carry() const { return false; }
@@ -126,6 +129,14 @@ struct GenBuffers {
     double spawn_ratio = 16, move_ratio = 4;  // spawns and moves per board of S in the last layer step
 };
 
+// a layer step in flight (Engine::quick_launch): its sizes as they were planned
+struct QuickStep {
+    bool on = false;      // launched and not yet taken
+    u64 room = 0;         // spawns that there is room for
+    int passes[2] = {0, 0};
+    u32 *host = nullptr;  // pinned copy of the step's control words
+};
+
 // device memory of the calls that solve or look up one layer, kept for the next
 // such call up to KEEP bytes an index: allocating and freeing hundreds of MB costs
 // a call more than its copies and launches
@@ -170,7 +181,9 @@ struct Engine {
     // layers of at most so many boards to move take quick_step: above, kernels
     // of a millisecond hide the waits
     static constexpr u64 QUICK_BOARDS = 1u << 21;
-    bool quick_step(GenTimes *tm, bool last, bool *moved_done, bool *done);
+    QuickStep quick;
+    bool quick_launch(bool last);
+    bool quick_take(GenTimes *tm, bool last, bool *moved_done, bool *done);
     bool next_inputs(GenTimes *tm);     // g.S from the spawns of g.moved and g.prev
     bool sort_unique_step(DevBuf<u64> &x, DevBuf<u64> &y, u64 n, u64 *nu, DevBuf<u64> **out, GenTimes *tm,
                           u64 *empties = nullptr, KeyBits *bits = nullptr);

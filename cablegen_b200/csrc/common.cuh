@@ -56,7 +56,8 @@ class KClock {
     void begin(cudaStream_t s, double *acc);
     void next(cudaStream_t s, double *acc);  // end and begin with one event
     void end(cudaStream_t s);
-    void flush();  // call after the stream has been synchronised
+    size_t pending() const { return pend_.size(); }
+    void flush(size_t first = ~(size_t)0);  // adds up the first so many spans, which are over
   private:
     struct Pending {
         cudaEvent_t a, b;

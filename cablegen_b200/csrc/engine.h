@@ -86,7 +86,7 @@ bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace 
 bool bucket_clear(BucketWorkspace &w, cudaStream_t s);
 int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,
                    BucketWorkspace &w, cudaStream_t s);
-BucketResult bucket_result(const BucketWorkspace &w, int slot);
+BucketResult bucket_result(const u32 *heads, int slot);
 // out[0, *n_out) = keys[0, n) ascending, without repeats when `unique`; out must
 // not alias keys, which are only read.  empties (optional): the empty cells over
 // the keys kept.  *done = false (and nothing written) where the sort by buckets

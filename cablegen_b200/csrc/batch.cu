@@ -327,15 +327,13 @@ bool run_group(Engine &e, const cgb_batch *b, std::vector<Plan> &plans, cgb_batc
                                                    8 * x.second.n, cudaMemcpyDeviceToDevice, s));
             at++;
         }
-        enq = enq && solve_layer_enqueue(cur.keys, n, cur.vals, vbytes, t2.ix, t4.ix, rules, e.rt, d_probes, s);
         cur.ix.keys = cur.keys;
         cur.ix.vals = cur.vals;
         cur.ix.n = n;
-        enq = enq && build_hash_enqueue(cur.ix, vbytes, cur.slots, cap, d_err, s);
+        enq = enq && solve_index_enqueue(cur.ix, vbytes, t2.ix, t4.ix, rules, e.rt, d_probes, cur.slots, cap, d_err, s);
         if (capture) ok = graph.finish(s, enq);
         else ok = enq;
         if (!ok) break;
-        kstats().launches += 2;
         st->boards_solved += n;
         st->solve_steps++;
         const bool enqueued = b->table_fn != nullptr;  // this step's copy reads only cur

@@ -239,14 +239,13 @@ bool ensure_storage(IndexStorage &st, u64 bytes, cudaStream_t s);
 // gives back the scratch that index builds keep for the next
 void index_release_scratch(cudaStream_t s);
 
-// graph-capturable forms (no host round trip): the solve kernel, counting
-// probes into *probes, and the hash index into caller-owned slots
+// graph-capturable form (no host round trip) of a layer's solve, ix.keys into
+// ix.vals, counting probes into *probes, and of its hash index in caller-owned slots
 // (hash_capacity(n) slots of 16 bytes); device errors accumulate in *err
-bool solve_layer_enqueue(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
-                         const SolveRules &r, const DeviceRowTable &rt, u64 *probes, cudaStream_t s);
+bool solve_index_enqueue(LayerIndex &ix, int vbytes, const LayerIndex &t2, const LayerIndex &t4, const SolveRules &r,
+                         const DeviceRowTable &rt, u64 *probes, void *slots, u64 cap, u32 *err, cudaStream_t s);
 u64 hash_capacity(u64 n);
 bool solve_prepare();  // one-time kernel attributes (call before a capture)
-bool build_hash_enqueue(LayerIndex &ix, int vbytes, void *slots, u64 cap, u32 *err, cudaStream_t s);
 
 // builds ix (keys/vals/n already set) of the requested kind; vbytes = 8 or 4.
 // index_begin launches the build: kernels behind it on the stream may use ix;
@@ -287,6 +286,11 @@ bool solve_layer_f32(const u64 *keys, u64 n, float *out, const LayerIndex &t2, c
 bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
                         const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
                         const CanonPlan &plan);
+// solves the layer ix.keys into ix.vals, and where *indexed is true on return the
+// solve also fills ix's index, which index_finish then has to look at
+bool solve_index_launch(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, const LayerIndex &t2, const LayerIndex &t4,
+                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s, const CanonPlan &plan,
+                        const KeyBits &bits, bool *indexed);
 bool solve_collect(Counters &c, cudaStream_t s);
 
 // ---- resident layers ------------------------------------------------------

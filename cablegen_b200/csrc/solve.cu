@@ -404,6 +404,52 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 1) solve_direct_kernel(const u
     add_probes(probes, probes_out);
 }
 
+// ---- insertion into a hash index ---------------------------------------------
+template <typename V>
+__device__ __forceinline__ bool insert_wide(ulonglong2 *slots, u64 cap, u64 key, V val)
+{
+    u64 s = home_slot(key, cap);
+    for (u64 p = 0; p < cap; p++) {
+        if (atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)key) == 0ull) {
+            slots[s].y = to_bits<V>(val);
+            return true;
+        }
+        s = (s + 1 == cap) ? 0 : s + 1;
+    }
+    return false;
+}
+
+// false when the probe distance runs past what the tag holds
+__device__ __forceinline__ bool insert_compact(unsigned long long *slots, u64 cap, const CompactHash &c, u64 key, float val)
+{
+    const u32 last = (1u << c.dbits) - 1u;
+    u32 tag0;
+    const u64 h = compact_home(c, key, &tag0), vbits = (u64)__float_as_uint(val) << 32;
+    for (u32 d = 0; d + 1 < last; d++)
+        if (atomicCAS(slots + ((h + d) & (cap - 1)), 0ull, (unsigned long long)(vbits | (tag0 + d))) == 0ull) return true;
+    return false;
+}
+
+// The index that a solve fills with the boards it solves: none, 16-byte or 8-byte
+// slots, cleared before.
+enum : int { FILL_NONE = 0, FILL_WIDE = 1, FILL_COMPACT = 2 };
+struct IndexFill {
+    int kind = FILL_NONE;
+    void *slots = nullptr;
+    u64 cap = 0;
+    CompactHash ch;
+    u32 *err = nullptr;
+    template <typename V>
+    __device__ __forceinline__ void add(u64 key, V val) const
+    {
+        bool placed = true;
+        if (kind == FILL_WIDE) placed = insert_wide((ulonglong2 *)slots, cap, key, val);
+        else if (sizeof(V) == 4 && kind == FILL_COMPACT)
+            placed = insert_compact((unsigned long long *)slots, cap, ch, key, (float)val);
+        if (!placed) atomicOr(err, ERR_CAPACITY);
+    }
+};
+
 // Item form: the work of a warp is its boards' (board, empty cell) pairs, not
 // its boards.  Boards have 0..16 empty cells, so one thread per board leaves a
 // warp waiting on its fullest board; here the 32 lanes take the pairs of 32
@@ -421,7 +467,8 @@ constexpr int item_smem() { return TABLE_BYTES_S + ITEM_WARPS * (ITEM_MAX * 2 + 
 template <typename V, int FORM>
 __global__ void __launch_bounds__(ITEM_THREADS, 1)
     solve_items_kernel(const u64 *__restrict__ keys, u64 n, V *__restrict__ out, DevTable<V> t2, DevTable<V> t4,
-                       SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan, u32 per)
+                       SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan, u32 per,
+                       IndexFill fill)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     stage_table_s(smem, g_move);
@@ -471,7 +518,11 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
             for (u32 q = lo; q < hi; q++) sums.add(best_sh[q - r0], best_sh[32 + q - r0]);
             __syncwarp();
         }
-        if (active) out[i] = sat ? V(1) : sums.result(spaces, b, r);
+        if (active) {
+            const V val = sat ? V(1) : sums.result(spaces, b, r);
+            out[i] = val;
+            fill.add(b, val);
+        }
         __syncwarp();
     }
     add_probes(probes, probes_out);
@@ -495,19 +546,7 @@ __global__ void hash_build_kernel(const u64 *__restrict__ keys, const V *__restr
                                   ulonglong2 *slots, u64 cap, u32 *err)
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        const u64 key = keys[i];
-        u64 s = home_slot(key, cap);
-        bool placed = false;
-        for (u64 p = 0; p < cap; p++) {
-            const u64 prev = atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)key);
-            if (prev == 0) {
-                slots[s].y = to_bits<V>(vals[i]);
-                placed = true;
-                break;
-            }
-            s = (s + 1 == cap) ? 0 : s + 1;
-        }
-        if (!placed) atomicOr(err, ERR_CAPACITY);
+        if (!insert_wide(slots, cap, keys[i], vals[i])) atomicOr(err, ERR_CAPACITY);
     }
 }
 
@@ -534,22 +573,9 @@ __global__ void key_bits_kernel(const u64 *__restrict__ keys, u64 n, unsigned lo
 __global__ void compact_build_kernel(const u64 *__restrict__ keys, const float *__restrict__ vals, u64 n,
                                      unsigned long long *slots, CompactHash c, u64 cap, u32 *err)
 {
-    const u32 last = (1u << c.dbits) - 1u;
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        u32 tag0;
-        const u64 h = compact_home(c, keys[i], &tag0);
-        const u64 vbits = (u64)__float_as_uint(vals[i]) << 32;
-        bool placed = false;
-        for (u32 d = 0; d + 1 < last; d++) {
-            const unsigned long long prev =
-                atomicCAS(slots + ((h + d) & (cap - 1)), 0ull, (unsigned long long)(vbits | (tag0 + d)));
-            if (prev == 0ull) {
-                placed = true;
-                break;
-            }
-        }
-        if (!placed) atomicOr(err, ERR_CAPACITY);  // the host falls back to 16-byte slots
-    }
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
+        // where this fails the host falls back to 16-byte slots
+        if (!insert_compact(slots, cap, c, keys[i], vals[i])) atomicOr(err, ERR_CAPACITY);
 }
 
 // ---- region-partitioned build of the 16-byte-slot index ----------------------
@@ -655,17 +681,7 @@ __global__ void overflow_insert_kernel(const ulonglong2 *__restrict__ over, cons
     const u32 n = min(*n_over, max_over);
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const ulonglong2 e = over[i];
-        u64 s = home_slot(e.x, cap);
-        bool placed = false;
-        for (u64 p = 0; p < cap; p++) {
-            if (atomicCAS((unsigned long long *)&slots[s].x, 0ull, (unsigned long long)e.x) == 0ull) {
-                slots[s].y = e.y;
-                placed = true;
-                break;
-            }
-            s = (s + 1 == cap) ? 0 : s + 1;
-        }
-        if (!placed) atomicOr(err, ERR_CAPACITY);
+        if (!insert_wide(slots, cap, e.x, __longlong_as_double((long long)e.y))) atomicOr(err, ERR_CAPACITY);
     }
 }
 
@@ -715,6 +731,23 @@ int g_hash_compact = 1;  // FP32 hash tables in 8-byte slots where the keys allo
 static u32 *h_index_err = nullptr;
 static u32 *index_err(const LayerIndex &ix, Counters &c) { return (u32 *)(c.d + 40 + ix.slot); }
 
+// a cleared table of 8-byte slots for ix, where its keys allow one (ix.kind says so)
+static bool start_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStream_t s, const KeyBits &bits)
+{
+    int cbits = 0;
+    const CompactHash ch = plan_compact(bits.all, bits.any, ix.n, &cbits);
+    if (!ch.on) return true;
+    const u64 cap = 1ull << cbits;
+    if (!ensure_storage(st, cap * 8, s)) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 8, s))) return false;
+    if (!CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, sizeof(u32), s))) return false;
+    ix.kind = INDEX_HASH;
+    ix.slots = st.p;
+    ix.cap = cap;
+    ix.ch = ch;
+    return true;
+}
+
 // launches the build of the 8-byte-slot index of an FP32 layer: AND/OR of the keys
 // give the constant bytes; the table is the power of two at or above twice the
 // layer; the tag holds the remainder bits (at most 26) and the probe distance.
@@ -723,23 +756,14 @@ static u32 *index_err(const LayerIndex &ix, Counters &c) { return (u32 *)(c.d + 
 static bool begin_compact(LayerIndex &ix, IndexStorage &st, Counters &c, cudaStream_t s, KeyBits bits)
 {
     if (!bits.known && !key_bits(KeySet{ix.keys, ix.n}, KeySet{}, &bits, nullptr, c, s)) return false;
-    int cbits = 0;
-    const CompactHash ch = plan_compact(bits.all, bits.any, ix.n, &cbits);
-    if (!ch.on) return true;
-    const u64 cap = 1ull << cbits;
-    if (!ensure_storage(st, cap * 8, s)) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 8, s))) return false;
-    if (!CGB_CUDA(cudaMemsetAsync(index_err(ix, c), 0, sizeof(u32), s))) return false;
+    if (!start_compact(ix, st, c, s, bits)) return false;
+    if (ix.kind != INDEX_HASH) return true;
     kclock().begin(s, &kstats().index_ms);
-    compact_build_kernel<<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const float *)ix.vals, ix.n,
-                                                                 (unsigned long long *)st.p, ch, cap, index_err(ix, c));
+    compact_build_kernel<<<grid_for(ix.n, 256, 16), 256, 0, s>>>(
+        ix.keys, (const float *)ix.vals, ix.n, (unsigned long long *)st.p, ix.ch, ix.cap, index_err(ix, c));
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError()) || !words_to_host(h_index_err + ix.slot, index_err(ix, c), 1, s))
         return false;
-    ix.kind = INDEX_HASH;
-    ix.slots = st.p;
-    ix.cap = cap;
-    ix.ch = ch;
     ix.unchecked = true;
     return true;
 }
@@ -800,14 +824,25 @@ void index_release_scratch(cudaStream_t s)
     region_scratch = IndexStorage{};
 }
 
-// launches the atomic build into a zeroed table, which cannot fail: the table
-// has more slots than keys
-static bool begin_atomic(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s)
+// a cleared table of 16-byte slots for ix
+static bool start_atomic(LayerIndex &ix, IndexStorage &st, cudaStream_t s)
 {
     // load factor <= g_hash_load_pct: capacity rounded up to a multiple of 64 slots
     const u64 cap = hash_capacity(ix.n);
     if (!ensure_storage(st, cap * 16, s)) return false;
     if (!CGB_CUDA(cudaMemsetAsync(st.p, 0, cap * 16, s))) return false;
+    ix.kind = INDEX_HASH;
+    ix.slots = st.p;
+    ix.cap = cap;
+    return true;
+}
+
+// launches the atomic build into a zeroed table, which cannot fail: the table
+// has more slots than keys
+static bool begin_atomic(LayerIndex &ix, int vbytes, IndexStorage &st, Counters &c, cudaStream_t s)
+{
+    if (!start_atomic(ix, st, s)) return false;
+    const u64 cap = ix.cap;
     kclock().begin(s, &kstats().index_ms);
     if (vbytes == 8)
         hash_build_kernel<double><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const double *)ix.vals, ix.n,
@@ -817,15 +852,12 @@ static bool begin_atomic(LayerIndex &ix, int vbytes, IndexStorage &st, Counters 
                                                                         (ulonglong2 *)st.p, cap, index_err(ix, c));
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
-    ix.kind = INDEX_HASH;
-    ix.slots = st.p;
-    ix.cap = cap;
     kstats().index_builds++;
     return true;
 }
 
-bool index_begin(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c, cudaStream_t s,
-                 const KeyBits &bits, int slot)
+// ix without an index yet, which its `slot`-th error word belongs to
+static bool reset_index(LayerIndex &ix, int slot)
 {
     ix.slot = slot;
     ix.kind = INDEX_BISECT;
@@ -833,13 +865,19 @@ bool index_begin(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int buc
     ix.slots = nullptr;
     ix.cap = 0;
     ix.unchecked = false;
-    if (ix.n == 0 || kind == INDEX_BISECT) return true;
     ix.ch = CompactHash{};
-    if (!h_index_err) {
-        void *h = nullptr;
-        if (!CGB_CUDA(cudaHostAlloc(&h, INDEX_SLOTS * sizeof(u32), cudaHostAllocDefault))) return false;
-        h_index_err = (u32 *)h;
-    }
+    if (h_index_err) return true;
+    void *h = nullptr;
+    if (!CGB_CUDA(cudaHostAlloc(&h, INDEX_SLOTS * sizeof(u32), cudaHostAllocDefault))) return false;
+    h_index_err = (u32 *)h;
+    return true;
+}
+
+bool index_begin(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, int bucket_bits, Counters &c, cudaStream_t s,
+                 const KeyBits &bits, int slot)
+{
+    if (!reset_index(ix, slot)) return false;
+    if (ix.n == 0 || kind == INDEX_BISECT) return true;
     if (kind == INDEX_HASH && vbytes == 4 && g_hash_compact && ix.n >= 64) {
         if (!begin_compact(ix, st, c, s, bits)) return false;
         if (ix.kind == INDEX_HASH) return true;
@@ -952,7 +990,7 @@ static bool solve_attrs()
 template <class V>
 static void enqueue_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, const LayerIndex &t4,
                           const SolveRules &r, const DeviceRowTable &rt, u64 *probes, cudaStream_t s,
-                          const CanonPlan &plan)
+                          const CanonPlan &plan, const IndexFill &fill = IndexFill{})
 {
     if (g_solve_variant == 1) {
         const auto kernel = plan.form == CANON_ONE        ? solve_items_kernel<V, CANON_ONE>
@@ -965,24 +1003,36 @@ static void enqueue_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, 
         u32 per = 4;
         while (per < 32 && (u64)per * ITEM_WARPS * NUM_SMS_B200 < n) per *= 2;
         kernel<<<grid_for((n + per - 1) / per * 32, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
-            keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan, per);
+            keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan, per, fill);
     } else {
         solve_direct_kernel<V><<<grid_for(n, DIRECT_THREADS, 1), DIRECT_THREADS, TABLE_BYTES_S, s>>>(
             keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan);
     }
 }
 
+// An index is filled by the solve itself, a thread inserting the board whose value it
+// has just formed: the insertions hide under the probes' latency, where a build of
+// its own reads keys and values again and, for a small layer, costs a launch as
+// long as the solve.  8-byte slots always; 16-byte slots up to so many keys: above,
+// the table is far larger than L2, an insertion costs a sector read and written,
+// and the build by regions wins.  Solve and index of a sweep, apart / filled: 149
+// layers of 2x4 3.93 / 2.97 ms, dpdf FP32 (0.9M boards a layer) 5.17 / 4.17, LL to
+// 120 (5M) 12.5 / 10.8, to 240 (12M) 95.2 / 94.5, to 330 (22M) 221 / 230; LL to
+// 330 in 8-byte slots 220 / 205.
+constexpr u64 FILL_KEYS = 1ull << 23;
+static bool fills_wide(u64 n) { return g_solve_variant == 1 && n <= FILL_KEYS; }
+
 constexpr int PROBES_AT = 12;  // counter word of the probes not collected yet
 
-bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
-                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
-                        const CanonPlan &plan)
+static bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
+                               const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
+                               const CanonPlan &plan, const IndexFill &fill)
 {
     if (n == 0) return true;
     if (!solve_attrs()) return false;
     kclock().begin(s, &kstats().solve_ms);
-    if (vbytes == 4) enqueue_solve<float>(keys, n, (float *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan);
-    else enqueue_solve<double>(keys, n, (double *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan);
+    if (vbytes == 4) enqueue_solve<float>(keys, n, (float *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan, fill);
+    else enqueue_solve<double>(keys, n, (double *)out, t2, t4, r, rt, c.d + PROBES_AT, s, plan, fill);
     kclock().end(s);
     if (!CGB_CUDA(cudaGetLastError())) return false;
     KernelStats &k = kstats();
@@ -990,6 +1040,37 @@ bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const Lay
     k.solve_boards += n;
     k.solve_bytes += (8 + vbytes) * n;  // keys in, values out; the probes' sectors follow
     return true;
+}
+
+bool solve_layer_launch(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
+                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s,
+                        const CanonPlan &plan)
+{
+    return solve_layer_launch(keys, n, out, vbytes, t2, t4, r, rt, c, s, plan, IndexFill{});
+}
+
+bool solve_index_launch(LayerIndex &ix, int kind, int vbytes, IndexStorage &st, const LayerIndex &t2, const LayerIndex &t4,
+                        const SolveRules &r, const DeviceRowTable &rt, Counters &c, cudaStream_t s, const CanonPlan &plan,
+                        const KeyBits &bits, bool *indexed)
+{
+    *indexed = false;
+    IndexFill fill;
+    if (!reset_index(ix, 0)) return false;
+    if (ix.n && kind == INDEX_HASH && g_solve_variant == 1) {
+        if (vbytes == 4 && g_hash_compact && ix.n >= 64 && bits.known && !start_compact(ix, st, c, s, bits)) return false;
+        if (ix.kind != INDEX_HASH && fills_wide(ix.n) && !start_atomic(ix, st, s)) return false;
+        if (ix.kind == INDEX_HASH)
+            fill = IndexFill{ix.ch.on ? FILL_COMPACT : FILL_WIDE, st.p, ix.cap, ix.ch, index_err(ix, c)};
+    }
+    if (!solve_layer_launch(ix.keys, ix.n, const_cast<void *>(ix.vals), vbytes, t2, t4, r, rt, c, s, plan, fill)) return false;
+    if (fill.kind == FILL_NONE) return true;
+    *indexed = true;
+    if (fill.kind == FILL_WIDE) {
+        kstats().index_builds++;
+        return true;
+    }
+    ix.unchecked = true;
+    return words_to_host(h_index_err + ix.slot, index_err(ix, c), 1, s);
 }
 
 bool solve_collect(Counters &c, cudaStream_t s)
@@ -1005,18 +1086,6 @@ bool solve_collect(Counters &c, cudaStream_t s)
     return true;
 }
 
-bool solve_layer_enqueue(const u64 *keys, u64 n, void *out, int vbytes, const LayerIndex &t2, const LayerIndex &t4,
-                         const SolveRules &r, const DeviceRowTable &rt, u64 *probes, cudaStream_t s)
-{
-    if (n == 0) return true;
-    if (!solve_attrs()) return false;
-    if (vbytes == 4) enqueue_solve<float>(keys, n, (float *)out, t2, t4, r, rt, probes, s, CanonPlan{});
-    else enqueue_solve<double>(keys, n, (double *)out, t2, t4, r, rt, probes, s, CanonPlan{});
-    KernelStats &k = kstats();
-    k.solve_launches++;
-    k.solve_boards += n;
-    return CGB_CUDA(cudaGetLastError());
-}
 
 bool solve_prepare() { return solve_attrs(); }
 
@@ -1031,7 +1100,8 @@ u64 hash_capacity(u64 n)
     return hash_capacity_for(n, pct);
 }
 
-bool build_hash_enqueue(LayerIndex &ix, int vbytes, void *slots, u64 cap, u32 *err, cudaStream_t s)
+bool solve_index_enqueue(LayerIndex &ix, int vbytes, const LayerIndex &t2, const LayerIndex &t4, const SolveRules &r,
+                         const DeviceRowTable &rt, u64 *probes, void *slots, u64 cap, u32 *err, cudaStream_t s)
 {
     ix.ch = CompactHash{};
     ix.kind = INDEX_BISECT;
@@ -1039,11 +1109,20 @@ bool build_hash_enqueue(LayerIndex &ix, int vbytes, void *slots, u64 cap, u32 *e
     ix.slots = nullptr;
     ix.cap = 0;
     if (ix.n == 0) return true;
-    if (!CGB_CUDA(cudaMemsetAsync(slots, 0, cap * 16, s))) return false;
-    if (vbytes == 8)
+    if (!solve_attrs() || !CGB_CUDA(cudaMemsetAsync(slots, 0, cap * 16, s))) return false;
+    IndexFill fill;
+    if (fills_wide(ix.n)) fill = IndexFill{FILL_WIDE, slots, cap, CompactHash{}, err};
+    void *out = const_cast<void *>(ix.vals);
+    if (vbytes == 4) enqueue_solve<float>(ix.keys, ix.n, (float *)out, t2, t4, r, rt, probes, s, CanonPlan{}, fill);
+    else enqueue_solve<double>(ix.keys, ix.n, (double *)out, t2, t4, r, rt, probes, s, CanonPlan{}, fill);
+    KernelStats &k = kstats();
+    k.solve_launches++;
+    k.solve_boards += ix.n;
+    k.launches += fill.kind == FILL_NONE ? 2 : 1;
+    if (fill.kind == FILL_NONE && vbytes == 8)
         hash_build_kernel<double><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const double *)ix.vals, ix.n,
                                                                          (ulonglong2 *)slots, cap, err);
-    else
+    else if (fill.kind == FILL_NONE)
         hash_build_kernel<float><<<grid_for(ix.n, 256, 16), 256, 0, s>>>(ix.keys, (const float *)ix.vals, ix.n,
                                                                         (ulonglong2 *)slots, cap, err);
     ix.kind = INDEX_HASH;

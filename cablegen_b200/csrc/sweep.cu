@@ -140,6 +140,7 @@ struct Chain {
         KeyBits bits;
         IndexStorage store;
         LayerIndex ix;
+        bool indexed = false;   // the solve fills the index
     };
     Solved t2, t4, cur;
     // memory of the layer that left last, for the next one: three layers' tables
@@ -165,23 +166,28 @@ struct Chain {
         x.ix.n = x.n;
         return build_index(x.ix, e.index_kind, 4, x.store, e.bucket_bits, e.ctr, s);
     }
-    bool solve(Engine &e, const SolveRules &r, cudaStream_t s)
+    // fill: the solve may fill the layer's index too (one chain only: two would
+    // share the error word)
+    bool solve(Engine &e, const SolveRules &r, cudaStream_t s, bool fill)
     {
         cur.vb = layer_vbytes(cur.sum);
         if (cur.vb == 4 && !(narrow(e, t2, s) && narrow(e, t4, s))) return false;
         std::swap(cur.room, spare_room);
         if (!ensure_storage(cur.room, cur.n * cur.vb + 8, s)) return false;
         cur.vals = cur.room.p;
+        cur.ix.keys = cur.keys;
+        cur.ix.vals = cur.vals;
+        cur.ix.n = cur.n;
+        std::swap(cur.store, spare_store);
+        if (fill)
+            return solve_index_launch(cur.ix, e.index_kind, cur.vb, cur.store, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan,
+                                      cur.bits, &cur.indexed);
         return solve_layer_launch(cur.keys, cur.n, cur.vals, cur.vb, t2.ix, t4.ix, r, e.rt, e.ctr, s, e.plan);
     }
     // launches the index build of the solved layer; finish_index waits for it
     bool begin_index(Engine &e, cudaStream_t s)
     {
-        cur.ix.keys = cur.keys;
-        cur.ix.vals = cur.vals;
-        cur.ix.n = cur.n;
-        std::swap(cur.store, spare_store);
-        return index_begin(cur.ix, e.index_kind, cur.vb, cur.store, e.bucket_bits, e.ctr, s, cur.bits);
+        return cur.indexed || index_begin(cur.ix, e.index_kind, cur.vb, cur.store, e.bucket_bits, e.ctr, s, cur.bits);
     }
     bool finish_index(Engine &e, cudaStream_t s) { return index_finish(cur.ix, cur.vb, cur.store, e.ctr, s); }
     void rotate(cudaStream_t s)
@@ -324,7 +330,7 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
             c.cur.keys = keys;
             c.cur.n = n;
             c.cur.bits = it != by_sum.end() ? sink.layers[it->second].bits : KeyBits{};
-            ok = ok && c.solve(e, rules, s);
+            ok = ok && c.solve(e, rules, s, chains.size() == 1);
         }
         if (!ok) break;
         solved += n;

@@ -61,7 +61,8 @@ constexpr u32 BK_OVERFLOW = 1u << 16;   // a bucket ran full (beside the ERR_* b
 // control words of one sort (u32 indexes): its head, and its arrays, which start
 // with the counts of the coarse buckets
 constexpr u32 H_TICKET = 0, H_FLAGS = 1, H_BUCKETS = 2, H_COUNT = BUCKET_COUNT_AT, H_EMPTIES = 6, H_ZEROS = 8,
-              H_ONES = 10;  // bits that are 0 (1) in some key, each low word first
+              H_ONES = 10,  // bits that are 0 (1) in some key, each low word first
+              H_STAMP = BUCKET_STAMP_AT;
 constexpr u32 A_COARSE = 0, A_BASE = A_COARSE + BK_COARSE, A_NUM = A_BASE + BK_COARSE, A_FINE = A_NUM + BK_COARSE;
 
 // The number of keys of a call: known on the host, or counted by a kernel before
@@ -284,7 +285,7 @@ __device__ __forceinline__ u32 mix32(u32 x)
 // (in sorted order the candidates of a level are a power of two apart, on one
 // bank).  Unused boundaries stay at KEY_MAX: no key is above them.
 template <typename K, class Emit>
-__device__ __forceinline__ void write_bounds(K (&v)[BK_KPT], K *buf, u32 m, u32 nb, u64 *__restrict__ bounds, Emit emit)
+__device__ __forceinline__ void write_bounds(K (&v)[BK_KPT], K *buf, u32 m, u32 nb, u64 *bounds, Emit emit)
 {
     block_sort(buf, m, v);
     __syncthreads();
@@ -309,13 +310,15 @@ __device__ __forceinline__ void write_bounds(K (&v)[BK_KPT], K *buf, u32 m, u32 
 // sorted input biases it.  (Nothing to do for the keys of one bucket: the bucket
 // sort takes them from the input.)
 template <bool FINE>
-__global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u64 *__restrict__ src, KeyCount n,
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) bucket_split_kernel(const u64 *src, KeyCount n,
                                                                         u32 buckets, u32 coarse_cap, u32 *head,
-                                                                        u32 *arrays, u64 *__restrict__ bounds)
+                                                                        u32 *arrays, u64 *bounds)
 {
     extern __shared__ __align__(16) u64 split_buf[];
     __shared__ u32 scratch[33];
     __shared__ BitMoves moves[2];
+    after_previous();
+    if (!FINE) stamp((u64 *)(head + H_STAMP));
     u32 cnt = n.get(), nb = buckets;
     const bool one_step = cnt <= BK_ONE_STEP;
     if (cnt <= BK_CAP || (FINE && one_step)) return;
@@ -406,12 +409,12 @@ struct PartSmem {
 // does.
 template <bool FINE>
 __global__ void __launch_bounds__(PART_THREADS, 4)
-    bucket_partition_kernel(const u64 *__restrict__ src, KeyCount n, u32 src_cap, u32 tiles, u32 buckets,
-                            const u64 *__restrict__ bounds, u32 *head, u32 *arrays, u64 *coarse, u32 coarse_cap,
+    bucket_partition_kernel(const u64 *src, KeyCount n, u32 src_cap, u32 tiles, u32 buckets, const u64 *bounds, u32 *head, u32 *arrays, u64 *coarse, u32 coarse_cap,
                             u64 *fine)
 {
     extern __shared__ __align__(16) unsigned char part_smem[];
     PartSmem &S = *reinterpret_cast<PartSmem *>(part_smem);
+    after_previous();
     const u32 t = threadIdx.x;
     const u32 c = FINE ? blockIdx.x / tiles : 0, tile = FINE ? blockIdx.x % tiles : blockIdx.x;
     const u32 all = n.get();
@@ -591,7 +594,7 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
 // compare-exchange is two instructions instead of six (the low words as they
 // are where the high words agree); the others are sorted as they are.
 template <bool UNIQUE, bool DIRECT, int THREADS>
-__device__ __forceinline__ void sort_bucket(const u64 *__restrict__ src, u32 cnt, u32 tile, u32 tiles, u32 *look, u32 *head,
+__device__ __forceinline__ void sort_bucket(const u64 *src, u32 cnt, u32 tile, u32 tiles, u32 *look, u32 *head,
                                             u64 *__restrict__ out, u32 count_empties, BucketSmem<THREADS> &S)
 {
     constexpr u32 ALL = 0xffffffffu;
@@ -651,11 +654,13 @@ __device__ __forceinline__ void sort_bucket(const u64 *__restrict__ src, u32 cnt
 
 template <bool UNIQUE, bool DIRECT>
 __global__ void __launch_bounds__(BUCKET_THREADS, 4)
-    bucket_sort_kernel(const u64 *__restrict__ input, KeyCount n, const u64 *__restrict__ slots, u32 counters, u32 words,
-                       u32 *head, u32 *arrays, u64 *__restrict__ out, u32 count_empties)
+    bucket_sort_kernel(const u64 *input, KeyCount n, const u64 *slots, u32 counters, u32 words, u32 *head, u32 *arrays,
+                       u64 *__restrict__ out, u32 count_empties)
 {
     __shared__ BucketSmem<BUCKET_THREADS> S;
+    after_previous();
     const u32 t = threadIdx.x;
+    if (!slots || gridDim.x == 1) stamp((u64 *)(head + H_STAMP));  // no split before it
     const u32 all = n.get();
     if (t == 0 && !DIRECT) S.tile = atomicAdd(head + H_TICKET, 1u);
     if (t < 4) S.and_or[t] = t < 2 ? 0xffffffffu : 0u;
@@ -675,10 +680,12 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
 // 2x4 table (3400 moves and 14000 spawns each): 7.8 -> 6.0 ms.
 template <bool UNIQUE>
 __global__ void __launch_bounds__(SMALL_THREADS, 1)
-    small_sort_kernel(const u64 *__restrict__ input, KeyCount n, u32 *head, u64 *__restrict__ out, u32 count_empties)
+    small_sort_kernel(const u64 *input, KeyCount n, u32 *head, u64 *__restrict__ out, u32 count_empties)
 {
     extern __shared__ __align__(16) unsigned char small_smem[];
     BucketSmem<SMALL_THREADS> &S = *reinterpret_cast<BucketSmem<SMALL_THREADS> *>(small_smem);
+    after_previous();
+    stamp((u64 *)(head + H_STAMP));
     const u32 cnt = n.get();
     if (cnt > BK_SMALL && threadIdx.x == 0) head[H_FLAGS] = BK_OVERFLOW;
     if (cnt == 0 || cnt > BK_SMALL) return;
@@ -770,11 +777,11 @@ static void launch_sort(const BucketPlan &p, const u64 *keys, KeyCount kc, u64 *
                         BucketWorkspace &w, cudaStream_t s)
 {
     if (p.n <= BK_CAP && !kc.counted)
-        bucket_sort_kernel<UNIQUE, true><<<1, BUCKET_THREADS, 0, s>>>(keys, kc, nullptr, A_FINE, A_FINE + p.grid, head,
-                                                                      arrays, out, empties);
+        launch_after(bucket_sort_kernel<UNIQUE, true>, 1, BUCKET_THREADS, 0, s, keys, kc, nullptr, A_FINE,
+                     A_FINE + p.grid, head, arrays, out, empties);
     else
-        bucket_sort_kernel<UNIQUE, false><<<p.grid, BUCKET_THREADS, 0, s>>>(keys, kc, w.fine.p, A_FINE, A_FINE + p.grid,
-                                                                            head, arrays, out, empties);
+        launch_after(bucket_sort_kernel<UNIQUE, false>, p.grid, BUCKET_THREADS, 0, s, keys, kc, w.fine.p, A_FINE,
+                     A_FINE + p.grid, head, arrays, out, empties);
 }
 
 int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,
@@ -787,23 +794,24 @@ int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *co
     int np = 1;
     if (p.small) {
         constexpr u32 smem = sizeof(BucketSmem<SMALL_THREADS>);
-        if (unique) small_sort_kernel<true><<<1, SMALL_THREADS, smem, s>>>(keys, kc, head, out, empties);
-        else small_sort_kernel<false><<<1, SMALL_THREADS, smem, s>>>(keys, kc, head, out, 0);
+        launch_after(unique ? small_sort_kernel<true> : small_sort_kernel<false>, 1, SMALL_THREADS, smem, s, keys, kc,
+                     head, out, unique && empties);
         return np;
     }
     if (p.n > BK_CAP) {
-        bucket_split_kernel<false><<<1, SPLIT_THREADS, split_smem, s>>>(keys, kc, p.coarse, 0, head, arrays, w.bounds.p);
-        bucket_partition_kernel<false><<<tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-            keys, kc, 0, 1, p.coarse, w.bounds.p, head, arrays, w.coarse.p, p.coarse_cap, w.fine.p);
+        launch_after(bucket_split_kernel<false>, 1, SPLIT_THREADS, split_smem, s, keys, kc, p.coarse, 0, head, arrays,
+                     w.bounds.p);
+        launch_after(bucket_partition_kernel<false>, tiles, PART_THREADS, sizeof(PartSmem), s, keys, kc, 0, 1, p.coarse,
+                     w.bounds.p, head, arrays, w.coarse.p, p.coarse_cap, w.fine.p);
         np = 2;
     }
     if (p.coarse) {
         const u32 fine_tiles = (p.coarse_cap + BK_TILE - 1) / BK_TILE;
         u64 *fine_bounds = w.bounds.p + BK_FAN;
-        bucket_split_kernel<true><<<p.coarse, SPLIT_THREADS, split_smem, s>>>(w.coarse.p, kc, p.coarse, p.coarse_cap, head,
-                                                                              arrays, fine_bounds);
-        bucket_partition_kernel<true><<<p.coarse * fine_tiles, PART_THREADS, sizeof(PartSmem), s>>>(
-            w.coarse.p, kc, p.coarse_cap, fine_tiles, 0, fine_bounds, head, arrays, nullptr, 0, w.fine.p);
+        launch_after(bucket_split_kernel<true>, p.coarse, SPLIT_THREADS, split_smem, s, w.coarse.p, kc, p.coarse,
+                     p.coarse_cap, head, arrays, fine_bounds);
+        launch_after(bucket_partition_kernel<true>, p.coarse * fine_tiles, PART_THREADS, sizeof(PartSmem), s, w.coarse.p,
+                     kc, p.coarse_cap, fine_tiles, 0, fine_bounds, head, arrays, nullptr, 0, w.fine.p);
         np = 3;
     }
     if (unique) launch_sort<true>(p, keys, kc, out, empties, head, arrays, w, s);
@@ -819,6 +827,7 @@ BucketResult bucket_result(const u32 *heads, int slot)
     r.error = h[H_FLAGS] & ~BK_OVERFLOW;
     r.overflow = (h[H_FLAGS] & BK_OVERFLOW) != 0;
     memcpy(&r.count, h + H_COUNT, 8);
+    memcpy(&r.started, h + H_STAMP, 8);
     memcpy(&r.empties, h + H_EMPTIES, 8);
     memcpy(&r.bits.all, h + H_ZEROS, 8);
     memcpy(&r.bits.any, h + H_ONES, 8);

@@ -131,6 +131,7 @@ struct GenBuffers {
 
 // a layer step in flight (Engine::quick_launch): its sizes as they were planned
 struct QuickStep {
+    static constexpr u32 EXPAND = 4, SPAWN = 5;  // 64-bit words of the third head: their start
     bool on = false;      // launched and not yet taken
     u64 room = 0;         // spawns that there is room for
     int passes[2] = {0, 0};
@@ -178,7 +179,7 @@ struct Engine {
     bool move_layer(const u64 *d_in, u64 n, GenTimes *tm);
     bool spawn_streams(GenTimes *tm);   // g.u2, g.u4: the sorted unique 2- and 4-spawns of g.moved
     bool spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm);
-    // layers of at most so many boards to move take quick_step: above, kernels
+    // layers of at most so many boards to move take quick_launch: above, kernels
     // of a millisecond hide the waits
     static constexpr u64 QUICK_BOARDS = 1u << 21;
     QuickStep quick;

@@ -73,6 +73,43 @@ class KClock {
 KClock &kclock();
 
 #ifdef __CUDACC__
+// The kernels of a layer step follow one another as programmatic dependents
+// (launch_after): a kernel's blocks are placed while the one before it drains, and
+// wait in after_previous() for its end.  Every thread calls that first, so that the
+// end of a kernel is the end of all before it; what the one before wrote is read by
+// plain loads (no __restrict__ const, no __ldg: those promise memory that does not
+// change while the kernel runs).  A no-op in an ordinary launch.  With times that the
+// kernels take themselves (stamp) in place of events between them, the table of 149
+// small 2x4 layers takes 13.2 ms instead of 16.6, dpdf 20.7 instead of 22.4.
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), u32 grid, u32 threads, u32 smem, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+// the time in nanoseconds at which a kernel's first block runs, into *at
+__device__ __forceinline__ void stamp(u64 *at)
+{
+    if (blockIdx.x || threadIdx.x || !at) return;
+    u64 t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    *at = t;
+}
+
 __device__ __forceinline__ u32 ld_acquire(const u32 *p)
 {
     u32 v;

@@ -243,13 +243,16 @@ void dev_free(void *p, cudaStream_t s)
     cudaFreeAsync(p, s);
 }
 
-__global__ void words_kernel(u32 *dst, const u32 *src, int words)
+__global__ void words_kernel(u32 *dst, const u32 *src, int words, u64 *started)
 {
+    after_previous();
+    stamp(started);
     for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
 }
-bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s)
+bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s, u64 *started)
 {
-    words_kernel<<<1, 64, 0, s>>>(pinned, dev, words);
+    if (started) launch_after(words_kernel, 1, 64, 0, s, pinned, dev, words, started);
+    else words_kernel<<<1, 64, 0, s>>>(pinned, dev, words, started);
     return CGB_CUDA(cudaGetLastError());
 }
 
@@ -624,27 +627,27 @@ bool Engine::quick_launch(bool last)
     if (!bucket_prepare(sizes, last ? 1 : 2, plans, w, s, likely)) return true;
     // its own copy: what runs between launch and take may sort too
     if (!quick.host &&
-        !CGB_CUDA(cudaHostAlloc((void **)&quick.host, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4, cudaHostAllocDefault)))
+        !CGB_CUDA(cudaHostAlloc((void **)&quick.host, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4 + 8, cudaHostAllocDefault)))
         return false;
-    // the third head: counts of moves, raw moves and spawns, error word
+    // the third head: counts of moves, raw moves and spawns, error word, and the
+    // times at which the expansions started (events between the kernels would keep
+    // them from following one another as programmatic dependents)
     constexpr u32 OWN = 2 * BUCKET_HEAD_WORDS;
     u64 *own = (u64 *)(w.ctl.p + OWN);
     u32 *err = w.ctl.p + OWN + 6;
     u32 *const h0 = w.ctl.p;
     SpawnSource two{g.b.p, 4 * n, 1, 0, (u64 *)(h0 + BUCKET_COUNT_AT)}, four{g.prev.p, g.prev.n, 2, 0};
     if (!bucket_clear(w, s)) return false;
-    kclock().begin(s, &kstats().expand_ms);
-    if (!expand_moves_enqueue(g.S.p, n, g.a.p, 4 * n, rt, prune_params(), own, own + 1, err, s, filter, plan)) return false;
-    kclock().next(s, &kstats().onesweep_ms);
+    if (!expand_moves_enqueue(g.S.p, n, g.a.p, 4 * n, rt, prune_params(), own, own + 1, err, own + QuickStep::EXPAND, s,
+                              filter, plan))
+        return false;
     quick.passes[0] = bucket_enqueue(plans[0], 0, g.a.p, own, g.b.p, true, true, w, s);
     if (!last) {
-        kclock().next(s, &kstats().spawn_ms);
-        if (!expand_next_enqueue(two, four, g.c[0].p, room, own + 2, err, s, plan)) return false;
-        kclock().next(s, &kstats().onesweep_ms);
+        if (!expand_next_enqueue(two, four, g.c[0].p, room, own + 2, err, own + QuickStep::SPAWN, s, plan)) return false;
         quick.passes[1] = bucket_enqueue(plans[1], 1, g.c[0].p, own + 2, g.c[1].p, true, false, w, s);
     }
-    kclock().end(s);
-    if (!CGB_CUDA(cudaGetLastError()) || !words_to_host(quick.host, w.ctl.p, BUCKET_HEADS * BUCKET_HEAD_WORDS, s))
+    constexpr u32 WORDS = BUCKET_HEADS * BUCKET_HEAD_WORDS;  // the end's time lands behind them
+    if (!CGB_CUDA(cudaGetLastError()) || !words_to_host(quick.host, w.ctl.p, WORDS, s, (u64 *)(quick.host + WORDS)))
         return false;
     quick.room = room;
     quick.on = true;
@@ -667,8 +670,19 @@ bool Engine::quick_take(GenTimes *tm, bool last, bool *moved_done, bool *done)
         return false;
     }
     g.move_ratio = std::max(0.25, (double)counts[0] / (double)n);
-    if (moves.overflow) return true;
     KernelStats &k = kstats();
+    u64 at[2], end;  // the expansions' times and the end's
+    memcpy(at, own + 2 * QuickStep::EXPAND, sizeof at);
+    memcpy(&end, quick.host + BUCKET_HEADS * BUCKET_HEAD_WORDS, 8);
+    const double ms = 1e-6;
+    k.launches += last ? 2 : 4;
+    k.expand_ms += ms * (double)(moves.started - at[0]);
+    k.onesweep_ms += ms * (double)((last ? end : at[1]) - moves.started);
+    if (!last) {
+        k.spawn_ms += ms * (double)(next.started - at[1]);
+        k.onesweep_ms += ms * (double)(end - next.started);
+    }
+    if (moves.overflow) return true;
     auto sorted = [&](u64 keys, int passes) {
         k.onesweep_bytes += 16 * keys * passes;
         k.onesweep_launches += passes;

@@ -21,7 +21,7 @@ struct DevBuf {
 // a few words from the device to pinned memory, visible once the stream has been
 // waited for.  A kernel writes them: a copy would queue in the copy engine behind
 // whatever layers and tables other streams are sending to the host
-bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s);
+bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s, u64 *started = nullptr);
 
 bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
 void dev_free(void *p, cudaStream_t s);
@@ -62,6 +62,7 @@ struct BucketWorkspace {
     void release(cudaStream_t s);
 };
 constexpr u32 BUCKET_COUNT_AT = 4;  // head word of the 64-bit number of keys written
+constexpr u32 BUCKET_STAMP_AT = 12; // head word of the time (ns) at which the sort started
 struct BucketPlan {
     u64 n = 0;              // keys at most
     bool small = false;     // expected to fit one CTA: nothing but its sort is launched
@@ -71,6 +72,7 @@ struct BucketPlan {
 };
 struct BucketResult {
     u64 count = 0, empties = 0;
+    u64 started = 0;        // device time in ns
     KeyBits bits;           // of the keys (unique sorts)
     u32 error = 0;
     bool overflow = false;  // nothing was written: the digit passes take the input
@@ -165,7 +167,8 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
 // its launch alone: the counts (results, and legal unpruned moves before the
 // repeats went) and errors are added to *count, *raw and *err
 bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceRowTable &t, const PruneParams &p,
-                          u64 *count, u64 *raw, u32 *err, cudaStream_t s, FormationFilter ff, const CanonPlan &plan);
+                          u64 *count, u64 *raw, u32 *err, u64 *started, cudaStream_t s, FormationFilter ff,
+                          const CanonPlan &plan);
 // number of empty cells over all boards (exact size of the spawn streams)
 bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s);
 // one spawn stream: every empty cell of a set of boards filled with `value`
@@ -179,7 +182,7 @@ struct SpawnSource {
 // the launch of expand_next alone: the count and errors are added to *count and
 // *err; nothing is written beyond cap
 bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u64 cap, u64 *count, u32 *err,
-                         cudaStream_t s, const CanonPlan &plan);
+                         u64 *started, cudaStream_t s, const CanonPlan &plan);
 // the canonical spawns of both sources, a.total + b.total of them, in one array
 // and without a wait: the counters land in c.host, for check_spawns once the
 // stream has been waited for

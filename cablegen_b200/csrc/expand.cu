@@ -189,9 +189,11 @@ __global__ void __launch_bounds__(EXP_THREADS, 1) expand_moves_kernel(const u64 
                                                                       PruneParams pp, const PruneTables *g_prune,
                                                                       u32 *err, FormationFilter ff, CanonPlan plan,
                                                                       u64 *raw_count, u32 window, u32 boards,
-                                                                      u32 slots)
+                                                                      u32 slots, u64 *started)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    after_previous();
+    stamp(started);
     __shared__ u32 scan_scratch[33];
     __shared__ u64 base_sh;
     // the prune table next to the row table; both staged before the barrier in stage_table
@@ -334,10 +336,12 @@ __device__ __forceinline__ u64 spawn_any(const u64 im[8], int cell, u64 value)
 
 template <int FORM>
 __global__ void __launch_bounds__(256) expand_next_kernel(SpawnSource a, SpawnSource b, u64 *__restrict__ out, u64 cap,
-                                                          u64 *out_count, u32 *err, CanonPlan plan)
+                                                          u64 *out_count, u32 *err, CanonPlan plan, u64 *started)
 {
     __shared__ u32 scan_scratch[33];
     __shared__ u64 base_sh;
+    after_previous();
+    stamp(started);
     if (a.counted) a.n = min(a.n, *a.counted);
     // whole blocks of 256 boards of a, then of b
     const u64 blocks_a = (a.n + 255) / 256, blocks = blocks_a + (b.n + 255) / 256;
@@ -408,7 +412,8 @@ static bool read_counters(Counters &c, cudaStream_t s, const char *what)
 }
 
 bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceRowTable &t, const PruneParams &p,
-                          u64 *count, u64 *raw, u32 *err, cudaStream_t s, FormationFilter ff, const CanonPlan &plan)
+                          u64 *count, u64 *raw, u32 *err, u64 *started, cudaStream_t s, FormationFilter ff,
+                          const CanonPlan &plan)
 {
     static bool attr = false;
     if (!attr) {
@@ -450,7 +455,7 @@ bool expand_moves_enqueue(const u64 *in, u64 n, u64 *out, u64 cap, const DeviceR
                         : plan.form == CANON_MIRROR   ? expand_moves_kernel<CANON_MIRROR>
                                                       : expand_moves_kernel<CANON_LIST>;
     kernel<<<grid, EXP_THREADS, EXP_SMEM, s>>>(in, n, out, cap, count, t.move, p, d_prune, err, ff, plan, raw, window,
-                                               boards, slots);
+                                               boards, slots, started);
     return CGB_CUDA(cudaGetLastError());
 }
 
@@ -461,7 +466,7 @@ bool expand_moves(const u64 *in, u64 n, u64 *out, u64 cap, u64 *n_out, const Dev
     if (n == 0) return true;
     if (!clear_counters(c, s)) return false;
     kclock().begin(s, &kstats().expand_ms);
-    const bool ok = expand_moves_enqueue(in, n, out, cap, t, p, c.d, c.d + 5, c.err, s, ff, plan);
+    const bool ok = expand_moves_enqueue(in, n, out, cap, t, p, c.d, c.d + 5, c.err, nullptr, s, ff, plan);
     kclock().end(s);
     if (!ok) return false;
     if (!read_counters(c, s, "expand_moves")) return false;
@@ -491,7 +496,7 @@ bool count_spawns(const u64 *in, u64 n, u64 *total, Counters &c, cudaStream_t s)
 }
 
 bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u64 cap, u64 *count, u32 *err,
-                         cudaStream_t s, const CanonPlan &plan)
+                         u64 *started, cudaStream_t s, const CanonPlan &plan)
 {
     const u64 blocks = (a.n + 255) / 256 + (b.n + 255) / 256;
     if (blocks == 0) return true;
@@ -500,7 +505,7 @@ bool expand_next_enqueue(const SpawnSource &a, const SpawnSource &b, u64 *out, u
                         : plan.form == CANON_DIAGONAL ? expand_next_kernel<CANON_DIAGONAL>
                         : plan.form == CANON_MIRROR   ? expand_next_kernel<CANON_MIRROR>
                                                       : expand_next_kernel<CANON_LIST>;
-    kernel<<<grid, 256, 0, s>>>(a, b, out, cap, count, err, plan);
+    launch_after(kernel, (u32)grid, 256, 0, s, a, b, out, cap, count, err, plan, started);
     return CGB_CUDA(cudaGetLastError());
 }
 
@@ -510,7 +515,7 @@ bool expand_next(const SpawnSource &a, const SpawnSource &b, u64 *out, Counters 
     const u64 cap = a.total + b.total;
     if (!clear_counters(c, s)) return false;
     kclock().begin(s, &kstats().spawn_ms);
-    const bool ok = expand_next_enqueue(a, b, out, cap, c.d, c.err, s, plan);
+    const bool ok = expand_next_enqueue(a, b, out, cap, c.d, c.err, nullptr, s, plan);
     kclock().end(s);
     kstats().spawn_bytes += 8 * (a.n + b.n) + 8 * cap;
     return ok && fetch_counters(c, s);

@@ -372,22 +372,6 @@ void LayerStore::clear(cudaStream_t s)
     chunks_.clear();
 }
 
-u64 LayerStore::bytes_in_use() const
-{
-    u64 b = 0;
-    for (auto &c : chunks_)
-        if (c.base) b += c.top * 8;
-    return b;
-}
-
-u64 LayerStore::bytes_spilled() const
-{
-    u64 b = 0;
-    for (auto &c : chunks_)
-        if (c.host) b += c.top * 8;
-    return b;
-}
-
 // ---- engine -----------------------------------------------------------------
 Engine &Engine::get()
 {

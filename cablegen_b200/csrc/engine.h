@@ -331,9 +331,6 @@ class LayerStore {
     // the host; false when nothing could be spilled
     bool spill(u64 bytes, cudaStream_t s, cudaStream_t io);
     void clear(cudaStream_t s);
-    u64 bytes_in_use() const;
-    size_t chunk_count() const { return chunks_.size(); }
-    u64 bytes_spilled() const;
     u64 spills = 0, restores = 0;
   private:
     struct Block { u64 off, n; bool live; };

@@ -581,7 +581,7 @@ __global__ void compact_build_kernel(const u64 *__restrict__ keys, const float *
 // ---- region-partitioned build of the 16-byte-slot index ----------------------
 // The atomic build inserts every key with a compare-and-swap on a random slot of
 // a table that was zeroed first: a random read-modify-write per key.  This form
-// partitions the keys by region of their home slot (2048 slots = 32 KiB), builds
+// partitions the keys by region of their home slot (1024 slots = 16 KiB), builds
 // each region in shared memory and writes it out whole: the table is written
 // once, sequentially, and never zeroed.  A key whose linear probe runs past its
 // region's end (or whose region's bucket is full) goes to an overflow list,

@@ -45,9 +45,9 @@ PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes (read + write) per unit of work from the ncu captures summarised in profiles/
 # (smaller cases of the same kernels; their traffic grows in proportion to the units):
-# a sort digit pass per key (onesweep_byte512_88M_ll_keys.md), the solve per board
-# (solve_items_f64_ll_layer196.md).
-NCU_DRAM_BYTES_PER_UNIT = {"onesweep": 1.379122e9 / 88333334, "solve": 1.915215e9 / 5404078}
+# the sort per key and kernel that moves keys, the solve per board
+# (bucket_sort_and_solve_ll_layer196.md).
+NCU_DRAM_BYTES_PER_UNIT = {"onesweep": 3.119e9 / (3 * 64000000), "solve": 1.847e9 / 5000000}
 
 
 def parse():
@@ -566,7 +566,7 @@ def run_ours(args):
 
     # ---- roofline of the dominant kernel
     peak, peak_kind = hbm_peak()
-    fams = {"onesweep": "sort digit pass (onesweep)", "solve": "solve (expectimax + lookups)",
+    fams = {"onesweep": "sort (bucket partitions and bucket sort; digit passes)", "solve": "solve (expectimax + lookups)",
             "expand": "move expansion", "spawn": "spawn expansion", "unique": "unique", "merge": "merge",
             "hist": "sort histogram"}
     # the index builds have no algorithmic-byte figure of their own; their time is listed
@@ -574,7 +574,7 @@ def run_ours(args):
     achieved = kst[f"{dom}_bytes"] / 1e9 / (kst[f"{dom}_ms"] / 1000.0) if kst[f"{dom}_ms"] else 0.0
     # traffic of the dominant kernel per launch: ncu bytes per unit x the mean units per launch
     traffic, traffic_note = None, None
-    units = {"onesweep": (kst["onesweep_bytes"] / 16.0, kst["onesweep_launches"], "keys per pass"),
+    units = {"onesweep": (kst["onesweep_bytes"] / 16.0, kst["onesweep_launches"], "keys per kernel"),
              "solve": (kst["solve_boards"], kst["solve_launches"], "boards")}
     if dom in units and dom in NCU_DRAM_BYTES_PER_UNIT and units[dom][1]:
         per_launch_units = units[dom][0] / units[dom][1]

@@ -305,10 +305,12 @@ __device__ __forceinline__ V probe1(const DevTable<V> &t, u64 key, bool legal)
 // eight successors is large enough that warps wait on instruction fetch).  Both
 // successors' first slots are loaded before either is looked at: 1.06 -> 0.96 ms
 // for 5M LL boards, the kernel being bound by the latency of these loads.
+//
+// The views k0, k0 + step, ... only (all: 0 and 1); with step 4 the one view's values.
 template <int FORM, typename V>
 __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int cell, const CanonPlan &plan,
                                                   const DevTable<V> &t2, const DevTable<V> &t4, V &best2, V &best4,
-                                                  u32 &probes)
+                                                  u32 &probes, int k0, int step)
 {
     const Half h = halves(b), t = transpose(h);
     const int r0 = cell >> 2, q0 = cell & 3;
@@ -317,7 +319,7 @@ __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int
     const bool wide = t2.kind == INDEX_HASH && t4.kind == INDEX_HASH && !t2.ch.on && !t4.ch.on;
     const bool compact = sizeof(V) == 4 && t2.kind == INDEX_HASH && t4.kind == INDEX_HASH && t2.ch.on && t4.ch.on;
 #pragma unroll 1
-    for (int k = 0; k < 4; k++) {
+    for (int k = k0; k < 4; k += step) {
         // view k: id, H, T, H.T; the cell of the spawn in it
         const Half x = (k & 2) ? t : h;
         const u64 y = (k & 1) ? whole(flip_h(x)) : whole(x);
@@ -359,8 +361,8 @@ __device__ __forceinline__ void cell_bests_rolled(const RowTable &rt, u64 b, int
             v2 = probe1(t2, c2, ok2);
             v4 = probe1(t4, c4, ok4);
         }
-        best2 = vmax(best2, v2);
-        best4 = vmax(best4, v4);
+        best2 = step == 4 ? v2 : vmax(best2, v2);
+        best4 = step == 4 ? v4 : vmax(best4, v4);
     }
 }
 
@@ -464,7 +466,12 @@ constexpr int ITEM_MAX = 32 * 16;  // pairs of 32 boards at most
 template <typename V>
 constexpr int item_smem() { return TABLE_BYTES_S + ITEM_WARPS * (ITEM_MAX * 2 + 2 * 32 * (int)sizeof(V)); }
 
-template <typename V, int FORM>
+//
+// With VIEWS, for layers that leave the chip idle, four lanes share a pair, one view
+// each: the chain of four views, a move, a canonical form and a probe each, is what
+// such a layer's solve takes.  Every lane then takes the maximum of the four values in
+// the views' order, as one lane does, so that a NaN of a given table counts the same.
+template <typename V, int FORM, bool VIEWS>
 __global__ void __launch_bounds__(ITEM_THREADS, 1)
     solve_items_kernel(const u64 *__restrict__ keys, u64 n, V *__restrict__ out, DevTable<V> t2, DevTable<V> t4,
                        SolveRules r, const unsigned short *g_move, u64 *probes_out, CanonPlan plan, u32 per,
@@ -498,23 +505,34 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
         const bool planned = __all_sync(0xffffffffu, !active || fixed_pattern(b) == plan.mask);
         __syncwarp();
         SpawnSums<V> sums;
-        for (u32 r0 = 0; r0 < total; r0 += 32) {
-            const u32 j = r0 + (u32)lane;
+        constexpr u32 PAIRS = VIEWS ? 8 : 32;  // of a round
+        for (u32 r0 = 0; r0 < total; r0 += PAIRS) {
+            const u32 j = r0 + (u32)lane / (32 / PAIRS);
             const bool has = j < total;
             const u32 it = has ? items[j] : 0u;
             const int owner = (int)(it >> 4), cell = (int)(it & 15u);
             const u64 ob = __shfl_sync(0xffffffffu, b, owner);
             V best2 = 0, best4 = 0;
             if (has) {
-                if (planned) cell_bests_rolled<FORM>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
-                else cell_bests_rolled<-1>(rt, ob, cell, plan, t2, t4, best2, best4, probes);
+                const int k0 = VIEWS ? lane & 3 : 0, step = VIEWS ? 4 : 1;
+                if (planned) cell_bests_rolled<FORM>(rt, ob, cell, plan, t2, t4, best2, best4, probes, k0, step);
+                else cell_bests_rolled<-1>(rt, ob, cell, plan, t2, t4, best2, best4, probes, k0, step);
             }
-            best_sh[lane] = best2;
-            best_sh[32 + lane] = best4;
+            if (VIEWS) {
+                const V v2 = best2, v4 = best4;
+                best2 = best4 = V(0);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    best2 = vmax(best2, __shfl_sync(0xffffffffu, v2, (lane & ~3) | k));
+                    best4 = vmax(best4, __shfl_sync(0xffffffffu, v4, (lane & ~3) | k));
+                }
+            }
+            best_sh[j - r0] = best2;
+            best_sh[32 + j - r0] = best4;
             __syncwarp();
             // the owner adds the pairs of this round that are its own, in cell order
             const u32 lo = off > r0 ? off : r0;
-            const u32 hi = (off + (u32)spaces) < r0 + 32 ? off + (u32)spaces : r0 + 32;
+            const u32 hi = (off + (u32)spaces) < r0 + PAIRS ? off + (u32)spaces : r0 + PAIRS;
             for (u32 q = lo; q < hi; q++) sums.add(best_sh[q - r0], best_sh[32 + q - r0]);
             __syncwarp();
         }
@@ -956,13 +974,25 @@ static DevTable<V> dev_table(const LayerIndex &ix)
     return t;
 }
 
+// layers of up to so many boards per warp of the chip give a pair four lanes: the solves
+// of the 149 layers of a 2x4 table 3.06 -> 2.49 ms; limits of 1, 4 and 8 measured alike
+constexpr u64 VIEWS_PER = 2;
 int g_solve_variant = 1;  // 0: direct (one thread per board), 1: (board, cell) pairs per warp
 
 template <typename V, int FORM>
 static bool items_attr_one()
 {
-    return CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<V, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         item_smem<V>()));
+    const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    return CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<V, FORM, false>, smem, item_smem<V>())) &&
+           CGB_CUDA(cudaFuncSetAttribute(solve_items_kernel<V, FORM, true>, smem, item_smem<V>()));
+}
+template <typename V, bool VIEWS>
+static auto items_kernel(int form)
+{
+    return form == CANON_ONE        ? solve_items_kernel<V, CANON_ONE, VIEWS>
+           : form == CANON_DIAGONAL ? solve_items_kernel<V, CANON_DIAGONAL, VIEWS>
+           : form == CANON_MIRROR   ? solve_items_kernel<V, CANON_MIRROR, VIEWS>
+                                    : solve_items_kernel<V, CANON_LIST, VIEWS>;
 }
 template <typename V>
 static bool items_attr()
@@ -993,15 +1023,14 @@ static void enqueue_solve(const u64 *keys, u64 n, V *out, const LayerIndex &t2, 
                           const CanonPlan &plan, const IndexFill &fill = IndexFill{})
 {
     if (g_solve_variant == 1) {
-        const auto kernel = plan.form == CANON_ONE        ? solve_items_kernel<V, CANON_ONE>
-                            : plan.form == CANON_DIAGONAL ? solve_items_kernel<V, CANON_DIAGONAL>
-                            : plan.form == CANON_MIRROR   ? solve_items_kernel<V, CANON_MIRROR>
-                                                          : solve_items_kernel<V, CANON_LIST>;
         // a warp takes `per` boards at a time: 32, fewer where the layer does not
         // give every warp of the chip that many, so that it spreads over the SMs and
         // one round of pairs serves a warp (2600 2x4 boards: 27 -> 18 us)
-        u32 per = 4;
-        while (per < 32 && (u64)per * ITEM_WARPS * NUM_SMS_B200 < n) per *= 2;
+        const u64 warps = (u64)ITEM_WARPS * NUM_SMS_B200;
+        const bool views = n <= VIEWS_PER * warps;
+        u32 per = views ? 1 : 4;
+        while (per < 32 && per * warps < n) per *= 2;
+        const auto kernel = views ? items_kernel<V, true>(plan.form) : items_kernel<V, false>(plan.form);
         kernel<<<grid_for((n + per - 1) / per * 32, ITEM_THREADS, 1), ITEM_THREADS, item_smem<V>(), s>>>(
             keys, n, out, dev_table<V>(t2), dev_table<V>(t4), r, rt.move, probes, plan, per, fill);
     } else {

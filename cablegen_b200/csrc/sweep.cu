@@ -150,6 +150,13 @@ struct Chain {
 
     int layer_vbytes(int sum) const { return vbytes == 4 && sum > fp64_above ? 8 : vbytes; }
 
+    // whether the solve of cur starts with narrow()
+    bool narrows() const
+    {
+        auto wide = [](const Solved &x) { return x.vb == 8 && x.vals; };
+        return layer_vbytes(cur.sum) == 4 && (wide(t2) || wide(t4));
+    }
+
     // an FP64 table of the window turned into the FP32 table the chain below reads
     bool narrow(Engine &e, Solved &x, cudaStream_t s)
     {
@@ -327,6 +334,10 @@ extern "C" int cgb_sweep_run(const cgb_sweep *w, cgb_stats *stats)
         }
         for (auto &c : chains) {
             c.cur.sum = sum;
+            // narrow() gives back the FP64 values of the layers above, and the copy of
+            // the last layer's table may still be reading them on the I/O stream: the
+            // main stream waits for it, once per FP32 sweep
+            if (c.narrows()) ok = ok && out.fence_main();
             c.cur.keys = keys;
             c.cur.n = n;
             c.cur.bits = it != by_sum.end() ? sink.layers[it->second].bits : KeyBits{};

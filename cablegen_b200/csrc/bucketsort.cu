@@ -34,22 +34,13 @@
 // input.  The input itself is only read.
 #include "engine.h"
 #include "lookback.cuh"
-#include <cmath>
 #include <cstring>
 
 namespace cgb {
 
-constexpr u32 BK_TARGET = 1800;   // keys per bucket aimed at
-constexpr u32 BK_CAP = 4096;      // keys a bucket holds; 2.27 x the target: with 32 samples per bucket a
-                                  // size is off by 18 % (one sigma), so this is seven sigma
-constexpr u32 BK_FAN = 512;       // buckets of one partition step
-constexpr u32 BK_ONE_STEP = 400 * BK_TARGET;  // keys up to which one step is taken: 8192 samples bound 400
-                                              // buckets as well as 20 each do (2.27 x the size: one in a million)
-constexpr u32 BK_COARSE = 512;    // coarse buckets of the two-step form
 constexpr u32 BK_TILE = 4096;     // keys per partition CTA
 constexpr int BK_KPT = 16;        // keys per thread, every kernel
 constexpr int SPLIT_THREADS = 512;
-constexpr u32 BK_SAMPLES = 8192;
 constexpr int PART_THREADS = 256;
 constexpr int BUCKET_THREADS = 256;
 constexpr int SMALL_THREADS = 1024;
@@ -58,12 +49,10 @@ constexpr u32 BK_SMALL = SMALL_THREADS * BK_KPT;  // keys that one CTA sorts in 
 constexpr u64 KEY_MAX = ~0ull;
 constexpr u32 BK_OVERFLOW = 1u << 16;   // a bucket ran full (beside the ERR_* bits)
 
-// control words of one sort (u32 indexes): its head, and its arrays, which start
-// with the counts of the coarse buckets
+// control words of a sort's head (u32 indexes); its arrays: A_* of bucketplan.h
 constexpr u32 H_TICKET = 0, H_FLAGS = 1, H_BUCKETS = 2, H_COUNT = BUCKET_COUNT_AT, H_EMPTIES = 6, H_ZEROS = 8,
               H_ONES = 10,  // bits that are 0 (1) in some key, each low word first
               H_STAMP = BUCKET_STAMP_AT;
-constexpr u32 A_COARSE = 0, A_BASE = A_COARSE + BK_COARSE, A_NUM = A_BASE + BK_COARSE, A_FINE = A_NUM + BK_COARSE;
 
 // The number of keys of a call: known on the host, or counted by a kernel before
 // it (at most n, which sizes grids and buckets).
@@ -718,32 +707,6 @@ static bool attributes()
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<false>, smem, part)) &&
            CGB_CUDA(cudaFuncSetAttribute(bucket_partition_kernel<true>, smem, part));
     return done;
-}
-
-// Sizes of one call.  Two steps above BK_ONE_STEP keys: coarse buckets of
-// equal expected size, their space seven sigma above it (a coarse bucket is
-// bounded by 64 samples, or by 8192 / coarse).
-static bool plan_buckets(u64 n, BucketPlan *p)
-{
-    *p = BucketPlan{};
-    p->n = n;
-    if (n > BUCKET_SORT_KEYS) return false;
-    if (n <= BK_CAP) {
-        p->grid = 1;
-    } else if (n <= BK_ONE_STEP) {
-        p->grid = (u32)((n + BK_TARGET - 1) / BK_TARGET);
-    } else {
-        u32 c = (u32)std::ceil(std::sqrt((double)n / BK_TARGET));
-        if (c > BK_COARSE) c = BK_COARSE;
-        const double per = std::min(64.0, (double)BK_SAMPLES / c);
-        const u64 cap = ((u64)((double)n / c * (1.0 + 7.0 / std::sqrt(per))) + 63) / 64 * 64;
-        if (cap > (u64)BK_FAN * BK_TARGET) return false;  // more buckets than one step tells apart
-        p->coarse = c;
-        p->coarse_cap = (u32)cap;
-        p->grid = (u32)(n / BK_TARGET) + c;
-    }
-    p->words = A_FINE + 2 * p->grid;
-    return true;
 }
 
 bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace &w, cudaStream_t s, const u64 *likely)

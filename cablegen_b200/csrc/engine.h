@@ -6,6 +6,7 @@
 #include <vector>
 #include "common.cuh"
 #include "board.cuh"
+#include "bucketplan.h"
 #include "hashidx.cuh"
 
 namespace cgb {
@@ -51,7 +52,6 @@ struct KeyBits {
     u64 all = 0, any = 0;
     bool known = false;
 };
-constexpr u64 BUCKET_SORT_KEYS = 160ull << 20;  // the most keys one call takes (512 x 512 buckets hold them)
 constexpr u32 BUCKET_HEADS = 3, BUCKET_HEAD_WORDS = 16;  // heads: two sorts, and words of the caller's own
 struct BucketWorkspace {
     DevBuf<u32> ctl;           // the heads, then each sort's bucket counts and look-back words
@@ -63,13 +63,6 @@ struct BucketWorkspace {
 };
 constexpr u32 BUCKET_COUNT_AT = 4;  // head word of the 64-bit number of keys written
 constexpr u32 BUCKET_STAMP_AT = 12; // head word of the time (ns) at which the sort started
-struct BucketPlan {
-    u64 n = 0;              // keys at most
-    bool small = false;     // expected to fit one CTA: nothing but its sort is launched
-    u32 coarse = 0, coarse_cap = 0;  // two steps: coarse buckets and their space
-    u32 grid = 0;           // buckets at most
-    u64 words = 0, arrays_at = 0;
-};
 struct BucketResult {
     u64 count = 0, empties = 0;
     u64 started = 0;        // device time in ns

@@ -563,6 +563,7 @@ bool Engine::next_inputs(GenTimes *tm)
         return false;
     const SpawnSource two{g.moved.p, g.moved.n, 1, g.moved_empties}, four{g.prev.p, g.prev.n, 2, g.prev_empties};
     const u64 total = two.total + four.total;
+    if (g.S.n) g.spawn_ratio = std::max(1.0, (double)total / (double)g.S.n);
     g.S.n = 0;
     if (total <= std::min(max_sort_keys, BUCKET_SORT_KEYS)) {
         for (auto &x : g.c)
@@ -604,8 +605,12 @@ bool Engine::quick_launch(bool last)
     if (room > max_sort_keys) return true;
     const u64 sizes[2] = {4 * n, room};
     BucketPlan plans[2];
-    if (!reserve(g.a, 4 * n, s) || !reserve(g.b, 4 * n, s) || !reserve(g.c[0], room, s) || !reserve(g.c[1], room, s))
-        return false;
+    // without memory for the guess the step with waits, which knows its sizes, takes
+    // the layer, and what the guess has got of it goes back
+    if (!reserve(g.a, 4 * n, s) || !reserve(g.b, 4 * n, s) || !reserve(g.c[0], room, s) || !reserve(g.c[1], room, s)) {
+        for (auto &x : g.c) drop(x, s);
+        return true;
+    }
     BucketWorkspace &w = ws.buckets;
     const u64 likely[2] = {(u64)(1.25 * (double)n * g.move_ratio), (u64)(1.25 * (double)n * g.spawn_ratio)};
     if (!bucket_prepare(sizes, last ? 1 : 2, plans, w, s, likely)) return true;

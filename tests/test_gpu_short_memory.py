@@ -14,7 +14,7 @@ HEAD = """
     import ctypes as C, sys
     import numpy as np
     sys.path.insert(0, {root!r})
-    sys.path.insert(0, os.path.join({root!r}, "tests"))
+    sys.path.insert(0, {root!r} + "/tests")
     from cablegen_b200 import _lib, configs, device
     from helpers import realistic_boards
     import torch

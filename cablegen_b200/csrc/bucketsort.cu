@@ -725,9 +725,16 @@ bool bucket_prepare(const u64 *n, int calls, BucketPlan *plans, BucketWorkspace 
     }
     w.used_words = words;
     auto room = [&](auto &b, u64 want) { return (b.p && b.cap >= want) || !want || grow(b, want * 5 / 4, s); };
+    w.growing = true;
+    const bool have = room(w.ctl, words) && room(w.bounds, bounds) && room(w.fine, fine) && room(w.coarse, coarse);
+    w.growing = false;
+    if (!have) {  // the digit passes take over, and their caller may need the room
+        w.release(s);
+        return false;
+    }
     if (!w.host && !CGB_CUDA(cudaHostAlloc((void **)&w.host, BUCKET_HEADS * BUCKET_HEAD_WORDS * 4, cudaHostAllocDefault)))
         return false;
-    return room(w.ctl, words) && room(w.bounds, bounds) && room(w.fine, fine) && room(w.coarse, coarse) && attributes();
+    return attributes();
 }
 
 bool bucket_clear(BucketWorkspace &w, cudaStream_t s)

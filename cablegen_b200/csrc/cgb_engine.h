@@ -196,6 +196,10 @@ struct Engine {
                   const u64 *h_carry = nullptr, u64 n_carry = 0);
     OneShot one_shot;
     void end_one_shot();     // keeps what may be kept
+    // gives back what is kept only to make the next call faster: one-layer calls'
+    // indexes, the sort's buckets, the index builds' scratch (each after what the
+    // stream still does with it)
+    void drop_kept(cudaStream_t s);
     void release_buffers();
 };
 

@@ -123,7 +123,12 @@ void KClock::flush(size_t first)
 u64 g_dev_mem_cap = 0;
 static std::mutex g_mem_mu;
 static std::unordered_map<void *, u64> g_mem_blocks;
-static u64 g_mem_held = 0;
+static u64 g_mem_held = 0, g_mem_failed = 0;
+u64 failed_allocs()
+{
+    std::lock_guard<std::mutex> g(g_mem_mu);
+    return g_mem_failed;
+}
 
 // Large blocks that were freed, for the next allocation of about their size on
 // the same stream.  The stream-ordered pool under them splits a large free block
@@ -175,8 +180,7 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
         std::lock_guard<std::mutex> g(g_mem_mu);
         return g_dev_mem_cap && g_mem_held + bytes > g_dev_mem_cap;
     };
-    // what one-layer calls keep goes first
-    if (over_cap()) Engine::get().one_shot.drop(s);
+    if (over_cap()) Engine::get().drop_kept(s);
     {
         std::lock_guard<std::mutex> g(g_mem_mu);
         if (g_dev_mem_cap && g_mem_held + bytes > g_dev_mem_cap) {
@@ -184,6 +188,7 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
             snprintf(buf, sizeof buf, "device allocation of %.3f GB failed: over the cap of %.3f GB (%.3f GB held)",
                      bytes / 1e9, g_dev_mem_cap / 1e9, g_mem_held / 1e9);
             set_error(buf);
+            g_mem_failed++;
             return false;
         }
     }
@@ -198,7 +203,7 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
         // freed blocks of other sizes may still sit in the pool: return them
         // to the device and retry once
         cudaGetLastError();
-        Engine::get().one_shot.drop(s);
+        Engine::get().drop_kept(s);
         release_blocks();
         cudaStreamSynchronize(s);
         int dev = 0;
@@ -214,6 +219,8 @@ bool dev_alloc(void **p, u64 bytes, cudaStream_t s)
         set_error(buf);
         cudaGetLastError();
         *p = nullptr;
+        std::lock_guard<std::mutex> g(g_mem_mu);
+        g_mem_failed++;
         return false;
     }
     std::lock_guard<std::mutex> g(g_mem_mu);
@@ -774,6 +781,13 @@ void Engine::end_one_shot()
             x = IndexStorage{};
         }
     index_release_scratch(stream);
+}
+
+void Engine::drop_kept(cudaStream_t s)
+{
+    one_shot.drop(s);
+    if (!ws.buckets.growing) ws.buckets.release(s);
+    index_release_scratch(s);
 }
 
 void Engine::release_buffers()

@@ -25,6 +25,7 @@ struct DevBuf {
 bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s, u64 *started = nullptr);
 
 bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
+u64 failed_allocs();  // how many dev_alloc calls have found no memory
 void dev_free(void *p, cudaStream_t s);
 template <typename T>
 bool grow(DevBuf<T> &b, u64 n, cudaStream_t s)
@@ -59,6 +60,7 @@ struct BucketWorkspace {
     DevBuf<u64> coarse, fine;  // the buckets
     u64 used_words = 0;
     u32 *host = nullptr;       // pinned copy of the heads
+    bool growing = false;      // bucket_prepare is at work on it
     void release(cudaStream_t s);
 };
 constexpr u32 BUCKET_COUNT_AT = 4;  // head word of the 64-bit number of keys written

@@ -326,6 +326,21 @@ extern "C" int cgb_canonicalize(const uint64_t *d_in, uint64_t n, uint64_t *d_ou
     return 0;
 }
 
+// A call that works in the engine's one-shot memory.  Where memory runs out it starts
+// over, once and without what is kept: that may be larger than this call needs.
+template <class Call>
+static bool one_shot_call(Call call)
+{
+    Engine &e = E();
+    const u64 failed = failed_allocs();
+    for (bool again = false;; again = true) {
+        e.one_shot.busy = true;
+        const bool ok = call(e.one_shot);
+        e.end_one_shot();
+        if (ok || again || failed_allocs() == failed || !e.one_shot.drop(e.stream)) return ok;
+    }
+}
+
 extern "C" int cgb_solve_layer(const uint64_t *d_keys, uint64_t n, void *d_out, int precision,
                                const uint64_t *d_k2, const void *d_v2, uint64_t n2, const uint64_t *d_k4,
                                const void *d_v4, uint64_t n4, const uint64_t *h_winstates, int n_winstates)
@@ -333,41 +348,40 @@ extern "C" int cgb_solve_layer(const uint64_t *d_keys, uint64_t n, void *d_out, 
     CGB_TRY(ensure_rules_for_api());
     cudaStream_t s = E().stream;
     const std::vector<u64> ws = expand_winstates(h_winstates, n_winstates);
-    OneShot &o = E().one_shot;
-    o.busy = true;
-    bool ok = o.ws.cap >= ws.size() + 1 || grow(o.ws, 2 * ws.size() + 64, s);
-    if (ok && !ws.empty()) ok = CGB_CUDA(cudaMemcpyAsync(o.ws.p, ws.data(), ws.size() * 8, cudaMemcpyHostToDevice, s));
-    LayerIndex t2, t4;
-    t2.keys = d_k2;
-    t2.vals = d_v2;
-    t2.n = n2;
-    t4.keys = d_k4;
-    t4.vals = d_v4;
-    t4.n = n4;
-    const int vb = precision == 32 ? 4 : 8, kind = E().index_kind;
-    // one wait for what the host has to know first: the images that can be canonical
-    // follow the 0xf mask of the first board; FP32 tables' keys decide their slots
-    KeyBits bits[3];
-    CanonPlan plan;
-    if (ok && n) {
-        const KeySet none;
-        const bool want = vb == 4 && kind == INDEX_HASH;
-        ok = key_bits(want ? KeySet{d_k2, n2} : none, want ? KeySet{d_k4, n4} : none, bits, d_keys, E().ctr, s);
-        plan = make_canon_plan(bits[2].any, E().rules.free_formation != 0);
-    }
-    const SolveRules r = make_solve_rules(E().rules, o.ws.p, (int)ws.size());
-    // and one at the end, for the solve and both builds' error words
-    ok = ok && index_begin(t2, kind, vb, o.index[0], E().bucket_bits, E().ctr, s, bits[0], 0) &&
-         index_begin(t4, kind, vb, o.index[1], E().bucket_bits, E().ctr, s, bits[1], 1);
-    bool again = false;
-    do {
-        ok = ok && solve_layer_launch(d_keys, n, d_out, vb, t2, t4, r, E().rt, E().ctr, s, plan);
-        again = false;
-        ok = ok && solve_collect(E().ctr, s) && index_finish(t2, vb, o.index[0], E().ctr, s, &again) &&
-             index_finish(t4, vb, o.index[1], E().ctr, s, &again);
-    } while (ok && again);
-    E().end_one_shot();
-    CGB_TRY(ok);
+    CGB_TRY(one_shot_call([&](OneShot &o) {
+        bool ok = o.ws.cap >= ws.size() + 1 || grow(o.ws, 2 * ws.size() + 64, s);
+        if (ok && !ws.empty()) ok = CGB_CUDA(cudaMemcpyAsync(o.ws.p, ws.data(), ws.size() * 8, cudaMemcpyHostToDevice, s));
+        LayerIndex t2, t4;
+        t2.keys = d_k2;
+        t2.vals = d_v2;
+        t2.n = n2;
+        t4.keys = d_k4;
+        t4.vals = d_v4;
+        t4.n = n4;
+        const int vb = precision == 32 ? 4 : 8, kind = E().index_kind;
+        // one wait for what the host has to know first: the images that can be canonical
+        // follow the 0xf mask of the first board; FP32 tables' keys decide their slots
+        KeyBits bits[3];
+        CanonPlan plan;
+        if (ok && n) {
+            const KeySet none;
+            const bool want = vb == 4 && kind == INDEX_HASH;
+            ok = key_bits(want ? KeySet{d_k2, n2} : none, want ? KeySet{d_k4, n4} : none, bits, d_keys, E().ctr, s);
+            plan = make_canon_plan(bits[2].any, E().rules.free_formation != 0);
+        }
+        const SolveRules r = make_solve_rules(E().rules, o.ws.p, (int)ws.size());
+        // and one at the end, for the solve and both builds' error words
+        ok = ok && index_begin(t2, kind, vb, o.index[0], E().bucket_bits, E().ctr, s, bits[0], 0) &&
+             index_begin(t4, kind, vb, o.index[1], E().bucket_bits, E().ctr, s, bits[1], 1);
+        bool again = false;
+        do {
+            ok = ok && solve_layer_launch(d_keys, n, d_out, vb, t2, t4, r, E().rt, E().ctr, s, plan);
+            again = false;
+            ok = ok && solve_collect(E().ctr, s) && index_finish(t2, vb, o.index[0], E().ctr, s, &again) &&
+                 index_finish(t4, vb, o.index[1], E().ctr, s, &again);
+        } while (ok && again);
+        return ok;
+    }));
     return 0;
 }
 
@@ -394,12 +408,10 @@ int cgb_lookup_batch(const uint64_t *d_keys, const void *d_vals, uint64_t n, int
     if (search) {
         CGB_TRY(lookup_sorted(ix, vb, d_boards, m, canonicalize != 0, d_out, s));
     } else {
-        IndexStorage &st = E().one_shot.index[0];
-        E().one_shot.busy = true;
-        const bool ok = build_index(ix, E().index_kind, vb, st, E().bucket_bits, E().ctr, s) &&
-                        lookup_batch(ix, vb, d_boards, m, canonicalize != 0, d_out, s);
-        E().end_one_shot();
-        CGB_TRY(ok);
+        CGB_TRY(one_shot_call([&](OneShot &o) {
+            return build_index(ix, E().index_kind, vb, o.index[0], E().bucket_bits, E().ctr, s) &&
+                   lookup_batch(ix, vb, d_boards, m, canonicalize != 0, d_out, s);
+        }));
     }
     CGB_TRY(E().sync());
     return 0;

@@ -41,3 +41,44 @@ def test_layer_step_without_room_for_its_guess():
         assert sorted(got) == sorted(want) == [100, 102]
         assert all(len(want[s]) > 100_000 and np.array_equal(got[s], want[s]) for s in want)
     """)
+
+
+SOLVE = """
+        x = np.unique(realistic_boards(np.random.default_rng(2), 1_500_000))[:1_000_000]
+        many, few = device.to_device(x), device.to_device(x[:10])
+        val = torch.rand(len(x), dtype=torch.float64, device="cuda")
+        full, tiny = (many, val), (few, val[:10])
+        f = w.formations[0]
+
+        def solve(t2, t4):
+            return device.solve_layer(many[::100].contiguous(), t2, t4, f.winstates).cpu().numpy()
+
+        want = solve(tiny, full), solve(full, tiny)
+"""
+
+
+def test_kept_indexes_make_room():
+    """Two one-layer solves, each with one large table (64 MB of slots and 28 MB of build scratch), one
+    above and one below: what is kept from the first is in the way of the second."""
+    run(SOLVE + """
+        device.set_option("device_mem_cap_mb", 130)
+        for _ in range(2):
+            assert np.array_equal(solve(full, tiny), want[1])
+            assert np.array_equal(solve(tiny, full), want[0])
+            got = device.lookup_batch(few, val[:10], many[:40])   # more boards than keys: an index
+            assert torch.equal(got[:10], val[:10]) and not got[10:].any()
+    """)
+
+
+@pytest.mark.parametrize("cap", [150, 210])
+def test_sort_space_makes_room(cap):
+    """A sort of 4M keys keeps its buckets (168 MB; under the lower cap it gets half of them and gives
+    up), which are in the way of a one-layer solve that needs 92 MB."""
+    run(SOLVE + """
+        device.set_option("device_mem_cap_mb", 0)
+        k = torch.randint(0, 1 << 48, (4_000_000,), device="cuda", dtype=torch.int64)
+    """ + f"    device.set_option('device_mem_cap_mb', {cap})\n" + """
+        for _ in range(2):
+            assert torch.equal(device.sort(k)[0], torch.sort(k).values)
+            assert np.array_equal(solve(full, tiny), want[1])
+    """)

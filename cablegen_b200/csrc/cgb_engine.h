@@ -200,6 +200,7 @@ struct Engine {
     // indexes, the sort's buckets, the index builds' scratch (each after what the
     // stream still does with it)
     void drop_kept(cudaStream_t s);
+    bool give_back();        // that and freed blocks, all the way to the device
     void release_buffers();
 };
 

@@ -134,8 +134,8 @@ u64 failed_allocs()
 // the same stream.  The stream-ordered pool under them splits a large free block
 // for any smaller request, so a sweep that frees and allocates blocks of hundreds
 // of MB left it in pieces and made it map new memory, at 1 to 25 ms a time.
-// Bounded in bytes; everything goes back to the pool when an allocation fails,
-// under a memory cap, and with release_blocks().
+// Bounded in bytes; everything goes back to the pool when an allocation fails and
+// when a memory cap is set, under which nothing is kept.
 struct FreeBlock {
     void *p;
     u64 bytes;
@@ -790,13 +790,21 @@ void Engine::drop_kept(cudaStream_t s)
     index_release_scratch(s);
 }
 
+bool Engine::give_back()
+{
+    drop_kept(stream);
+    release_blocks();
+    if (!sync()) return false;
+    cudaMemPool_t pool;
+    return CGB_CUDA(cudaDeviceGetDefaultMemPool(&pool, device)) && CGB_CUDA(cudaMemPoolTrimTo(pool, 0));
+}
+
 void Engine::release_buffers()
 {
     GenBuffers &g = gen;
     for (DevBuf<u64> *b : {&g.a, &g.b, &g.c[0], &g.c[1], &g.S, &g.u2, &g.u4, &g.moved, &g.prev, &g.t})
         drop(*b, stream);
-    ws.buckets.release(stream);
-    one_shot.drop(stream);
+    drop_kept(stream);
     release_blocks();
 }
 

@@ -165,6 +165,8 @@ int cgb_set_option(const char *name, long long value)
             return -1;
         }
         g_dev_mem_cap = (u64)value << 20;
+        // what was kept without a cap, or under another, would not count towards it
+        if (E().ready && !E().give_back()) return -1;
     } else if (k == "region_build") {
         if (value < 0 || value > 1) {
             set_error("cgb_set_option: region_build must be 0 or 1");

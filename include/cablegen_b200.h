@@ -59,7 +59,9 @@ int cgb_set_rules(const cgb_rules *rules);
  * results of up to this many blocks of 1024 consecutive input boards at once),
  * "fp64_top_layers" (FP32 sweeps of cgb_sweep_run: the highest layers, solved
  * first, whose values come straight from the winstates, are solved in FP64 and
- * narrowed to FP32 for the layers below; default 4, 0 = none).
+ * narrowed to FP32 for the layers below; default 4, 0 = none),
+ * "device_mem_cap_mb" (a cap on the device memory that the engine holds, 0 = none;
+ * setting it, to any value, gives memory kept for later calls back to the device).
  * cgb_get_option returns -1 for an unknown name. */
 int cgb_set_option(const char *name, long long value);
 long long cgb_get_option(const char *name);

@@ -82,3 +82,41 @@ def test_sort_space_makes_room(cap):
             assert torch.equal(device.sort(k)[0], torch.sort(k).values)
             assert np.array_equal(solve(full, tiny), want[1])
     """)
+
+
+def test_cap_counts_what_was_kept_before_it():
+    """Blocks that a sweep freed are kept for the next; a cap set afterwards gives them back, so that the
+    engine holds what it says it holds, and a sweep under the cap stays below it."""
+    run("""
+        drv = C.CDLL("libcuda.so.1")
+        pool = C.c_void_p()
+        assert drv.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+
+        def used():
+            v = C.c_uint64()
+            assert drv.cuMemPoolGetAttribute(pool, 7, C.byref(v)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT
+            return v.value
+
+        f, peak = w.formations[0], []
+        def sweep():
+            device.tablebase(f.initial, f.start, 120, f.start, f.winstates,
+                             table_fn=lambda *a: peak.append(used()))
+
+        sweep()
+        torch.cuda.synchronize()
+        before = used()
+        device.set_option("device_mem_cap_mb", 1)
+        after = used()
+        try:
+            sweep()
+            raise SystemExit("a sweep within 1 MB")
+        except _lib.CablegenError as e:
+            held = float(str(e).split("(")[1].split(" GB held")[0]) * 1e9
+        small = 32 << 20  # the sort's own words are not counted
+        assert after <= held + small, (before, after, held)
+        cap = 4 << 30
+        device.set_option("device_mem_cap_mb", cap >> 20)
+        peak.clear()
+        sweep()
+        assert max(peak) <= cap + small, (max(peak), cap)
+    """)

@@ -504,7 +504,8 @@ struct BucketSmem {
 // their offset by look-back, write.  EMIT turns a sorted key into the u64.
 template <bool UNIQUE, bool DIRECT, int THREADS, typename K, class Emit>
 __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh, u32 cnt, u32 tile, u32 tiles, u32 *look,
-                                              u32 *head, u64 *__restrict__ out, u32 count_empties, BucketSmem<THREADS> &S, Emit emit)
+                                              u32 *head, u64 *__restrict__ out, u32 count_empties, LookbackLimit lb,
+                                              BucketSmem<THREADS> &S, Emit emit)
 {
     constexpr u32 ALL = 0xffffffffu;
     constexpr u32 AGG = 1u << 30, PRE = 2u << 30;
@@ -538,9 +539,9 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
         if (!DIRECT) {
             if (tile > 0) {
                 if (UNIQUE && lane == 0) st_relaxed(look + tile, AGG | total);
-                prefix = warp_lookback_sum<u32>(look, (int)tile - 1, head + H_FLAGS, SPIN_LIMIT);
+                prefix = warp_lookback_sum<u32>(look, (int)tile - 1, head + H_FLAGS, lb.polls);
             }
-            if (lane == 0) st_relaxed(look + tile, PRE | (prefix + total));
+            if (lane == 0 && !(lb.hold && tile == 0)) st_relaxed(look + tile, PRE | (prefix + total));
         }
         if (lane < THREADS / 32) S.warp[lane] = wi - c;
         if (lane == 0) {
@@ -584,7 +585,8 @@ __device__ __forceinline__ void finish_bucket(K (&v)[BK_KPT], K *buf, K *last_sh
 // are where the high words agree); the others are sorted as they are.
 template <bool UNIQUE, bool DIRECT, int THREADS>
 __device__ __forceinline__ void sort_bucket(const u64 *src, u32 cnt, u32 tile, u32 tiles, u32 *look, u32 *head,
-                                            u64 *__restrict__ out, u32 count_empties, BucketSmem<THREADS> &S)
+                                            u64 *__restrict__ out, u32 count_empties, LookbackLimit lb,
+                                            BucketSmem<THREADS> &S)
 {
     constexpr u32 ALL = 0xffffffffu;
     const u32 t = threadIdx.x;
@@ -620,7 +622,7 @@ __device__ __forceinline__ void sort_bucket(const u64 *src, u32 cnt, u32 tile, u
 #pragma unroll
         for (int i = 0; i < BK_KPT; i++) v[i] = (u32)k[i];  // KEY_MAX beyond cnt
         finish_bucket<UNIQUE, DIRECT, THREADS>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out,
-                                               count_empties, S, [=](u32 x) { return make64(high, x); });
+                                               count_empties, lb, S, [=](u32 x) { return make64(high, x); });
     } else if (low + __popc(vary_hi) <= 32) {
         if (t == 0) plan_moves(vary_lo, &S.lo);
         if (t == 32) plan_moves(vary_hi, &S.hi);
@@ -633,35 +635,37 @@ __device__ __forceinline__ void sort_bucket(const u64 *src, u32 cnt, u32 tile, u
             for (int i = 0; i < BK_KPT; i++) v[i] = warp_key(i) < cnt ? narrow_key(k[i], lo, hi, low) : ALL;
         }
         finish_bucket<UNIQUE, DIRECT, THREADS>(v, S.narrow, (u32 *)S.last64, cnt, tile, tiles, look, head, out,
-                                               count_empties, S,
+                                               count_empties, lb, S,
                                                [&](u32 x) { return wide_key(x, S.lo, S.hi, low) | fixed; });
     } else {
-        finish_bucket<UNIQUE, DIRECT, THREADS>(k, S.wide, S.last64, cnt, tile, tiles, look, head, out, count_empties, S,
-                                               [](u64 x) { return x; });
+        finish_bucket<UNIQUE, DIRECT, THREADS>(k, S.wide, S.last64, cnt, tile, tiles, look, head, out, count_empties, lb,
+                                               S, [](u64 x) { return x; });
     }
 }
 
 template <bool UNIQUE, bool DIRECT>
 __global__ void __launch_bounds__(BUCKET_THREADS, 4)
     bucket_sort_kernel(const u64 *input, KeyCount n, const u64 *slots, u32 counters, u32 words, u32 *head, u32 *arrays,
-                       u64 *__restrict__ out, u32 count_empties)
+                       u64 *__restrict__ out, u32 count_empties, LookbackLimit lb)
 {
     __shared__ BucketSmem<BUCKET_THREADS> S;
     after_previous();
     const u32 t = threadIdx.x;
     if (!slots || gridDim.x == 1) stamp((u64 *)(head + H_STAMP));  // no split before it
     const u32 all = n.get();
-    if (t == 0 && !DIRECT) S.tile = atomicAdd(head + H_TICKET, 1u);
+    // one thread reads the flags for all: another CTA's wait may run out and set one
+    // while this CTA starts
+    if (t == 0 && !DIRECT) S.tile = head[H_FLAGS] ? 0xFFFFFFFFu : atomicAdd(head + H_TICKET, 1u);
     if (t < 4) S.and_or[t] = t < 2 ? 0xffffffffu : 0u;
     const bool whole = DIRECT || all <= BK_CAP;
     __syncthreads();
     const u32 tile = DIRECT ? 0 : S.tile, tiles = whole ? 1 : head[H_BUCKETS];
-    if (!DIRECT && (tile >= tiles || head[H_FLAGS])) return;
+    if (!DIRECT && tile >= tiles) return;
     const u32 cnt = whole ? all : arrays[counters + tile];
     u32 *look = arrays + words;
     if (!UNIQUE && t == 0 && tile > 0) st_relaxed(look + tile, (1u << 30) | cnt);
     const u64 *src = whole ? input : slots + (u64)tile * BK_CAP;
-    sort_bucket<UNIQUE, DIRECT, BUCKET_THREADS>(src, cnt, tile, tiles, look, head, out, count_empties, S);
+    sort_bucket<UNIQUE, DIRECT, BUCKET_THREADS>(src, cnt, tile, tiles, look, head, out, count_empties, lb, S);
 }
 
 // Up to 16384 keys in one CTA of 1024 threads: a launch in place of three, whose
@@ -680,7 +684,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
     if (cnt == 0 || cnt > BK_SMALL) return;
     if (threadIdx.x < 4) S.and_or[threadIdx.x] = threadIdx.x < 2 ? 0xffffffffu : 0u;
     __syncthreads();
-    sort_bucket<UNIQUE, true, SMALL_THREADS>(input, cnt, 0, 1, nullptr, head, out, count_empties, S);
+    sort_bucket<UNIQUE, true, SMALL_THREADS>(input, cnt, 0, 1, nullptr, head, out, count_empties, LookbackLimit{}, S);
 }
 
 // ---------------------------------------------------------------------------
@@ -748,10 +752,10 @@ static void launch_sort(const BucketPlan &p, const u64 *keys, KeyCount kc, u64 *
 {
     if (p.n <= BK_CAP && !kc.counted)
         launch_after(bucket_sort_kernel<UNIQUE, true>, 1, BUCKET_THREADS, 0, s, keys, kc, nullptr, A_FINE,
-                     A_FINE + p.grid, head, arrays, out, empties);
+                     A_FINE + p.grid, head, arrays, out, empties, g_lookback);
     else
         launch_after(bucket_sort_kernel<UNIQUE, false>, p.grid, BUCKET_THREADS, 0, s, keys, kc, w.fine.p, A_FINE,
-                     A_FINE + p.grid, head, arrays, out, empties);
+                     A_FINE + p.grid, head, arrays, out, empties, g_lookback);
 }
 
 int bucket_enqueue(const BucketPlan &p, int slot, const u64 *keys, const u64 *counted, u64 *out, bool unique, bool empties,

@@ -16,6 +16,14 @@ __device__ __forceinline__ void st_relaxed64(u64 *p, u64 v)
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Polls of a look-back wait, and the test switch that keeps the first tile from
+// publishing its count (options "lookback_spin_limit", "lookback_hold_first_tile")
+struct LookbackLimit {
+    u32 polls = SPIN_LIMIT;
+    u32 hold = 0;
+};
+extern LookbackLimit g_lookback;
+
 // Warp-wide form of the walk back over one count per tile, called by all 32
 // lanes of one warp: lane i reads the word of tile j - i, so one round trip
 // covers 32 predecessors.  The words from tile j down to the nearest inclusive

@@ -57,6 +57,7 @@ constexpr int MRG_TILE = MRG_THREADS * MRG_KPT;
 // out of polls and reports ERR_LOOKBACK_TIMEOUT (the bounded-wait path).
 __device__ u32 g_spin_limit = SPIN_LIMIT;
 __device__ u32 g_hold_first_tile = 0;
+LookbackLimit g_lookback;  // the same for the bucket sort, which takes them as arguments
 
 __device__ __forceinline__ u32 lookback_sum(const u32 *words, u64 stride, int j, u32 *err)
 {
@@ -684,6 +685,7 @@ bool set_lookback_test(u32 spin_limit, int hold_first_tile)
 {
     const u32 lim = spin_limit ? spin_limit : SPIN_LIMIT;
     const u32 hold = hold_first_tile ? 1u : 0u;
+    g_lookback = LookbackLimit{lim, hold};
     return CGB_CUDA(cudaMemcpyToSymbol(g_spin_limit, &lim, sizeof lim)) &&
            CGB_CUDA(cudaMemcpyToSymbol(g_hold_first_tile, &hold, sizeof hold));
 }

@@ -14,8 +14,9 @@
 //                 above 400 buckets this runs twice: coarse buckets first, then
 //                 every coarse bucket by boundaries of its own;
 //   3. bucket:    one CTA per bucket (at most 4096 keys, 1800 on average) sorts
-//                 it in shared memory -- 16 keys per thread through a register
-//                 network, then merge-path merges -- drops repeats when asked
+//                 it -- 16 keys per thread through a register network, the 512
+//                 of a warp by bitonic merges across its lanes, runs of 512 by
+//                 merge-path steps in shared memory -- drops repeats when asked
 //                 (equal keys always share a bucket) and writes at the offset
 //                 that a look-back over the buckets' counts gives.
 // Inputs of up to 16384 keys are one bucket, sorted by one CTA of 1024 threads
@@ -26,7 +27,7 @@
 // instruction issue (280 warp instructions per 32 keys at 2.3 per cycle), neither
 // by HBM.  Measured on B200, against byte-digit passes over 4096-key tiles:
 // 11.5M LL moves 0.73 -> 0.40 ms, 1.27M DPDF moves 141 -> 92 us, 34M moves of
-// LL with free formation 2.18 -> 1.33 ms, 4100 2x4 moves 53 -> 28 us.
+// LL with free formation 2.18 -> 1.33 ms, 4100 2x4 moves (one CTA) 53 -> 15 us.
 //
 // The space of a bucket is fixed, so an input whose keys repeat so often that
 // one bucket cannot hold them (or whose sample misleads) sets a flag and
@@ -261,6 +262,7 @@ __device__ __forceinline__ void reduce_and_or(u64 a, u64 o, u32 *and_or)
     else if (lane < 4) atomicOr(and_or + lane, lane == 3 ? r[3] : r[2]);
 }
 
+// lowbias32 (Wellons, Hash Prospector, 2018)
 __device__ __forceinline__ u32 mix32(u32 x)
 {
     x = (x ^ (x >> 16)) * 0x7feb352du;

@@ -37,7 +37,9 @@ const char *last_error();
 
 // Per-kernel device time and algorithmic bytes, accumulated over launches.
 // Launch time comes from CUDA events recorded around each launch on the
-// launching stream and resolved at the next host synchronisation point.
+// launching stream and resolved at the next host synchronisation point; in a
+// layer step without waits, whose kernels events would keep apart, from the
+// times at which they start (stamp), which come back with the step's sizes.
 struct KernelStats {
     u64 launches = 0;
     double hist_ms = 0, onesweep_ms = 0, unique_ms = 0, merge_ms = 0, expand_ms = 0, spawn_ms = 0,
@@ -54,7 +56,6 @@ KernelStats &kstats();
 class KClock {
   public:
     void begin(cudaStream_t s, double *acc);
-    void next(cudaStream_t s, double *acc);  // end and begin with one event
     void end(cudaStream_t s);
     size_t pending() const { return pend_.size(); }
     void flush(size_t first = ~(size_t)0);  // adds up the first so many spans, which are over
@@ -62,7 +63,6 @@ class KClock {
     struct Pending {
         cudaEvent_t a, b;
         double *acc;
-        bool last;  // b is not the next entry's a
     };
     cudaEvent_t take();
     std::vector<cudaEvent_t> free_;

@@ -91,17 +91,8 @@ void KClock::end(cudaStream_t s)
     if (!open_) return;
     cudaEvent_t b = take();
     cudaEventRecord(b, s);
-    pend_.push_back({open_, b, open_acc_, true});
+    pend_.push_back({open_, b, open_acc_});
     open_ = nullptr;
-}
-void KClock::next(cudaStream_t s, double *acc)
-{
-    cudaEvent_t b = take();
-    cudaEventRecord(b, s);
-    pend_.push_back({open_, b, open_acc_, false});
-    open_ = b;
-    open_acc_ = acc;
-    kstats().launches++;
 }
 void KClock::flush(size_t first)
 {
@@ -111,7 +102,7 @@ void KClock::flush(size_t first)
         float ms = 0;
         if (cudaEventElapsedTime(&ms, p.a, p.b) == cudaSuccess && p.acc) *p.acc += ms;
         free_.push_back(p.a);
-        if (p.last) free_.push_back(p.b);
+        free_.push_back(p.b);
     }
     pend_.erase(pend_.begin(), pend_.begin() + first);
 }

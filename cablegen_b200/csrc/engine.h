@@ -116,8 +116,8 @@ int sort_plan(const u32 *hist_host, u64 n, int *digits);
 // sorts keys[0,n) ascending using tmp[0,n); *sorted points at keys or tmp
 bool sort_keys(u64 *keys, u64 *tmp, u64 n, u64 **sorted, SortWorkspace &ws, cudaStream_t s,
                SortStats *stats = nullptr);
-// reports device errors a sort left behind (when no unique_keys follows)
 bool bucket_sorts();  // whether the "sort_variant" option lets the bucket sort run
+// reports device errors a sort left behind (when no unique_keys follows)
 bool sort_check(SortWorkspace &ws, cudaStream_t s);
 // sort_keys then unique_keys, in one pass over the buckets where they apply:
 // *out points at keys or tmp

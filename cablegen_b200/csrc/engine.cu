@@ -134,7 +134,7 @@ struct FreeBlock {
 };
 static std::vector<FreeBlock> g_free_blocks;
 static u64 g_free_bytes = 0;
-static constexpr u64 LARGE_BLOCK = 16ull << 20, FREE_BLOCK_BYTES = 8ull << 30;
+static constexpr u64 FREE_BLOCK_BYTES = 8ull << 30;
 
 void release_blocks()
 {

@@ -24,6 +24,7 @@ struct DevBuf {
 // whatever layers and tables other streams are sending to the host
 bool words_to_host(u32 *pinned, const u32 *dev, int words, cudaStream_t s, u64 *started = nullptr);
 
+constexpr u64 LARGE_BLOCK = 16ull << 20;  // freed blocks from this size up are kept for the next allocation
 bool dev_alloc(void **p, u64 bytes, cudaStream_t s);
 u64 failed_allocs();  // how many dev_alloc calls have found no memory
 void dev_free(void *p, cudaStream_t s);

@@ -1,10 +1,10 @@
 // bucketsort.cu -- sort of u64 keys, with or without their repeats, by sampled
-// splitters and a merge sort of each bucket in shared memory.
+// splitters and a merge sort of each bucket by one CTA.
 //
-// The layer streams (move results, spawns) are sorted three times per layer
-// step.  An LSD radix sort moves every key once per varying byte (six times
-// for an LL board) and pays a fixed latency per pass, so both large and small
-// streams are slow.  Here a key moves two or three times whatever its width:
+// The layer streams (move results, spawns) are sorted in every layer step.  An LSD
+// radix sort moves every key once per varying byte (six times for an LL board) and
+// pays a fixed latency per pass, so both large and small streams are slow.  Here a
+// key moves two or three times whatever its width:
 //   1. split:     one CTA sorts a sample of the input (20 to 64 keys per bucket) and
 //                 keeps the bucket boundaries;
 //   2. partition: each tile of 4096 keys finds its keys' buckets by binary
@@ -27,7 +27,8 @@
 // instruction issue (280 warp instructions per 32 keys at 2.3 per cycle), neither
 // by HBM.  Measured on B200, against byte-digit passes over 4096-key tiles:
 // 11.5M LL moves 0.73 -> 0.40 ms, 1.27M DPDF moves 141 -> 92 us, 34M moves of
-// LL with free formation 2.18 -> 1.33 ms, 4100 2x4 moves (one CTA) 53 -> 15 us.
+// LL with free formation 2.18 -> 1.33 ms, 4100 2x4 moves (one CTA) 53 -> 15 us; against
+// those over 8192-key tiles, 120M keys of 48 bits 4.94 -> 4.36 ms, 168M 6.81 -> 5.82.
 //
 // The space of a bucket is fixed, so an input whose keys repeat so often that
 // one bucket cannot hold them (or whose sample misleads) sets a flag and

@@ -126,7 +126,9 @@ struct GenBuffers {
     static constexpr u64 UNKNOWN = ~0ull;
     u64 moved_empties = UNKNOWN, prev_empties = 0;
     KeyBits moved_bits;        // AND and OR of the moved layer, where its sort gave them
-    double spawn_ratio = 16, move_ratio = 4;  // spawns and moves per board of S in the last layer step
+    // spawns and moves per board of S in the last layer step; before the first, a
+    // guess for boards with few tiles (8 spawns in place of 16: no difference)
+    double spawn_ratio = 16, move_ratio = 4;
 };
 
 // a layer step in flight (Engine::quick_launch): its sizes as they were planned
@@ -180,8 +182,11 @@ struct Engine {
     bool move_layer(const u64 *d_in, u64 n, GenTimes *tm);
     bool spawn_streams(GenTimes *tm);   // g.u2, g.u4: the sorted unique 2- and 4-spawns of g.moved
     bool spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm);
-    // layers of at most so many boards to move take quick_launch: above, kernels
-    // of a millisecond hide the waits
+    // Layers of at most so many boards to move take quick_launch: above, kernels
+    // of a millisecond hide the waits.  Generation with a limit of 0 / 2^19 / 2^21 /
+    // 2^23 boards: 2x4 18.6 / 8.3 / 8.3 / 8.3 ms, dpdf to 380 13.2 / 12.2 / 10.8 / 10.8,
+    // LL to 120 28.7 / 27.4 / 26.9 / 26.1, to 200 106.9 / 105.6 / 104.9 / 104.3; four times
+    // the boards would mean four times the room for guessed spawns (0.4 GB for 2M LL boards)
     static constexpr u64 QUICK_BOARDS = 1u << 21;
     QuickStep quick;
     bool quick_launch(bool last);
@@ -200,7 +205,7 @@ struct Engine {
     // gives back what is kept only to make the next call faster: one-layer calls'
     // indexes, the sort's buckets, the index builds' scratch (each after what the
     // stream still does with it)
-    void drop_kept(cudaStream_t s);
+    void drop_kept();
     bool give_back();        // that and freed blocks, all the way to the device
     void release_buffers();
 };

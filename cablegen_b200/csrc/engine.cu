@@ -614,6 +614,8 @@ bool Engine::quick_launch(bool last)
         return true;
     }
     BucketWorkspace &w = ws.buckets;
+    // a quarter more than the last ratios give decides whether one CTA will do; where it
+    // does not, the step with waits repeats what overflowed
     const u64 likely[2] = {(u64)(1.25 * (double)n * g.move_ratio), (u64)(1.25 * (double)n * g.spawn_ratio)};
     if (!bucket_prepare(sizes, last ? 1 : 2, plans, w, s, likely)) return true;
     // its own copy: what runs between launch and take may sort too

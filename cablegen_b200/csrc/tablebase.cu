@@ -402,12 +402,19 @@ int cgb_lookup_batch(const uint64_t *d_keys, const void *d_vals, uint64_t n, int
     ix.vals = d_vals;
     ix.n = n;
     const int vb = precision == 32 ? 4 : 8;
-    // Building the hash index costs 43 ps per key, a lookup in it 20 to 30 ps; a
-    // search of the sorted layer costs 70 ps per board while the layer fits in L2
-    // (16M keys), 200 ps beyond.  So the search wins up to about n boards, or n / 4.
-    // Measured (search / index): 100 boards in 0.88M keys 28 / 184 us, 1M in 5.4M
-    // 103 / 366 us, 5.4M in 5.4M 365 / 456 us, 36M in 36M 7.3 / 2.6 ms.
-    const bool search = E().index_kind == INDEX_HASH && m <= (n <= (1u << 24) ? n : n / 4);
+    // Building the hash index costs 40 to 50 ps per key (33 to 38 in 8-byte slots of 2M to 4M
+    // keys), a lookup in it 6 to 27 ps; a search of the sorted layer costs 62 to 73 ps per
+    // board while the layer fits in L2 (16M keys), 200 ps beyond.  So the search wins up to n
+    // boards, or a share of n where the index is cheap or the layer large.  Measured (search /
+    // index, us): 100 boards in 0.88M keys 28 / 184, 1M in 1M 90 / 122, 3M in 3M FP64 226 / 230,
+    // 16M in 16M 1244 / 1118 and three quarters of that 952 / 1014, 36M in 36M 7300 / 2600;
+    // FP32 (where its keys allow 8-byte slots) 3M in 3M 223 / 177, half of that 133 / 164,
+    // 7M in 7M 489 / 433, half 275 / 391, 10M in 10M 715 / 737.
+    const u64 M = 1u << 20;
+    const u64 most = n <= 2 * M ? n : n > 16 * M ? n / 4
+                     : vb == 8  ? (n <= 8 * M ? n : n - n / 5)
+                                : (n <= 4 * M ? n - 3 * n / 8 : n <= 8 * M ? n - n / 4 : n);
+    const bool search = E().index_kind == INDEX_HASH && m <= most;
     if (search) {
         CGB_TRY(lookup_sorted(ix, vb, d_boards, m, canonicalize != 0, d_out, s));
     } else {

@@ -658,7 +658,10 @@ __global__ void __launch_bounds__(BUCKET_THREADS, 4)
     const u32 all = n.get();
     // one thread reads the flags for all: another CTA's wait may run out and set one
     // while this CTA starts
-    if (t == 0 && !DIRECT) S.tile = head[H_FLAGS] ? 0xFFFFFFFFu : atomicAdd(head + H_TICKET, 1u);
+    if (t == 0 && !DIRECT) {
+        const u32 ticket = atomicAdd(head + H_TICKET, 1u);  // (with the flags on their way too)
+        S.tile = ld_relaxed(head + H_FLAGS) ? 0xFFFFFFFFu : ticket;
+    }
     if (t < 4) S.and_or[t] = t < 2 ? 0xffffffffu : 0u;
     const bool whole = DIRECT || all <= BK_CAP;
     __syncthreads();

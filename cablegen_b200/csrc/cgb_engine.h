@@ -184,8 +184,8 @@ struct Engine {
     bool spawn_into(SpawnSource src, DevBuf<u64> &acc, GenTimes *tm);
     // Layers of at most so many boards to move take quick_launch: above, kernels
     // of a millisecond hide the waits.  Generation with a limit of 0 / 2^19 / 2^21 /
-    // 2^23 boards: 2x4 18.6 / 8.3 / 8.3 / 8.3 ms, dpdf to 380 13.2 / 12.2 / 10.8 / 10.8,
-    // LL to 120 28.7 / 27.4 / 26.9 / 26.1, to 200 106.9 / 105.6 / 104.9 / 104.3; four times
+    // 2^23 boards: 2x4 18.9 / 8.4 / 8.4 / 8.4 ms, dpdf to 380 13.2 / 12.2 / 10.7 / 10.7,
+    // LL to 120 28.5 / 27.2 / 26.6 / 26.1, to 200 106.0 / 104.6 / 103.9 / 103.8; four times
     // the boards would mean four times the room for guessed spawns (0.4 GB for 2M LL boards)
     static constexpr u64 QUICK_BOARDS = 1u << 21;
     QuickStep quick;
